@@ -202,8 +202,8 @@ __device__ __forceinline__ void run_steps(const CostCtx& c, const RunGeom& g, in
     uint32_t* pp = s_pre + xs * W2 + WPL * lane;                             // prefix words of (xs)
     uint16_t* cp = s_cnt + xs * W2 + WPL * lane;                             // count words of (xs)
     uint32_t* vp = out_vol + ((size_t)row + (xbase + xs)) * W2 + WPL * lane;  // volume words of (xs)
-    // byte volume: the lane's 2 * WPL disparities of (xs) as WPL / 2 words
-    uint32_t* vp8 = out_vol + ((size_t)row + (xbase + xs)) * (W2 / 2) + (WPL / 2) * lane;
+    // byte volume: the lane's P disparities of (xs)
+    uint8_t* vp8 = reinterpret_cast<uint8_t*>(out_vol) + ((size_t)row + (xbase + xs)) * (2 * W2) + P * lane;
     for (int xi = xs; xi < xe; xi += 4) {
         const uint4 lc4 = *reinterpret_cast<const uint4*>(s_lc + xi);
         uint4 lg4 = make_uint4(0, 0, 0, 0);
@@ -293,10 +293,17 @@ __device__ __forceinline__ void run_steps(const CostCtx& c, const RunGeom& g, in
                     for (int w = 0; w < WPL; ++w) wd[w] = qp[w] | ~vm[w];  // invalid halves: 0xFFFF
                     if constexpr (U8) {
                         // the low byte of each half: costs are below 255, the invalid 0xFFFF becomes 0xFF
-                        uint32_t wb[WPL / 2];
+                        if constexpr (WPL % 2 == 0) {
+                            uint32_t wb[WPL / 2];
 #pragma unroll
-                        for (int w = 0; w < WPL / 2; ++w) wb[w] = __byte_perm(wd[2 * w], wd[2 * w + 1], 0x6420);
-                        store_words<WPL / 2>(vp8 + (size_t)s * (W2 / 2), wb);
+                            for (int w = 0; w < WPL / 2; ++w) wb[w] = __byte_perm(wd[2 * w], wd[2 * w + 1], 0x6420);
+                            store_words<WPL / 2>(reinterpret_cast<uint32_t*>(vp8 + (size_t)s * (2 * W2)), wb);
+                        } else {
+#pragma unroll
+                            for (int w = 0; w < WPL; ++w)
+                                *reinterpret_cast<uint16_t*>(vp8 + (size_t)s * (2 * W2) + 2 * w) =
+                                    (uint16_t)__byte_perm(wd[w], 0u, 0x4420);
+                        }
                     } else {
                         store_words<WPL>(vp + (size_t)s * W2, wd);
                     }
@@ -307,7 +314,7 @@ __device__ __forceinline__ void run_steps(const CostCtx& c, const RunGeom& g, in
         pp += 4 * W2;
         cp += 4 * W2;
         vp += 4 * (size_t)W2;
-        vp8 += 2 * (size_t)W2;
+        vp8 += 8 * (size_t)W2;
     }
     __syncwarp();
     if (xe > xs) {
@@ -598,12 +605,15 @@ cudaError_t launch_runs_w(const CostCtx& c, int txc, int lmax, int tau, uint32_t
 template <bool CROSS, bool STORE, bool FULL, bool PRIOR>
 cudaError_t launch_runs_p(const CostCtx& c, int txc, int lmax, int tau, uint32_t* vol, uint32_t* rkey,
                           const uint32_t* magic, cudaStream_t s) {
-    if constexpr (STORE && !CROSS && !FULL && !PRIOR) {
-        // the byte volume (Fast census-only costs below 255): 128 or 256 padded disparities
+    if constexpr (STORE && !CROSS && !FULL) {
+        // the byte volume (Fast census-only costs below 255)
         if (c.vol8) {
-            if (c.Dp == 128) return launch_runs_w<CROSS, STORE, FULL, 2, PRIOR, true>(c, txc, lmax, tau, vol, rkey, magic, s);
-            if (c.Dp == 256) return launch_runs_w<CROSS, STORE, FULL, 4, PRIOR, true>(c, txc, lmax, tau, vol, rkey, magic, s);
-            return cudaErrorInvalidValue;
+            switch (c.Dp) {
+                case 64: return launch_runs_w<CROSS, STORE, FULL, 1, PRIOR, true>(c, txc, lmax, tau, vol, rkey, magic, s);
+                case 128: return launch_runs_w<CROSS, STORE, FULL, 2, PRIOR, true>(c, txc, lmax, tau, vol, rkey, magic, s);
+                case 192: return launch_runs_w<CROSS, STORE, FULL, 3, PRIOR, true>(c, txc, lmax, tau, vol, rkey, magic, s);
+                default: return launch_runs_w<CROSS, STORE, FULL, 4, PRIOR, true>(c, txc, lmax, tau, vol, rkey, magic, s);
+            }
         }
     } else {
         if (c.vol8) return cudaErrorInvalidValue;

@@ -186,6 +186,10 @@ static int max_full_cost(const apg_pipeline_config_t& c) {
     return std::min((int)(v * scale + 0.5 + 1e-3), c.cost_max);
 }
 
+static SgmPen pen_of(const apg_pipeline_config_t& c) {
+    return SgmPen{c.P1, c.P2_base, c.adaptive_penalties, c.piecewise_p2, c.grad_t1, c.grad_t2, c.p2_alpha};
+}
+
 Layout Engine::make_layout(const apg_pipeline_config_t& c, int w, int h, int ch, int debug) {
     Layout L;
     L.w = w; L.h = h; L.ch = ch;
@@ -198,20 +202,20 @@ Layout Engine::make_layout(const apg_pipeline_config_t& c, int w, int h, int ch,
     L.fused_fast = !L.cross && c.census_type == APG_CENSUS_SYMMETRIC_9X7 && !c.use_ad && !c.use_grad &&
                    !c.prior_enable && !c.hier_enable && (debug & kLayoutFastFused) && !(debug & 4);
     L.raw_cost = (debug & 1) != 0;
-    // Fast census-only path with its volume stored: one byte per voxel when every quantised cost is
-    // below 255, so 0xFF marks the invalid voxels exactly (the sweeps' 32-lane form, the pixel-run
-    // cost kernel).  At a padded range of 256 it is the default: one B200, Fast 1920x1080 D256, 2.64
-    // vs 2.83 ms per frame (first phase 0.96 vs 1.20 ms).  At 128 only on request (kLayoutCost8):
-    // Fast 1280x720 D128 0.757 vs 0.749 ms, the first phase's chains there wait on the latency of
-    // each step (widening the bytes) more than on the volume's bytes.  kLayoutCost16 keeps two bytes.
-    // The same holds for the aggregated volume of Balanced / HighQuality (one aggregation pass),
-    // written by the vertical aggregation: aggregated costs are window averages of quantised costs,
-    // so below 255 when every quantised cost is.
+    // The byte sweeps (sgm8.cu) run where every quantised cost is below 255, so 0xFF marks the invalid
+    // voxels exactly, and the largest P2 is at most 255, so the path values' distances above the costs
+    // fit a byte: the census-only Fast volume (written by the pixel-run cost kernel) and the aggregated
+    // volume of one aggregation pass (window averages of quantised costs, written by the vertical
+    // aggregation).  kLayoutCost16 (tuning cost8 = 1, other lane counts) keeps the 16-bit sweeps.  The
+    // arena's volume and sum buffers keep the 16-bit sweeps' sizes, so either form runs in it, but for
+    // the volume at a padded range of 256 (at 128 on request, kLayoutCost8).
     const bool fast8 = !L.cross && !L.fused_fast && c.census_type == APG_CENSUS_SYMMETRIC_9X7 && !c.use_ad &&
-                       !c.use_grad && !c.prior_enable && !c.hier_enable && max_census_cost(c) < 255;
+                       !c.use_grad && max_census_cost(c) < 255;
     const bool cross8 = L.cross && c.agg_iterations <= 1 && max_full_cost(c) < 255;
-    L.cost8 = (fast8 || cross8) && (L.Dp == 256 || (L.Dp == 128 && (debug & kLayoutCost8))) &&
-              !(debug & kLayoutCost16);
+    // (the byte sweeps address a volume by 32-bit byte offsets)
+    L.bytes = (fast8 || cross8) && sgm8_supported(L.Dp, pen_of(c)) && !(debug & kLayoutCost16) &&
+              (unsigned long long)w * h * L.Dp < (1ull << 32);
+    L.cost8 = L.bytes && (L.Dp == 256 || (L.Dp == 128 && (debug & kLayoutCost8)));
     const size_t n = (size_t)w * h;
     const size_t csz = c.census_type == APG_CENSUS_9X7 ? 8 : 4;
     const size_t vol = n * (size_t)L.Dp * 2;
@@ -413,7 +417,8 @@ int Engine::prepare_arena(int w, int h, int ch) {
                                  debug_ | (fast_fused_ ? kLayoutFastFused : 0) | (cost16 ? kLayoutCost16 : 0) |
                                      (cost8_ == 2 ? kLayoutCost8 : 0));
     if (arena_ && arena_bytes_ >= L.total && lay_.w == w && lay_.h == h && lay_.ch == ch &&
-        lay_.raw_cost == L.raw_cost && lay_.fused_fast == L.fused_fast && lay_.cost8 == L.cost8) {
+        lay_.raw_cost == L.raw_cost && lay_.fused_fast == L.fused_fast && lay_.cost8 == L.cost8 &&
+        lay_.bytes == L.bytes) {
         return kOk;
     }
     if (arena_ && arena_bytes_ >= L.total) {
@@ -776,7 +781,7 @@ int Engine::run_pre(const uint8_t* dl, int lstride, const uint8_t* dr, int rstri
         if (!L.raw_cost) RUN(launch_cost(cc, 2, lmax, 0, nullptr, ptr<uint32_t>(L.rkey), magic, s), "right argmin");
     } else {
         CostCtx cv = cc;
-        cv.vol8 = L.cost8 ? 1 : 0;
+        cv.vol8 = L.bytes ? 1 : 0;
         RUN(launch_cost(cv, 0, lmax, 0, ptr<uint32_t>(L.volA), ptr<uint32_t>(L.rkey), magic, s), "cost");
         sgm_src = ptr<uint32_t>(L.volA);
     }
@@ -798,7 +803,7 @@ int Engine::run_pre(const uint8_t* dl, int lstride, const uint8_t* dr, int rstri
     if (L.cross) {
         const int tau = cfg_.color_threshold;
         RUN(launch_cross_v(w, h, d0, D, Dp, lmax, tau, ptr<uint8_t>(L.lgray), ptr<int16_t>(L.rmin), ptr<int16_t>(L.rmax),
-                           ptr<uint32_t>(L.volA), ptr<uint32_t>(L.volB), magic, !ranged(), L.cost8, s), "crossV");
+                           ptr<uint32_t>(L.volA), ptr<uint32_t>(L.volB), magic, !ranged(), L.bytes, s), "crossV");
         const int iters = std::max(1, cfg_.agg_iterations);
         for (int it = 1; it < iters; ++it) {
             RUN(launch_cross_h(w, h, d0, D, Dp, lmax, tau, ptr<uint8_t>(L.lgray), ptr<int16_t>(L.rmin), ptr<int16_t>(L.rmax),
@@ -818,8 +823,7 @@ int Engine::sgm_launch(SgmLaunch* out, uint32_t** sbufs) const {
     const Layout& L = lay_;
     SgmLaunch& pl = *out;
     pl.w = L.w; pl.h = L.h; pl.d0 = cfg_.min_disparity; pl.D = L.D; pl.Dp = L.Dp;
-    pl.pen = SgmPen{cfg_.P1, cfg_.P2_base, cfg_.adaptive_penalties, cfg_.piecewise_p2, cfg_.grad_t1, cfg_.grad_t2,
-                    cfg_.p2_alpha};
+    pl.pen = pen_of(cfg_);
     pl.gray = ptr<uint8_t>(L.lgray);
     // the volume run_pre leaves for the sweeps: cross-aggregated (volB), raw (volA), or none when
     // the Fast sweeps recompute their census costs
@@ -833,7 +837,16 @@ int Engine::sgm_launch(SgmLaunch* out, uint32_t** sbufs) const {
     pl.store_final = (debug_ & 2) != 0;
     pl.lanes = sgm_lanes_;
     pl.split = sgm_split_;
-    pl.cost8 = (!L.fused_fast && L.cost8) ? 1 : 0;
+    pl.cost8 = L.bytes ? 1 : 0;
+    pl.default_ranges = ranged() ? 0 : 1;
+    if (L.bytes) {
+        // two directions' byte buffers in each of the sum buffers but the first, which the stage
+        // dump of the final sums takes
+        const size_t vb = (size_t)L.w * L.h * L.Dp;
+        for (int i = 0; i < L.nsbuf; ++i) sbufs[i] = ptr<uint32_t>(L.sbuf[1 + i / 2] + (i & 1 ? vb : 0));
+        pl.sum = pl.store_final ? ptr<uint32_t>(L.sbuf[0]) : nullptr;
+        return L.nsbuf;
+    }
     for (int i = 0; i < L.nsbuf; ++i) sbufs[i] = ptr<uint32_t>(L.sbuf[i]);
     return L.nsbuf;
 }
@@ -943,6 +956,14 @@ int Engine::run_sgm() {
     SgmLaunch pl;
     uint32_t* sb[7];
     sgm_launch(&pl, sb);
+    if (L.bytes) {
+        uint8_t* const* d8 = reinterpret_cast<uint8_t* const*>(sb);
+        RUN(launch_sgm8_first(pl, L.nsbuf, L.nsbuf == 7 ? first8 : first4, d8, s), "sgm_first");
+        RUN(launch_sgm8_last(pl, 0, -1, L.nsbuf, d8, s), "sgm_last_wta");
+        cudaEventRecord(ev_[6], s);
+        count_launches(launches);
+        return kOk;
+    }
     RUN(launch_sgm_first(pl, L.nsbuf, L.nsbuf == 7 ? first8 : first4, sb, s), "sgm_first");
     if (L.nsbuf == 7) {
         RUN(launch_sgm_fold(sb, 5, n * (size_t)(Dp / 2), s), "sgm_fold5");
@@ -1075,9 +1096,10 @@ int Engine::host_band_count(bool device) const {
     SgmLaunch pl;
     uint32_t* sb[7];
     sgm_launch(&pl, sb);
-    if (!sgm_last_band_supported(pl, 3)) return 0;
+    if (!L.bytes && !sgm_last_band_supported(pl, 3)) return 0;
     // the chains' state between bands lives in the refiner's map, unused without the refiner
-    if ((size_t)32 * (L.Dp / 64 + 1) * 4 > (size_t)L.h * 4) return 0;
+    const size_t carry = L.bytes ? sgm8_carry_words(L.w, L.Dp) : (size_t)L.w * 32 * (L.Dp / 64 + 1);
+    if (carry > (size_t)L.w * L.h) return 0;
     return req > 1 ? std::min(req, (int)kMaxBands) : (int)kBands;
 }
 
@@ -1094,7 +1116,8 @@ int Engine::run_banded(int nb, float* hdisp, float* hconf, uint8_t* hreason, uin
     SgmLaunch pl;
     uint32_t* sb[7];
     sgm_launch(&pl, sb);
-    RUN(launch_sgm_first(pl, 3, first4, sb, s), "sgm_first");
+    uint8_t* const* d8 = reinterpret_cast<uint8_t* const*>(sb);
+    RUN(L.bytes ? launch_sgm8_first(pl, 3, first4, d8, s) : launch_sgm_first(pl, 3, first4, sb, s), "sgm_first");
     RUNC(cudaEventRecord(ev_fork_, s), "event");
     RUNC(cudaStreamWaitEvent(ss, ev_fork_, 0), "event");
     // the confidence stage reads the right-image disparity
@@ -1143,7 +1166,8 @@ int Engine::run_banded(int nb, float* hdisp, float* hconf, uint8_t* hreason, uin
     int fill_hi = h, fin_hi = h;  // rows [fill_hi, h) of the fill map, [fin_hi, h) of the final map are done
     for (int band = 0; band < nband; ++band) {
         const int t0 = tb[band], t1 = tb[band + 1];
-        RUN(launch_sgm_last_band(pl, 0, -1, 3, sb, t0, t1, carry, ss), "sgm_last_band");
+        RUN(L.bytes ? launch_sgm8_last_band(pl, 0, -1, 3, d8, t0, t1, carry, ss)
+                    : launch_sgm_last_band(pl, 0, -1, 3, sb, t0, t1, carry, ss), "sgm_last_band");
         RUNC(cudaEventRecord(band_ev_[2 * band], ss), "event");
         RUNC(cudaStreamWaitEvent(ps, band_ev_[2 * band], 0), "event");
         const int ylo = h - t1, yhi = h - t0;
@@ -1418,7 +1442,7 @@ int Engine::dump(int what, void* dst, size_t bytes) {
             if (!L.cross) return fail(kInternalError, "no aggregated volume");
             off = L.volB;
             vol = true;
-            vol8 = L.cost8;
+            vol8 = L.bytes;
             break;
         case 12: if (!(debug_ & 2)) return fail(kInternalError, "path sum not kept"); off = L.sbuf[0]; vol = true; break;
         case 13: off = L.disp_wta; sz = n * 4; break;

@@ -38,7 +38,9 @@ struct Layout {
     bool fused_fast = false;  // Fast path: costs recomputed inside the SGM sweeps, no volume
     bool cross = false;
     bool raw_cost = false;    // debug: materialise the raw volume
-    bool cost8 = false;       // Fast path: the volume the sweeps read holds one byte per voxel (0xFF invalid)
+    bool bytes = false;       // the byte sweeps (sgm8.cu): the volume they read holds one byte per voxel (0xFF
+                              // invalid) and the first phase one byte per voxel and direction
+    bool cost8 = false;       // with `bytes`: the volume is allocated at one byte per voxel
     size_t total = 0;
     // offsets
     size_t in_left, in_right;

@@ -76,7 +76,9 @@ struct SgmLaunch {
     int lanes;        // lanes per scanline chain (8, 16, 32; 0 = default for Dp)
     int split = 0;    // volume-fed last sweep over two warps per chain: 0 = where it pays (Dp 64),
                       // 1 = never, 2 = always (32 lanes per chain only)
-    int cost8 = 0;    // cvol holds one byte per voxel, 0xFF invalid (32 lanes, Dp 128 or 256)
+    int cost8 = 0;    // cvol holds one byte per voxel, 0xFF invalid: the byte sweeps (launch_sgm8_*)
+    int default_ranges = 0;    // byte sweeps: every pixel has the default range
+    uint32_t* sum = nullptr;   // byte sweeps: the final sums as a 16-bit volume (stage dumps), or none
 };
 // First phase: ndir directions in one launch, direction i writing its path values to out[i].
 cudaError_t launch_sgm_first(const SgmLaunch& l, int ndir, const int (*dirs)[2], uint32_t* const* out,
@@ -90,6 +92,16 @@ cudaError_t launch_sgm_last(const SgmLaunch& l, int dx, int dy, int nin, const u
 bool sgm_last_band_supported(const SgmLaunch& l, int nin);
 cudaError_t launch_sgm_last_band(const SgmLaunch& l, int dx, int dy, int nin, const uint32_t* const* in, int t_begin,
                                  int t_end, uint32_t* carry, cudaStream_t s);
+// sgm8.cu: the same sweeps over the byte volume (l.cost8), two scanlines per warp, the first phase
+// writing one byte per voxel and direction (Dp bytes per pixel): where every quantised cost is below
+// 255, the largest P2 at most 255 and Dp at most 256.  nin is 3 or 7 (every direction of the first
+// phase); bands as above with nin 3 and sgm8_carry_words(w, Dp) words in `carry`.
+bool sgm8_supported(int Dp, const SgmPen& pen);
+size_t sgm8_carry_words(int w, int Dp);
+cudaError_t launch_sgm8_first(const SgmLaunch& l, int ndir, const int (*dirs)[2], uint8_t* const* out, cudaStream_t s);
+cudaError_t launch_sgm8_last(const SgmLaunch& l, int dx, int dy, int nin, const uint8_t* const* in, cudaStream_t s);
+cudaError_t launch_sgm8_last_band(const SgmLaunch& l, int dx, int dy, int nin, const uint8_t* const* in, int t_begin,
+                                  int t_end, uint32_t* carry, cudaStream_t s);
 // bufs[0] += bufs[1..6] (saturating u16 lanes), `words` 32-bit words each.
 // Path8: adds bufs[1 .. nbuf) into bufs[0] (nbuf 5 or 7), saturating per halfword.
 cudaError_t launch_sgm_fold(uint32_t* const* bufs, int nbuf, size_t words, cudaStream_t s);

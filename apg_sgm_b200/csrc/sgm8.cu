@@ -1,0 +1,733 @@
+// Semi-global matching sweeps over the byte volume, two scanlines per warp.
+//
+// Restates the recurrence of sgm.cu (SgmOptimizer::process_pixel, src/sgm_optimizer.cpp:44-80, and
+// wta_impl, :436-555) for configurations whose quantised costs stay below 255 and whose largest P2
+// is at most 255 (every preset), at up to 256 padded disparities:
+//   * the volume holds one byte per voxel (0xFF invalid);
+//   * with the path value L(d) = C(d) + delta(d), delta(d) = min(L'(d), L'(d-1) + P1, L'(d+1) + P1,
+//     m' + P2) - m' lies in [0, P2].  The sweeps of the first phase store delta, one byte per voxel
+//     and direction, instead of the 16-bit path value; the sum over n directions is n * C + the sum
+//     of the deltas, exactly.  The sums leave the device only through the WTA (and stage dumps).
+//     Per voxel the first phase moves 2 bytes a direction where 16-bit path values over a 16-bit
+//     volume took 4, the last sweep 1 + (n - 1) where it took 2 n, and eight directions need no fold;
+//   * a warp runs two neighbouring scanlines of one direction: a 32-bit word holds the path values
+//     of one disparity, scanline A's in the low half and scanline B's in the high half.  Neighbouring
+//     disparities are neighbouring words, so the recurrence needs no byte permutes and one shuffle
+//     each way serves both scanlines; widening bytes to halves costs 1.5 operations a word, which
+//     interleaves the scanlines at the same time;
+//   * per word: t = min(L'(d-1), L'(d+1)); x = min(t + P1, L'(d)); delta = min(x - m', P2);
+//     L = C + delta: three DPX / SIMD minima and one 32-bit add.  m' enters last, so the warp's two
+//     min-reductions run beside the neighbour shuffles and the first two minima.
+// Values: valid costs are at most 254 and valid path values at most 254 + 255.  An invalid cost is
+// widened to at least 0x0F00, above any candidate min' + P2, so an invalid neighbour never wins; all
+// halves stay below 0x2000, so plain 32-bit adds never carry between them and the signed minima are
+// exact.  A pixel whose predecessor has no valid entry (m' >= 0x0800) takes L = C: P2 reads as 0
+// there, which makes every delta 0; the first pixel of a scanline does the same with L' = 0.
+//
+// Steps whose pixels have every disparity of the range valid (default ranges: x >= dmax - 1) skip the
+// invalid-byte test: only the padded disparities are invalid there, a constant mask per lane.
+//
+// Loads run PF steps ahead through a per-warp shared-memory ring of cp.async groups, 16 bytes per
+// lane: one copy instruction brings both scanlines' costs of a step (two at 128 padded disparities
+// with three partial sums).  Bound: HBM for full frames, else each step's dependent chain (reduction,
+// two minima, add; about 60 cycles).
+#include "sgm8.cuh"
+
+#include <algorithm>
+#include <cstring>
+#include <vector>
+
+namespace apgcu {
+
+namespace {
+
+constexpr int kMaxIn = 7;                   // first-phase directions of Path8
+// Halves of a path-value word: kBias + L.  The bias keeps a low half above zero, so that one 32-bit
+// subtraction negates both halves (n = 0x10000 - acc, exact in each half modulo 2^16).
+constexpr uint32_t kBias = 0x0400u;
+constexpr uint32_t kBias2 = 0x04000400u;
+constexpr uint32_t kPad2 = 0x07000700u;     // bias and the invalid marker 0x0300 (with the byte 0xFF: 0x03FF)
+constexpr uint32_t kEdge2 = 0x0FFF0FFFu;    // beyond the ends of the range: above every path value
+// A max-reduction of negated minima holds -(kBias + m') in its high half; below this m' is invalid.
+constexpr uint32_t kNoPred = (0x10000u - kBias - 0x0300u) << 16;
+constexpr uint32_t kFresh = (0x10000u - kBias) << 16;  // m' = 0
+
+struct Args8 {
+    int w, h, d0, D, dmax;
+    int def_ranges;  // every pixel has the default range
+    SgmPen pen;
+    const uint8_t* gray;
+    const uint8_t* vol;
+    WtaOut wta;
+    uint32_t* sum;  // final sums (u16, 0xFFFF invalid) for stage dumps, or null
+    int t_begin, t_end;
+    uint32_t* carry;
+};
+struct Dirs8 {
+    int n;
+    int dx[kMaxIn], dy[kMaxIn], nscan[kMaxIn];
+    int warp_begin[kMaxIn + 1];
+    uint8_t* out[kMaxIn];
+};
+struct In8 {
+    const uint8_t* d[kMaxIn];
+};
+
+// W disparities per lane, AL lanes with disparities, CH 16-byte chunks per pixel.
+template <int DP>
+struct Geo {
+    static constexpr int W = DP == 64 ? 2 : (DP == 128 ? 4 : 8);
+    static constexpr int AL = DP / W;
+    static constexpr int CH = DP / 16;
+    static constexpr int SPI = 32 / (2 * CH);  // steps (both scanlines) per 16-byte copy instruction
+    static constexpr int RS = DP / 2 + 4;  // words per row of the WTA buffer: 4 mod 32, so 16-byte accesses
+                                           // of eight rows fall in distinct banks
+    static constexpr int wta_words = 32 * RS;
+};
+constexpr int kTail = 64;  // bytes behind a ring: idle lanes (192 padded disparities) read past a slot
+constexpr int kG = 4;      // steps per group: one cp.async group, waited for once and read together
+
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) { return __byte_perm(a, b, sel); }
+
+__device__ __forceinline__ void cp16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+// This lane's words of one pixel of both scanlines (A's slice at a, B's DP bytes on).
+template <int DP>
+struct Raw {
+    static constexpr int N = Geo<DP>::W >= 8 ? 2 : 1;
+    uint32_t a[N], b[N];
+};
+template <int DP>
+__device__ __forceinline__ Raw<DP> load_raw(const uint8_t* p) {
+    Raw<DP> r;
+    if constexpr (Geo<DP>::W == 2) {
+        r.a[0] = *reinterpret_cast<const uint16_t*>(p);
+        r.b[0] = *reinterpret_cast<const uint16_t*>(p + DP);
+    } else if constexpr (Geo<DP>::W == 4) {
+        r.a[0] = *reinterpret_cast<const uint32_t*>(p);
+        r.b[0] = *reinterpret_cast<const uint32_t*>(p + DP);
+    } else {
+        const uint2 va = *reinterpret_cast<const uint2*>(p), vb = *reinterpret_cast<const uint2*>(p + DP);
+        r.a[0] = va.x; r.a[1] = va.y;
+        r.b[0] = vb.x; r.b[1] = vb.y;
+    }
+    return r;
+}
+// u[i]: bytes 2i, 2i + 1 of scanline A, then of scanline B.
+template <int DP>
+__device__ __forceinline__ void interleave(const Raw<DP>& r, uint32_t (&u)[Geo<DP>::W / 2]) {
+    u[0] = prmt(r.a[0], r.b[0], 0x5410);
+    if constexpr (Geo<DP>::W >= 4) u[1] = prmt(r.a[0], r.b[0], 0x7632);
+    if constexpr (Geo<DP>::W == 8) {
+        u[2] = prmt(r.a[1], r.b[1], 0x5410);
+        u[3] = prmt(r.a[1], r.b[1], 0x7632);
+    }
+}
+
+// State of a warp's two chains: path values, the neighbouring lanes' words (shuffled as soon as a step
+// has its values, so the shuffles and the reductions run under the next step's loads), and the
+// reductions' results: -(kBias + m') in the high halves of lo (A) and hi (B).
+template <int W>
+struct Chain {
+    uint32_t L[W];
+    uint32_t up, dn, lo, hi;
+};
+
+template <int W>
+__device__ __forceinline__ void chain_reduce(Chain<W>& s) {
+    s.up = __shfl_up_sync(0xffffffffu, s.L[W - 1], 1);
+    s.dn = __shfl_down_sync(0xffffffffu, s.L[0], 1);
+    uint32_t acc = s.L[0];
+#pragma unroll
+    for (int k = 1; k + 1 < W; k += 2) acc = __vimin3_s16x2(acc, s.L[k], s.L[k + 1]);
+    acc = __vmins2(acc, s.L[W - 1]);
+    const uint32_t n = 0x00010000u - acc;
+    s.lo = __reduce_max_sync(0xffffffffu, n << 16);
+    s.hi = __reduce_max_sync(0xffffffffu, n);
+}
+template <int W>
+__device__ __forceinline__ void chain_init(Chain<W>& s) {
+#pragma unroll
+    for (int k = 0; k < W; ++k) s.L[k] = kBias2;
+    s.up = s.dn = kBias2;
+    s.lo = s.hi = kFresh;
+}
+
+// One step of both chains: r (the volume's bytes), p2 (A | B << 16) -> the deltas.  pad[k]: kPad2 for
+// words past the range, else kBias2.  c receives the widened, biased costs.
+template <int DP, bool CLEAN>
+__device__ __forceinline__ void path_step(Chain<Geo<DP>::W>& s, const Raw<DP>& r, const uint32_t (&pad)[Geo<DP>::W],
+                                          uint32_t p1x2, uint32_t p2, int lane, uint32_t (&c)[Geo<DP>::W],
+                                          uint32_t (&dl)[Geo<DP>::W]) {
+    constexpr int W = Geo<DP>::W;
+    uint32_t u[W / 2];
+    interleave<DP>(r, u);
+#pragma unroll
+    for (int i = 0; i < W / 2; ++i) {
+        c[2 * i] = (u[i] & 0x00FF00FFu) | pad[2 * i];
+        c[2 * i + 1] = prmt(u[i], pad[2 * i + 1], 0x7351);
+    }
+    if constexpr (!CLEAN) {
+#pragma unroll
+        for (int k = 0; k < W; ++k) {
+            const uint32_t inv = (c[k] + 0x00010001u) & 0x01000100u;  // 0x100 where the byte is 0xFF
+            c[k] += inv * 3u;                                          // 0xFF -> 0x03FF
+        }
+        p2 &= (s.lo > kNoPred ? 0x0000FFFFu : 0u) | (s.hi > kNoPred ? 0xFFFF0000u : 0u);
+    }
+    const uint32_t up = lane == 0 ? kEdge2 : s.up;
+    const uint32_t dn = lane == Geo<DP>::AL - 1 ? kEdge2 : s.dn;
+    const uint32_t nm = prmt(s.lo, s.hi, 0x7632);
+    uint32_t Ln[W];
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+        const uint32_t t = __vmins2(k == 0 ? up : s.L[k - 1], k == W - 1 ? dn : s.L[k + 1]);
+        const uint32_t x = __viaddmin_s16x2(t, p1x2, s.L[k]);
+        dl[k] = __viaddmin_s16x2(x, nm, p2);
+        Ln[k] = c[k] + dl[k];
+    }
+#pragma unroll
+    for (int k = 0; k < W; ++k) s.L[k] = Ln[k];
+    chain_reduce(s);
+}
+
+// First pixel and length of scanline s (0 when s is past the last one).
+__device__ __forceinline__ void scan_start8(int w, int h, int dx, int dy, int s, int nscan, int& x, int& y, int& len) {
+    x = 0; y = 0; len = 0;
+    if (s >= nscan) return;
+    if (dy == 0) {
+        y = s; x = dx > 0 ? 0 : w - 1; len = w;
+    } else if (dx == 0) {
+        x = s; y = dy > 0 ? 0 : h - 1; len = h;
+    } else {
+        // ray s: start pixel whose predecessor (x - dx, y - dy) is outside the image (the reference's
+        // ray enumeration, src/sgm_optimizer.cpp:325-365)
+        if (s < w) { x = s; y = dy > 0 ? 0 : h - 1; }
+        else { x = dx > 0 ? 0 : w - 1; y = dy > 0 ? (s - w + 1) : (h - 1 - (s - w + 1)); }
+        const int rx = dx > 0 ? w - x : x + 1;
+        const int ry = dy > 0 ? h - y : y + 1;
+        len = rx < ry ? rx : ry;
+    }
+}
+
+// The two scanlines of a warp: their geometry, and the P2 of 32 steps at a time (lane j: step t0 + j).
+struct Pair {
+    int xA, pA, lenA, xB, pB, lenB, step, maxlen, minlen;
+};
+__device__ __forceinline__ Pair pair_start(const Args8& a, int dx, int dy, int s, int nscan) {
+    Pair q;
+    int y;
+    scan_start8(a.w, a.h, dx, dy, s, nscan, q.xA, y, q.lenA);
+    q.pA = y * a.w + q.xA;
+    // an odd last scanline runs as both halves of its warp (the same values, stored twice)
+    scan_start8(a.w, a.h, dx, dy, s + 1 < nscan ? s + 1 : s, nscan, q.xB, y, q.lenB);
+    q.pB = y * a.w + q.xB;
+    q.step = dy * a.w + dx;
+    q.maxlen = max(q.lenA, q.lenB);
+    q.minlen = min(q.lenA, q.lenB);
+    return q;
+}
+struct GrayRun {
+    int nextA, nextB, carryA, carryB;
+};
+__device__ __forceinline__ void gray_init(const Args8& a, const Pair& q, int tb, int lane, GrayRun& g) {
+    const int t = tb + lane;
+    g.nextA = t < q.lenA ? (int)__ldg(a.gray + q.pA + t * q.step) : 0;
+    g.nextB = t < q.lenB ? (int)__ldg(a.gray + q.pB + t * q.step) : 0;
+    g.carryA = tb > 0 && tb <= q.lenA ? (int)__ldg(a.gray + q.pA + (tb - 1) * q.step) : 0;
+    g.carryB = tb > 0 && tb <= q.lenB ? (int)__ldg(a.gray + q.pB + (tb - 1) * q.step) : 0;
+}
+__device__ __forceinline__ uint32_t p2_block(const Args8& a, const Pair& q, int t0, int lane, GrayRun& g) {
+    const int gA = g.nextA, gB = g.nextB;
+    const int tn = t0 + 32 + lane;
+    g.nextA = tn < q.lenA ? (int)__ldg(a.gray + q.pA + tn * q.step) : 0;
+    g.nextB = tn < q.lenB ? (int)__ldg(a.gray + q.pB + tn * q.step) : 0;
+    int prA = __shfl_up_sync(0xffffffffu, gA, 1), prB = __shfl_up_sync(0xffffffffu, gB, 1);
+    if (lane == 0) { prA = g.carryA; prB = g.carryB; }
+    g.carryA = __shfl_sync(0xffffffffu, gA, 31);
+    g.carryB = __shfl_sync(0xffffffffu, gB, 31);
+    // a scanline's first pixel: P2 = 0 (with L' = 0, every delta is 0)
+    if (t0 + lane == 0) return 0;
+    return (uint32_t)adaptive_p2(a.pen, gA - prA) | ((uint32_t)adaptive_p2(a.pen, gB - prB) << 16);
+}
+// Every disparity of the range is valid for every pixel of the steps [t0, t0 + 32) (default ranges:
+// d0 <= d < min(dmax, x + 1), x - d < w).
+__device__ __forceinline__ bool clean_block(const Args8& a, const Pair& q, int dx, int t0) {
+    const int xa = q.xA + t0 * dx, xb = q.xB + t0 * dx, xe = 31 * dx;
+    const int lo = min(xa, xb) + min(xe, 0), hi = max(xa, xb) + max(xe, 0);
+    return a.def_ranges && lo >= a.dmax - 1 && hi <= a.w - 1 + min(a.d0, 0);
+}
+
+template <int DP>
+__device__ __forceinline__ void pad_words(const Args8& a, int lane, uint32_t (&pad)[Geo<DP>::W]) {
+    constexpr int W = Geo<DP>::W;
+#pragma unroll
+    for (int k = 0; k < W; ++k) pad[k] = lane * W + k >= a.D ? kPad2 : kBias2;
+}
+
+// Copies of whole groups into a ring of NG groups of kG steps, `narr` arrays of equal shape per step
+// (slot layout: [array][A, B][DP]): lane l brings 16 bytes, of step `sub` of its copy instruction.
+template <int DP>
+struct Copier {
+    using G = Geo<DP>;
+    int sub, mylen, it;
+    int64_t bstep, off;  // byte step of a pixel step; byte offset of the lane's next chunk in every array
+    __device__ __forceinline__ void init(const Pair& q, int tb, int lane) {
+        sub = lane / (2 * G::CH);
+        const int r = lane - sub * (2 * G::CH);
+        const bool isB = r >= G::CH;
+        mylen = sub < G::SPI ? (isB ? q.lenB : q.lenA) : 0;
+        bstep = (int64_t)q.step * DP;
+        off = (int64_t)(isB ? q.pB : q.pA) * DP + (tb + sub) * bstep + (isB ? r - G::CH : r) * 16;
+        it = tb;
+    }
+    // dst: the slot of the group's first step plus this lane's place (place()); SLOT: bytes per step
+    template <int SLOT, int NARR, typename BASE>
+    __device__ __forceinline__ void group(uint8_t* dst, BASE base) {
+#pragma unroll
+        for (int i = 0; i < kG; i += G::SPI) {
+            if (it + i + sub < mylen) {
+#pragma unroll
+                for (int b = 0; b < NARR; ++b) cp16(dst + i * SLOT + b * 2 * DP, base(b) + off);
+            }
+            off += G::SPI * bstep;
+        }
+        it += kG;
+        cp_commit();
+    }
+    template <int SLOT>
+    __device__ __forceinline__ static int place(int lane) {
+        return lane / (2 * G::CH) * SLOT + lane % (2 * G::CH) * 16;
+    }
+};
+
+template <int DP>
+__device__ __forceinline__ void store_deltas(uint8_t* base, uint32_t oa, uint32_t ob, bool doA, bool doB,
+                                             const uint32_t (&dl)[Geo<DP>::W]) {
+    constexpr int W = Geo<DP>::W;
+    uint32_t u[W / 2];
+#pragma unroll
+    for (int i = 0; i < W / 2; ++i) u[i] = dl[2 * i + 1] * 256u + dl[2 * i];
+    if constexpr (W == 2) {
+        if (doA) *reinterpret_cast<uint16_t*>(base + oa) = (uint16_t)u[0];
+        if (doB) *reinterpret_cast<uint16_t*>(base + ob) = (uint16_t)(u[0] >> 16);
+    } else if constexpr (W == 4) {
+        if (doA) *reinterpret_cast<uint32_t*>(base + oa) = prmt(u[0], u[1], 0x5410);
+        if (doB) *reinterpret_cast<uint32_t*>(base + ob) = prmt(u[0], u[1], 0x7632);
+    } else {
+        if (doA) *reinterpret_cast<uint2*>(base + oa) = make_uint2(prmt(u[0], u[1], 0x5410), prmt(u[2], u[3], 0x5410));
+        if (doB) *reinterpret_cast<uint2*>(base + ob) = make_uint2(prmt(u[0], u[1], 0x7632), prmt(u[2], u[3], 0x7632));
+    }
+}
+
+// ---- first phase: one warp, scanlines s and s + 1 of direction (dx, dy), deltas to `out`
+template <int DP>
+__host__ __device__ constexpr int first_groups() { return DP >= 192 ? 4 : 8; }  // ring depth in groups
+template <int DP>
+__host__ __device__ constexpr int first_bytes() { return first_groups<DP>() * kG * 2 * DP + kTail; }
+
+template <int DP>
+__device__ __forceinline__ void run_first8(const Args8& a, uint8_t* ring, int dx, int dy, int s, int nscan,
+                                           uint8_t* out) {
+    using G = Geo<DP>;
+    constexpr int W = G::W, SLOT = 2 * DP, NG = first_groups<DP>();
+    const int lane = threadIdx.x & 31;
+    const Pair q = pair_start(a, dx, dy, s, nscan);
+    if (q.maxlen == 0) return;
+    Copier<DP> cp;
+    cp.init(q, 0, lane);
+    uint8_t* dst = ring + Copier<DP>::template place<SLOT>(lane);
+    auto base = [&](int) { return a.vol; };
+#pragma unroll
+    for (int t = 0; t < NG - 1; ++t) cp.template group<SLOT, 1>(dst + t * kG * SLOT, base);
+    uint32_t pad[W];
+    pad_words<DP>(a, lane, pad);
+    Chain<W> st;
+    chain_init(st);
+    GrayRun g;
+    gray_init(a, q, 0, lane, g);
+    const uint32_t p1x2 = (uint32_t)a.pen.P1 * 0x00010001u;
+    const uint8_t* rd = ring + lane * W;
+    // 32-bit byte offsets (the host checks the volume's size)
+    uint32_t oa = (uint32_t)q.pA * DP + lane * W, ob = (uint32_t)q.pB * DP + lane * W;
+    const uint32_t ostep = (uint32_t)(q.step * DP);
+    const bool act = G::AL == 32 || lane < G::AL;
+    int slot = 0;
+    auto groups = [&](auto clean, auto full, int t0, uint32_t p2v) {
+#pragma unroll 1
+        for (int u0 = 0; u0 < 32; u0 += kG) {
+            const int tb = t0 + u0;
+            if (!decltype(full)::value && tb >= q.maxlen) break;
+            cp_wait<NG - 2>();
+            __syncwarp();
+            cp.template group<SLOT, 1>(dst + (slot == 0 ? NG - 1 : slot - 1) * (kG * SLOT), base);
+            const uint8_t* sl = rd + slot * (kG * SLOT);
+            Raw<DP> raw[kG];
+            uint32_t p2[kG];
+#pragma unroll
+            for (int v = 0; v < kG; ++v) {
+                raw[v] = load_raw<DP>(sl + v * SLOT);
+                p2[v] = __shfl_sync(0xffffffffu, p2v, u0 + v);
+            }
+#pragma unroll
+            for (int v = 0; v < kG; ++v) {
+                uint32_t c[W], dl[W];
+                path_step<DP, decltype(clean)::value>(st, raw[v], pad, p1x2, p2[v], lane, c, dl);
+                if (decltype(full)::value) store_deltas<DP>(out, oa, ob, act, act, dl);
+                else store_deltas<DP>(out, oa, ob, act && tb + v < q.lenA, act && tb + v < q.lenB, dl);
+                oa += ostep;
+                ob += ostep;
+            }
+            slot = slot == NG - 1 ? 0 : slot + 1;
+        }
+    };
+    for (int t0 = 0; t0 < q.maxlen; t0 += 32) {
+        const uint32_t p2v = p2_block(a, q, t0, lane, g);
+        if (t0 + 32 > q.minlen) groups(std::false_type(), std::false_type(), t0, p2v);
+        else if (clean_block(a, q, dx, t0)) groups(std::true_type(), std::true_type(), t0, p2v);
+        else groups(std::false_type(), std::true_type(), t0, p2v);
+    }
+    cp_wait<0>();
+    __syncwarp();
+}
+
+// ---- last sweep: the sums n * C + deltas of NIN first-phase directions and of this sweep, the WTA
+//
+// PS: two deltas of one voxel fit a byte, so two arrays are added before they are widened.
+template <int NIN>
+__host__ __device__ constexpr uint32_t sum_bias() { return kBias * (NIN + 1); }
+template <int NIN>
+__host__ __device__ constexpr uint32_t sum_inf() { return (kBias + 0x0300u) * (NIN + 1); }
+
+// sum[] += the deltas of NIN arrays at sl (layout [array][A, B][DP]).
+template <int DP, int NIN, bool PS>
+__device__ __forceinline__ void add_deltas(const uint8_t* sl, uint32_t (&sum)[Geo<DP>::W]) {
+    constexpr int W = Geo<DP>::W;
+#pragma unroll
+    for (int b = 0; b < NIN;) {
+        Raw<DP> r = load_raw<DP>(sl + b * 2 * DP);
+        ++b;
+        if (PS && b < NIN) {
+            const Raw<DP> r2 = load_raw<DP>(sl + b * 2 * DP);
+#pragma unroll
+            for (int i = 0; i < Raw<DP>::N; ++i) {
+                r.a[i] += r2.a[i];
+                r.b[i] += r2.b[i];
+            }
+            ++b;
+        }
+        uint32_t e[W / 2];
+        interleave<DP>(r, e);
+#pragma unroll
+        for (int i = 0; i < W / 2; ++i) {
+            sum[2 * i] += e[i] & 0x00FF00FFu;
+            sum[2 * i + 1] += prmt(e[i], 0u, 0x4341);
+        }
+    }
+}
+
+// The sums of one step into the WTA buffer: rows v (A) and 16 + v (B), two consecutive disparities a word.
+template <int DP, int NIN>
+__device__ __forceinline__ void put_sums(const Args8& a, const Pair& q, uint32_t* s_wta, int v, int t, int lane, bool act,
+                                         const uint32_t (&sum)[Geo<DP>::W]) {
+    using G = Geo<DP>;
+    constexpr int W = G::W;
+    if (!act) return;
+    uint32_t* wa = s_wta + v * G::RS + lane * (W / 2);
+    uint32_t* wb = wa + 16 * G::RS;
+    uint32_t oa[W / 2], ob[W / 2];
+#pragma unroll
+    for (int i = 0; i < W / 2; ++i) {
+        oa[i] = prmt(sum[2 * i], sum[2 * i + 1], 0x5410);
+        ob[i] = prmt(sum[2 * i], sum[2 * i + 1], 0x7632);
+    }
+    if constexpr (W == 2) {
+        wa[0] = oa[0];
+        wb[0] = ob[0];
+    } else if constexpr (W == 4) {
+        *reinterpret_cast<uint2*>(wa) = make_uint2(oa[0], oa[1]);
+        *reinterpret_cast<uint2*>(wb) = make_uint2(ob[0], ob[1]);
+    } else {
+        *reinterpret_cast<uint4*>(wa) = make_uint4(oa[0], oa[1], oa[2], oa[3]);
+        *reinterpret_cast<uint4*>(wb) = make_uint4(ob[0], ob[1], ob[2], ob[3]);
+    }
+    if (a.sum) {
+        constexpr uint32_t inf = sum_inf<NIN>() * 0x00010001u, bias = sum_bias<NIN>() * 0x00010001u;
+#pragma unroll
+        for (int i = 0; i < W / 2; ++i) {
+            const size_t o = (size_t)lane * (W / 2) + i;
+            if (t < q.lenA)
+                a.sum[(size_t)(q.pA + t * q.step) * (DP / 2) + o] = (oa[i] - bias) | __vcmpgeu2(oa[i], inf);
+            if (t < q.lenB)
+                a.sum[(size_t)(q.pB + t * q.step) * (DP / 2) + o] = (ob[i] - bias) | __vcmpgeu2(ob[i], inf);
+        }
+    }
+}
+
+// The WTA of the block of 16 steps at tb: lane l takes step tb + l % 16 of scanline A (l < 16) or B.
+template <int DP, int NIN>
+__device__ __forceinline__ void wta_block(const Args8& a, const Pair& q, const uint32_t* s_wta, int tb, int lane) {
+    const int t = tb + (lane & 15);
+    const bool b = lane >= 16;
+    if (t < (b ? q.lenB : q.lenA))
+        wta_row<DP / 2, sum_inf<NIN>(), sum_bias<NIN>()>(a.wta, a.d0, a.D, s_wta + lane * Geo<DP>::RS,
+                                                         (b ? q.pB : q.pA) + t * q.step);
+}
+
+// Bands of steps [t_begin, t_end): the chains' path values enter and leave through a.carry.
+template <int DP>
+__device__ __forceinline__ bool band_limits(const Args8& a, Pair& q, int& tb0) {
+    tb0 = a.t_begin;
+    const bool carry_out = a.t_end < q.maxlen;
+    q.lenA = min(q.lenA, a.t_end);
+    q.lenB = min(q.lenB, a.t_end);
+    q.maxlen = min(q.maxlen, a.t_end);
+    q.minlen = min(q.minlen, a.t_end);
+    return carry_out;
+}
+template <int DP>
+__device__ __forceinline__ void band_load(const Args8& a, int s, int lane, Chain<Geo<DP>::W>& st) {
+    const uint32_t* cs = a.carry + (size_t)(s >> 1) * Geo<DP>::W * 32 + lane;
+#pragma unroll
+    for (int k = 0; k < Geo<DP>::W; ++k) st.L[k] = __ldcg(cs + k * 32);
+    chain_reduce(st);
+}
+template <int DP>
+__device__ __forceinline__ void band_store(const Args8& a, int s, int lane, const Chain<Geo<DP>::W>& st) {
+    uint32_t* cs = a.carry + (size_t)(s >> 1) * Geo<DP>::W * 32 + lane;
+#pragma unroll
+    for (int k = 0; k < Geo<DP>::W; ++k) __stcg(cs + k * 32, st.L[k]);
+}
+
+// One warp per pair of scanlines.
+template <int DP, int NIN, int NG>
+__host__ __device__ constexpr int last_bytes() {
+    return Geo<DP>::wta_words * 4 + NG * kG * (1 + NIN) * 2 * DP + kTail;
+}
+template <int DP, int NIN, int NG, bool PS, bool BAND>
+__device__ __forceinline__ void run_last8(const Args8& a, const uint8_t* const* in, uint8_t* smem, int dx, int dy, int s,
+                                          int nscan) {
+    using G = Geo<DP>;
+    constexpr int W = G::W, NARR = 1 + NIN, SLOT = NARR * 2 * DP;
+    uint32_t* s_wta = reinterpret_cast<uint32_t*>(smem);
+    uint8_t* ring = smem + G::wta_words * 4;
+    const int lane = threadIdx.x & 31;
+    Pair q = pair_start(a, dx, dy, s, nscan);
+    int tb0 = 0;
+    bool carry_out = false;
+    if constexpr (BAND) carry_out = band_limits<DP>(a, q, tb0);
+    if (q.maxlen <= tb0) return;
+    Copier<DP> cp;
+    cp.init(q, tb0, lane);
+    uint8_t* dst = ring + Copier<DP>::template place<SLOT>(lane);
+    auto base = [&](int b) { return b == 0 ? a.vol : in[b - 1]; };
+#pragma unroll
+    for (int t = 0; t < NG - 1; ++t) cp.template group<SLOT, NARR>(dst + t * kG * SLOT, base);
+    uint32_t pad[W];
+    pad_words<DP>(a, lane, pad);
+    Chain<W> st;
+    chain_init(st);
+    if constexpr (BAND)
+        if (tb0 > 0) band_load<DP>(a, s, lane, st);
+    GrayRun g;
+    gray_init(a, q, tb0, lane, g);
+    const uint32_t p1x2 = (uint32_t)a.pen.P1 * 0x00010001u;
+    const uint8_t* rd = ring + lane * W;
+    const bool act = G::AL == 32 || lane < G::AL;
+    int slot = 0;
+    auto groups = [&](auto clean, int t0, uint32_t p2v) {
+#pragma unroll 1
+        for (int u0 = 0; u0 < 32; u0 += kG) {
+            const int tb = t0 + u0;
+            if (tb >= q.maxlen) break;
+            cp_wait<NG - 2>();
+            __syncwarp();
+            cp.template group<SLOT, NARR>(dst + (slot == 0 ? NG - 1 : slot - 1) * (kG * SLOT), base);
+            const uint8_t* sl = rd + slot * (kG * SLOT);
+            Raw<DP> raw[kG];
+            uint32_t p2[kG];
+#pragma unroll
+            for (int v = 0; v < kG; ++v) {
+                raw[v] = load_raw<DP>(sl + v * SLOT);
+                p2[v] = __shfl_sync(0xffffffffu, p2v, u0 + v);
+            }
+#pragma unroll
+            for (int v = 0; v < kG; ++v) {
+                uint32_t c[W], dl[W], sum[W];
+                path_step<DP, decltype(clean)::value>(st, raw[v], pad, p1x2, p2[v], lane, c, dl);
+#pragma unroll
+                for (int k = 0; k < W; ++k) sum[k] = c[k] * (uint32_t)(NIN + 1) + dl[k];
+                add_deltas<DP, NIN, PS>(sl + v * SLOT + 2 * DP, sum);
+                put_sums<DP, NIN>(a, q, s_wta, (u0 + v) & 15, tb + v, lane, act, sum);
+            }
+            slot = slot == NG - 1 ? 0 : slot + 1;
+            if ((u0 & 15) == 12 || tb + kG >= q.maxlen) {
+                __syncwarp();
+                wta_block<DP, NIN>(a, q, s_wta, t0 + (u0 & 16), lane);
+                __syncwarp();
+            }
+        }
+    };
+    for (int t0 = tb0; t0 < q.maxlen; t0 += 32) {
+        const uint32_t p2v = p2_block(a, q, t0, lane, g);
+        if (clean_block(a, q, dx, t0)) groups(std::true_type(), t0, p2v);
+        else groups(std::false_type(), t0, p2v);
+    }
+    if constexpr (BAND)
+        if (carry_out) band_store<DP>(a, s, lane, st);
+    cp_wait<0>();
+    __syncwarp();
+}
+
+// One warp per block: chains of different lengths end independently.
+template <int DP>
+__global__ void __launch_bounds__(32) sgm8_first_kernel(Args8 a, Dirs8 tab) {
+    extern __shared__ __align__(16) uint8_t s8[];
+    int d = 0;
+#pragma unroll
+    for (int i = 1; i < kMaxIn; ++i)
+        if (i < tab.n && (int)blockIdx.x >= tab.warp_begin[i]) d = i;
+    const int s = 2 * ((int)blockIdx.x - tab.warp_begin[d]);
+    run_first8<DP>(a, s8, tab.dx[d], tab.dy[d], s, tab.nscan[d], tab.out[d]);
+}
+
+template <int DP, int NIN, int NG, bool PS, bool BAND>
+__global__ void __launch_bounds__(32) sgm8_last_kernel(Args8 a, In8 in, int dx, int dy, int nscan) {
+    extern __shared__ __align__(16) uint8_t s8[];
+    run_last8<DP, NIN, NG, PS, BAND>(a, in.d, s8, dx, dy, 2 * (int)blockIdx.x, nscan);
+}
+
+int nscan8(int w, int h, int dx, int dy) { return dy == 0 ? h : (dx == 0 ? w : w + h - 1); }
+
+Args8 make_args8(const SgmLaunch& l) {
+    Args8 a{};
+    a.w = l.w; a.h = l.h; a.d0 = l.d0; a.D = l.D; a.dmax = l.d0 + l.D;
+    a.def_ranges = l.default_ranges;
+    a.pen = l.pen;
+    a.gray = l.gray;
+    a.vol = reinterpret_cast<const uint8_t*>(l.cvol);
+    a.wta = WtaOut{l.disp, l.best, l.second, l.subpixel, l.sp_method, l.sp_param, l.sp_tel};
+    a.sum = l.sum;
+    a.t_begin = 0;
+    a.t_end = 0x7FFFFFFF;
+    return a;
+}
+
+// Shared memory of a one-warp block, rounded up so that an SM takes no more than its even share of the
+// launch's blocks (at least `least`).  Every chain of a launch is resident at once, so where a block
+// lands decides how many chains its SM steps: without the cap, blocks placed while another stream's
+// kernel (the right-image finalize) still held most SMs crowded onto the others (Fast 1280x720 D128
+// SHARE_FIGURES).
+size_t even_share(int blocks, size_t need, int least) {
+    int dev = 0, nsm = 0, per_sm = 0, reserved = 0, optin = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
+        cudaGetLastError();
+        return need;
+    }
+    const int share = std::max(least, (blocks + nsm - 1) / nsm);
+    const long long cap = std::min<long long>(per_sm / share - reserved, optin) / 128 * 128;
+    return std::max<long long>((long long)need, cap);
+}
+
+int max_p2(const SgmPen& p) { return p.P2_base > p.P1 + 1 ? p.P2_base : p.P1 + 1; }
+
+template <typename F>
+cudaError_t by_dp(int Dp, F f) {
+    switch (Dp) {
+        case 64: return f(std::integral_constant<int, 64>());
+        case 128: return f(std::integral_constant<int, 128>());
+        case 192: return f(std::integral_constant<int, 192>());
+        case 256: return f(std::integral_constant<int, 256>());
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+template <int DP, int NIN, int PF, bool PS, bool BAND>
+cudaError_t launch_last_t(const Args8& a, const In8& in, int dx, int dy, int nscan, cudaStream_t st) {
+    auto kern = sgm8_last_kernel<DP, NIN, PF, PS, BAND>;
+    const size_t smem = even_share((nscan + 1) / 2, last_bytes<DP, NIN, PF>(), 4);
+    const cudaError_t e = allow_dynamic_smem(kern, smem);
+    if (e != cudaSuccess) return e;
+    kern<<<(nscan + 1) / 2, 32, smem, st>>>(a, in, dx, dy, nscan);
+    return cudaGetLastError();
+}
+
+template <bool BAND>
+cudaError_t launch_last_any(const SgmLaunch& l, const Args8& a, int dx, int dy, int nin, const uint8_t* const* in,
+                            cudaStream_t st) {
+    if (nin != 3 && (nin != 7 || BAND)) return cudaErrorInvalidValue;
+    In8 t{};
+    for (int i = 0; i < nin; ++i) t.d[i] = in[i];
+    const int nscan = nscan8(l.w, l.h, dx, dy);
+    const bool ps = 2 * max_p2(l.pen) <= 255;
+    return by_dp(l.Dp, [&](auto dp) -> cudaError_t {
+        constexpr int DP = decltype(dp)::value;
+        constexpr int PF3 = DP == 256 ? 2 : 4;
+        if (nin == 3)
+            return ps ? launch_last_t<DP, 3, PF3, true, BAND>(a, t, dx, dy, nscan, st)
+                      : launch_last_t<DP, 3, PF3, false, BAND>(a, t, dx, dy, nscan, st);
+        if constexpr (!BAND) {
+            constexpr int PF7 = DP >= 192 ? 2 : 3;
+            return ps ? launch_last_t<DP, 7, PF7, true, false>(a, t, dx, dy, nscan, st)
+                      : launch_last_t<DP, 7, PF7, false, false>(a, t, dx, dy, nscan, st);
+        }
+        return cudaErrorInvalidValue;
+    });
+}
+
+}  // namespace
+
+bool sgm8_supported(int Dp, const SgmPen& pen) { return Dp <= 256 && Dp % 64 == 0 && max_p2(pen) <= 255; }
+
+size_t sgm8_carry_words(int w, int Dp) { return (size_t)((w + 1) / 2) * 32 * ((Dp >= 192 ? 8 : Dp / 32)); }
+
+cudaError_t launch_sgm8_first(const SgmLaunch& l, int ndir, const int (*dirs)[2], uint8_t* const* out,
+                              cudaStream_t st) {
+    if (ndir < 1 || ndir > kMaxIn || !sgm8_supported(l.Dp, l.pen)) return cudaErrorInvalidValue;
+    const Args8 a = make_args8(l);
+    Dirs8 tab{};
+    tab.n = ndir;
+    for (int i = 0; i < ndir; ++i) {
+        tab.dx[i] = dirs[i][0];
+        tab.dy[i] = dirs[i][1];
+        tab.out[i] = out[i];
+        tab.nscan[i] = nscan8(l.w, l.h, dirs[i][0], dirs[i][1]);
+        tab.warp_begin[i + 1] = tab.warp_begin[i] + (tab.nscan[i] + 1) / 2;
+    }
+    return by_dp(l.Dp, [&](auto dp) -> cudaError_t {
+        constexpr int DP = decltype(dp)::value;
+        const size_t smem = even_share(tab.warp_begin[ndir], first_bytes<DP>(), 8);
+        const cudaError_t e = allow_dynamic_smem(sgm8_first_kernel<DP>, smem);
+        if (e != cudaSuccess) return e;
+        sgm8_first_kernel<DP><<<tab.warp_begin[ndir], 32, smem, st>>>(a, tab);
+        return cudaGetLastError();
+    });
+}
+
+cudaError_t launch_sgm8_last(const SgmLaunch& l, int dx, int dy, int nin, const uint8_t* const* in, cudaStream_t st) {
+    if (!sgm8_supported(l.Dp, l.pen)) return cudaErrorInvalidValue;
+    return launch_last_any<false>(l, make_args8(l), dx, dy, nin, in, st);
+}
+
+cudaError_t launch_sgm8_last_band(const SgmLaunch& l, int dx, int dy, int nin, const uint8_t* const* in, int t_begin,
+                                  int t_end, uint32_t* carry, cudaStream_t st) {
+    if (!sgm8_supported(l.Dp, l.pen) || t_begin < 0 || (t_begin & 31) || t_end <= t_begin || !carry)
+        return cudaErrorInvalidValue;
+    Args8 a = make_args8(l);
+    a.t_begin = t_begin;
+    a.t_end = t_end;
+    a.carry = carry;
+    return launch_last_any<true>(l, a, dx, dy, nin, in, st);
+}
+
+}  // namespace apgcu
