@@ -55,7 +55,8 @@ constexpr uint32_t kFresh = (0x10000u - kBias) << 16;  // m' = 0
 struct Args8 {
     int w, h, d0, D, dmax;
     int def_ranges;  // every pixel has the default range
-    SgmPen pen;
+    int P1;
+    uint8_t p2[256];  // adaptive P2 by |gray difference|
     const uint8_t* gray;
     const uint8_t* vol;
     WtaOut wta;
@@ -85,7 +86,6 @@ struct Geo {
     static constexpr int wta_words = 32 * RS;
 };
 constexpr int kTail = 64;  // bytes behind a ring: idle lanes (192 padded disparities) read past a slot
-constexpr int kG = 4;      // steps per group: one cp.async group, waited for once and read together
 
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) { return __byte_perm(a, b, sel); }
 
@@ -136,13 +136,14 @@ __device__ __forceinline__ void interleave(const Raw<DP>& r, uint32_t (&u)[Geo<D
 template <int W>
 struct Chain {
     uint32_t L[W];
+    uint32_t q[W];  // L + P1
     uint32_t up, dn, lo, hi;
 };
 
 template <int W>
 __device__ __forceinline__ void chain_reduce(Chain<W>& s) {
-    s.up = __shfl_up_sync(0xffffffffu, s.L[W - 1], 1);
-    s.dn = __shfl_down_sync(0xffffffffu, s.L[0], 1);
+    s.up = __shfl_up_sync(0xffffffffu, s.q[W - 1], 1);
+    s.dn = __shfl_down_sync(0xffffffffu, s.q[0], 1);
     uint32_t acc = s.L[0];
 #pragma unroll
     for (int k = 1; k + 1 < W; k += 2) acc = __vimin3_s16x2(acc, s.L[k], s.L[k + 1]);
@@ -154,7 +155,7 @@ __device__ __forceinline__ void chain_reduce(Chain<W>& s) {
 template <int W>
 __device__ __forceinline__ void chain_init(Chain<W>& s) {
 #pragma unroll
-    for (int k = 0; k < W; ++k) s.L[k] = kBias2;
+    for (int k = 0; k < W; ++k) s.L[k] = s.q[k] = kBias2;
     s.up = s.dn = kBias2;
     s.lo = s.hi = kFresh;
 }
@@ -184,16 +185,16 @@ __device__ __forceinline__ void path_step(Chain<Geo<DP>::W>& s, const Raw<DP>& r
     const uint32_t up = lane == 0 ? kEdge2 : s.up;
     const uint32_t dn = lane == Geo<DP>::AL - 1 ? kEdge2 : s.dn;
     const uint32_t nm = prmt(s.lo, s.hi, 0x7632);
-    uint32_t Ln[W];
 #pragma unroll
     for (int k = 0; k < W; ++k) {
-        const uint32_t t = __vmins2(k == 0 ? up : s.L[k - 1], k == W - 1 ? dn : s.L[k + 1]);
-        const uint32_t x = __viaddmin_s16x2(t, p1x2, s.L[k]);
+        const uint32_t x = __vimin3_s16x2(k == 0 ? up : s.q[k - 1], k == W - 1 ? dn : s.q[k + 1], s.L[k]);
         dl[k] = __viaddmin_s16x2(x, nm, p2);
-        Ln[k] = c[k] + dl[k];
     }
 #pragma unroll
-    for (int k = 0; k < W; ++k) s.L[k] = Ln[k];
+    for (int k = 0; k < W; ++k) {
+        s.L[k] = c[k] + dl[k];
+        s.q[k] = s.L[k] + p1x2;
+    }
     chain_reduce(s);
 }
 
@@ -216,9 +217,10 @@ __device__ __forceinline__ void scan_start8(int w, int h, int dx, int dy, int s,
     }
 }
 
-// The two scanlines of a warp: their geometry, and the P2 of 32 steps at a time (lane j: step t0 + j).
+// The geometry of a warp's two scanlines.
 struct Pair {
     int xA, pA, lenA, xB, pB, lenB, step, maxlen, minlen;
+    int fullA, fullB;  // the scanlines' own lengths (a band cuts the others)
 };
 __device__ __forceinline__ Pair pair_start(const Args8& a, int dx, int dy, int s, int nscan) {
     Pair q;
@@ -231,30 +233,58 @@ __device__ __forceinline__ Pair pair_start(const Args8& a, int dx, int dy, int s
     q.step = dy * a.w + dx;
     q.maxlen = max(q.lenA, q.lenB);
     q.minlen = min(q.lenA, q.lenB);
+    q.fullA = q.lenA;
+    q.fullB = q.lenB;
     return q;
 }
+// P2 of a warp's steps, 32 at a time: lane j looks up step t0 + j of both scanlines (the grays prefetched
+// one block ahead, through clamped addresses: a select behind a load would wait for it) and leaves
+// P2(A) | P2(B) << 16 in shared memory, from where a group of steps reads its words together.
+struct P2Smem {
+    uint32_t w[32];
+    uint8_t lut[256];
+};
 struct GrayRun {
     int nextA, nextB, carryA, carryB;
 };
-__device__ __forceinline__ void gray_init(const Args8& a, const Pair& q, int tb, int lane, GrayRun& g) {
-    const int t = tb + lane;
-    g.nextA = t < q.lenA ? (int)__ldg(a.gray + q.pA + t * q.step) : 0;
-    g.nextB = t < q.lenB ? (int)__ldg(a.gray + q.pB + t * q.step) : 0;
-    g.carryA = tb > 0 && tb <= q.lenA ? (int)__ldg(a.gray + q.pA + (tb - 1) * q.step) : 0;
-    g.carryB = tb > 0 && tb <= q.lenB ? (int)__ldg(a.gray + q.pB + (tb - 1) * q.step) : 0;
+__device__ __forceinline__ void gray_load(const Args8& a, const Pair& q, int t, GrayRun& g) {
+    g.nextA = (int)__ldg(a.gray + q.pA + min(t, q.fullA - 1) * q.step);
+    g.nextB = (int)__ldg(a.gray + q.pB + min(t, q.fullB - 1) * q.step);
 }
-__device__ __forceinline__ uint32_t p2_block(const Args8& a, const Pair& q, int t0, int lane, GrayRun& g) {
+__device__ __forceinline__ void gray_init(const Args8& a, const Pair& q, int tb, int lane, P2Smem* sm, GrayRun& g) {
+    *reinterpret_cast<uint2*>(sm->lut + lane * 8) = *reinterpret_cast<const uint2*>(a.p2 + lane * 8);
+    gray_load(a, q, max(tb - 1, 0), g);
+    g.carryA = g.nextA;
+    g.carryB = g.nextB;
+    gray_load(a, q, tb + lane, g);
+}
+__device__ __forceinline__ void p2_block(const Args8& a, const Pair& q, int t0, int lane, P2Smem* sm, GrayRun& g) {
     const int gA = g.nextA, gB = g.nextB;
-    const int tn = t0 + 32 + lane;
-    g.nextA = tn < q.lenA ? (int)__ldg(a.gray + q.pA + tn * q.step) : 0;
-    g.nextB = tn < q.lenB ? (int)__ldg(a.gray + q.pB + tn * q.step) : 0;
+    gray_load(a, q, t0 + 32 + lane, g);
     int prA = __shfl_up_sync(0xffffffffu, gA, 1), prB = __shfl_up_sync(0xffffffffu, gB, 1);
     if (lane == 0) { prA = g.carryA; prB = g.carryB; }
     g.carryA = __shfl_sync(0xffffffffu, gA, 31);
     g.carryB = __shfl_sync(0xffffffffu, gB, 31);
+    __syncwarp();  // the last block's words are read (and, at first, the table is written)
+    uint32_t v = (uint32_t)sm->lut[abs(gA - prA)] | ((uint32_t)sm->lut[abs(gB - prB)] << 16);
     // a scanline's first pixel: P2 = 0 (with L' = 0, every delta is 0)
-    if (t0 + lane == 0) return 0;
-    return (uint32_t)adaptive_p2(a.pen, gA - prA) | ((uint32_t)adaptive_p2(a.pen, gB - prB) << 16);
+    if (t0 + lane == 0) v = 0;
+    sm->w[lane] = v;
+    __syncwarp();
+}
+// P2 of the KG steps from u0 (a multiple of KG) of the block.
+template <int KG>
+__device__ __forceinline__ void p2_group(const P2Smem* sm, int u0, uint32_t (&p2)[KG]) {
+    if constexpr (KG % 4 == 0) {
+#pragma unroll
+        for (int v = 0; v < KG; v += 4) {
+            const uint4 t = *reinterpret_cast<const uint4*>(sm->w + u0 + v);
+            p2[v] = t.x; p2[v + 1] = t.y; p2[v + 2] = t.z; p2[v + 3] = t.w;
+        }
+    } else {
+#pragma unroll
+        for (int v = 0; v < KG; ++v) p2[v] = sm->w[u0 + v];
+    }
 }
 // Every disparity of the range is valid for every pixel of the steps [t0, t0 + 32) (default ranges:
 // d0 <= d < min(dmax, x + 1), x - d < w).
@@ -271,7 +301,7 @@ __device__ __forceinline__ void pad_words(const Args8& a, int lane, uint32_t (&p
     for (int k = 0; k < W; ++k) pad[k] = lane * W + k >= a.D ? kPad2 : kBias2;
 }
 
-// Copies of whole groups into a ring of NG groups of kG steps, `narr` arrays of equal shape per step
+// Copies of whole groups into a ring of groups of KG steps, `narr` arrays of equal shape per step
 // (slot layout: [array][A, B][DP]): lane l brings 16 bytes, of step `sub` of its copy instruction.
 template <int DP>
 struct Copier {
@@ -288,17 +318,19 @@ struct Copier {
         it = tb;
     }
     // dst: the slot of the group's first step plus this lane's place (place()); SLOT: bytes per step
-    template <int SLOT, int NARR, typename BASE>
+    template <int SLOT, int NARR, int KG, typename BASE>
     __device__ __forceinline__ void group(uint8_t* dst, BASE base) {
+        // (a group shorter than a copy instruction's steps leaves its upper lanes idle)
+        constexpr int STEP = KG < G::SPI ? KG : G::SPI;
 #pragma unroll
-        for (int i = 0; i < kG; i += G::SPI) {
-            if (it + i + sub < mylen) {
+        for (int i = 0; i < KG; i += STEP) {
+            if (sub < STEP && it + i + sub < mylen) {
 #pragma unroll
                 for (int b = 0; b < NARR; ++b) cp16(dst + i * SLOT + b * 2 * DP, base(b) + off);
             }
-            off += G::SPI * bstep;
+            off += STEP * bstep;
         }
-        it += kG;
+        it += KG;
         cp_commit();
     }
     template <int SLOT>
@@ -327,16 +359,22 @@ __device__ __forceinline__ void store_deltas(uint8_t* base, uint32_t oa, uint32_
 }
 
 // ---- first phase: one warp, scanlines s and s + 1 of direction (dx, dy), deltas to `out`
+//
+// Steps go in groups of kFirstG: a group's costs are one cp.async group, waited for once and read from
+// the ring together, so the steps of a group hold nothing but the recurrence and the stores.
+constexpr int kFirstG = 8;
 template <int DP>
-__host__ __device__ constexpr int first_groups() { return DP >= 192 ? 4 : 8; }  // ring depth in groups
+__host__ __device__ constexpr int first_groups() { return DP >= 192 ? 3 : 4; }  // ring depth in groups
 template <int DP>
-__host__ __device__ constexpr int first_bytes() { return first_groups<DP>() * kG * 2 * DP + kTail; }
+__host__ __device__ constexpr int first_bytes() { return (int)sizeof(P2Smem) + first_groups<DP>() * kFirstG * 2 * DP + kTail; }
 
 template <int DP>
-__device__ __forceinline__ void run_first8(const Args8& a, uint8_t* ring, int dx, int dy, int s, int nscan,
+__device__ __forceinline__ void run_first8(const Args8& a, uint8_t* smem, int dx, int dy, int s, int nscan,
                                            uint8_t* out) {
     using G = Geo<DP>;
-    constexpr int W = G::W, SLOT = 2 * DP, NG = first_groups<DP>();
+    constexpr int W = G::W, SLOT = 2 * DP, NG = first_groups<DP>(), KG = kFirstG;
+    P2Smem* sm = reinterpret_cast<P2Smem*>(smem);
+    uint8_t* ring = smem + sizeof(P2Smem);
     const int lane = threadIdx.x & 31;
     const Pair q = pair_start(a, dx, dy, s, nscan);
     if (q.maxlen == 0) return;
@@ -345,38 +383,38 @@ __device__ __forceinline__ void run_first8(const Args8& a, uint8_t* ring, int dx
     uint8_t* dst = ring + Copier<DP>::template place<SLOT>(lane);
     auto base = [&](int) { return a.vol; };
 #pragma unroll
-    for (int t = 0; t < NG - 1; ++t) cp.template group<SLOT, 1>(dst + t * kG * SLOT, base);
+    for (int t = 0; t < NG - 1; ++t) cp.template group<SLOT, 1, KG>(dst + t * KG * SLOT, base);
     uint32_t pad[W];
     pad_words<DP>(a, lane, pad);
     Chain<W> st;
     chain_init(st);
     GrayRun g;
-    gray_init(a, q, 0, lane, g);
-    const uint32_t p1x2 = (uint32_t)a.pen.P1 * 0x00010001u;
+    gray_init(a, q, 0, lane, sm, g);
+    const uint32_t p1x2 = (uint32_t)a.P1 * 0x00010001u;
     const uint8_t* rd = ring + lane * W;
     // 32-bit byte offsets (the host checks the volume's size)
     uint32_t oa = (uint32_t)q.pA * DP + lane * W, ob = (uint32_t)q.pB * DP + lane * W;
     const uint32_t ostep = (uint32_t)(q.step * DP);
     const bool act = G::AL == 32 || lane < G::AL;
     int slot = 0;
-    auto groups = [&](auto clean, auto full, int t0, uint32_t p2v) {
+    auto groups = [&](auto clean, auto full, int t0) {
 #pragma unroll 1
-        for (int u0 = 0; u0 < 32; u0 += kG) {
+        for (int u0 = 0; u0 < 32; u0 += KG) {
             const int tb = t0 + u0;
             if (!decltype(full)::value && tb >= q.maxlen) break;
             cp_wait<NG - 2>();
             __syncwarp();
-            cp.template group<SLOT, 1>(dst + (slot == 0 ? NG - 1 : slot - 1) * (kG * SLOT), base);
-            const uint8_t* sl = rd + slot * (kG * SLOT);
-            Raw<DP> raw[kG];
-            uint32_t p2[kG];
+            cp.template group<SLOT, 1, KG>(dst + (slot == 0 ? NG - 1 : slot - 1) * (KG * SLOT), base);
+            const uint8_t* sl = rd + slot * (KG * SLOT);
+            Raw<DP> raw[KG];
+            uint32_t p2[KG];
+            p2_group<KG>(sm, u0, p2);
 #pragma unroll
-            for (int v = 0; v < kG; ++v) {
+            for (int v = 0; v < KG; ++v) {
                 raw[v] = load_raw<DP>(sl + v * SLOT);
-                p2[v] = __shfl_sync(0xffffffffu, p2v, u0 + v);
             }
 #pragma unroll
-            for (int v = 0; v < kG; ++v) {
+            for (int v = 0; v < KG; ++v) {
                 uint32_t c[W], dl[W];
                 path_step<DP, decltype(clean)::value>(st, raw[v], pad, p1x2, p2[v], lane, c, dl);
                 if (decltype(full)::value) store_deltas<DP>(out, oa, ob, act, act, dl);
@@ -388,10 +426,10 @@ __device__ __forceinline__ void run_first8(const Args8& a, uint8_t* ring, int dx
         }
     };
     for (int t0 = 0; t0 < q.maxlen; t0 += 32) {
-        const uint32_t p2v = p2_block(a, q, t0, lane, g);
-        if (t0 + 32 > q.minlen) groups(std::false_type(), std::false_type(), t0, p2v);
-        else if (clean_block(a, q, dx, t0)) groups(std::true_type(), std::true_type(), t0, p2v);
-        else groups(std::false_type(), std::true_type(), t0, p2v);
+        p2_block(a, q, t0, lane, sm, g);
+        if (t0 + 32 > q.minlen) groups(std::false_type(), std::false_type(), t0);
+        else if (clean_block(a, q, dx, t0)) groups(std::true_type(), std::true_type(), t0);
+        else groups(std::false_type(), std::true_type(), t0);
     }
     cp_wait<0>();
     __syncwarp();
@@ -405,25 +443,37 @@ __host__ __device__ constexpr uint32_t sum_bias() { return kBias * (NIN + 1); }
 template <int NIN>
 __host__ __device__ constexpr uint32_t sum_inf() { return (kBias + 0x0300u) * (NIN + 1); }
 
-// sum[] += the deltas of NIN arrays at sl (layout [array][A, B][DP]).
+// The deltas of NIN arrays at sl (layout [array][A, B][DP]); with PS in pairs, added as bytes.
 template <int DP, int NIN, bool PS>
-__device__ __forceinline__ void add_deltas(const uint8_t* sl, uint32_t (&sum)[Geo<DP>::W]) {
-    constexpr int W = Geo<DP>::W;
+struct Deltas {
+    static constexpr int N = PS ? (NIN + 1) / 2 : NIN;
+    Raw<DP> r[N];
+};
+template <int DP, int NIN, bool PS>
+__device__ __forceinline__ Deltas<DP, NIN, PS> load_deltas(const uint8_t* sl) {
+    Deltas<DP, NIN, PS> d;
 #pragma unroll
-    for (int b = 0; b < NIN;) {
-        Raw<DP> r = load_raw<DP>(sl + b * 2 * DP);
-        ++b;
-        if (PS && b < NIN) {
-            const Raw<DP> r2 = load_raw<DP>(sl + b * 2 * DP);
+    for (int b = 0; b < NIN; ++b) {
+        const Raw<DP> r = load_raw<DP>(sl + b * 2 * DP);
+        if (PS && (b & 1)) {
 #pragma unroll
             for (int i = 0; i < Raw<DP>::N; ++i) {
-                r.a[i] += r2.a[i];
-                r.b[i] += r2.b[i];
+                d.r[b / 2].a[i] += r.a[i];
+                d.r[b / 2].b[i] += r.b[i];
             }
-            ++b;
+        } else {
+            d.r[PS ? b / 2 : b] = r;
         }
+    }
+    return d;
+}
+template <int DP, int NIN, bool PS>
+__device__ __forceinline__ void add_deltas(const Deltas<DP, NIN, PS>& d, uint32_t (&sum)[Geo<DP>::W]) {
+    constexpr int W = Geo<DP>::W;
+#pragma unroll
+    for (int b = 0; b < Deltas<DP, NIN, PS>::N; ++b) {
         uint32_t e[W / 2];
-        interleave<DP>(r, e);
+        interleave<DP>(d.r[b], e);
 #pragma unroll
         for (int i = 0; i < W / 2; ++i) {
             sum[2 * i] += e[i] & 0x00FF00FFu;
@@ -472,7 +522,7 @@ __device__ __forceinline__ void put_sums(const Args8& a, const Pair& q, uint32_t
 
 // The WTA of the block of 16 steps at tb: lane l takes step tb + l % 16 of scanline A (l < 16) or B.
 template <int DP, int NIN>
-__device__ __forceinline__ void wta_block(const Args8& a, const Pair& q, const uint32_t* s_wta, int tb, int lane) {
+__device__ __forceinline__ void wta_block(const Args8& a, const Pair& q, uint32_t* s_wta, int tb, int lane) {
     const int t = tb + (lane & 15);
     const bool b = lane >= 16;
     if (t < (b ? q.lenB : q.lenA))
@@ -481,7 +531,6 @@ __device__ __forceinline__ void wta_block(const Args8& a, const Pair& q, const u
 }
 
 // Bands of steps [t_begin, t_end): the chains' path values enter and leave through a.carry.
-template <int DP>
 __device__ __forceinline__ bool band_limits(const Args8& a, Pair& q, int& tb0) {
     tb0 = a.t_begin;
     const bool carry_out = a.t_end < q.maxlen;
@@ -492,10 +541,13 @@ __device__ __forceinline__ bool band_limits(const Args8& a, Pair& q, int& tb0) {
     return carry_out;
 }
 template <int DP>
-__device__ __forceinline__ void band_load(const Args8& a, int s, int lane, Chain<Geo<DP>::W>& st) {
+__device__ __forceinline__ void band_load(const Args8& a, int s, int lane, uint32_t p1x2, Chain<Geo<DP>::W>& st) {
     const uint32_t* cs = a.carry + (size_t)(s >> 1) * Geo<DP>::W * 32 + lane;
 #pragma unroll
-    for (int k = 0; k < Geo<DP>::W; ++k) st.L[k] = __ldcg(cs + k * 32);
+    for (int k = 0; k < Geo<DP>::W; ++k) {
+        st.L[k] = __ldcg(cs + k * 32);
+        st.q[k] = st.L[k] + p1x2;
+    }
     chain_reduce(st);
 }
 template <int DP>
@@ -505,69 +557,75 @@ __device__ __forceinline__ void band_store(const Args8& a, int s, int lane, cons
     for (int k = 0; k < Geo<DP>::W; ++k) __stcg(cs + k * 32, st.L[k]);
 }
 
-// One warp per pair of scanlines.
-template <int DP, int NIN, int NG>
+// One warp per pair of scanlines: rings of NG groups of KG steps.
+template <int DP, int NIN, int KG, int NG>
 __host__ __device__ constexpr int last_bytes() {
-    return Geo<DP>::wta_words * 4 + NG * kG * (1 + NIN) * 2 * DP + kTail;
+    return (int)sizeof(P2Smem) + Geo<DP>::wta_words * 4 + NG * KG * (1 + NIN) * 2 * DP + kTail;
 }
-template <int DP, int NIN, int NG, bool PS, bool BAND>
+template <int DP, int NIN, int KG, int NG, bool PS, bool BAND>
 __device__ __forceinline__ void run_last8(const Args8& a, const uint8_t* const* in, uint8_t* smem, int dx, int dy, int s,
                                           int nscan) {
     using G = Geo<DP>;
     constexpr int W = G::W, NARR = 1 + NIN, SLOT = NARR * 2 * DP;
-    uint32_t* s_wta = reinterpret_cast<uint32_t*>(smem);
-    uint8_t* ring = smem + G::wta_words * 4;
+    static_assert(16 % KG == 0, "a WTA block is whole groups");
+    P2Smem* sm = reinterpret_cast<P2Smem*>(smem);
+    uint32_t* s_wta = reinterpret_cast<uint32_t*>(smem + sizeof(P2Smem));
+    uint8_t* ring = smem + sizeof(P2Smem) + G::wta_words * 4;
     const int lane = threadIdx.x & 31;
     Pair q = pair_start(a, dx, dy, s, nscan);
     int tb0 = 0;
     bool carry_out = false;
-    if constexpr (BAND) carry_out = band_limits<DP>(a, q, tb0);
+    if constexpr (BAND) carry_out = band_limits(a, q, tb0);
     if (q.maxlen <= tb0) return;
     Copier<DP> cp;
     cp.init(q, tb0, lane);
     uint8_t* dst = ring + Copier<DP>::template place<SLOT>(lane);
     auto base = [&](int b) { return b == 0 ? a.vol : in[b - 1]; };
 #pragma unroll
-    for (int t = 0; t < NG - 1; ++t) cp.template group<SLOT, NARR>(dst + t * kG * SLOT, base);
+    for (int t = 0; t < NG - 1; ++t) cp.template group<SLOT, NARR, KG>(dst + t * KG * SLOT, base);
     uint32_t pad[W];
     pad_words<DP>(a, lane, pad);
+    const uint32_t p1x2 = (uint32_t)a.P1 * 0x00010001u;
     Chain<W> st;
     chain_init(st);
     if constexpr (BAND)
-        if (tb0 > 0) band_load<DP>(a, s, lane, st);
+        if (tb0 > 0) band_load<DP>(a, s, lane, p1x2, st);
     GrayRun g;
-    gray_init(a, q, tb0, lane, g);
-    const uint32_t p1x2 = (uint32_t)a.pen.P1 * 0x00010001u;
+    gray_init(a, q, tb0, lane, sm, g);
     const uint8_t* rd = ring + lane * W;
     const bool act = G::AL == 32 || lane < G::AL;
     int slot = 0;
-    auto groups = [&](auto clean, int t0, uint32_t p2v) {
+    auto groups = [&](auto clean, int t0) {
 #pragma unroll 1
-        for (int u0 = 0; u0 < 32; u0 += kG) {
+        for (int u0 = 0; u0 < 32; u0 += KG) {
             const int tb = t0 + u0;
             if (tb >= q.maxlen) break;
             cp_wait<NG - 2>();
             __syncwarp();
-            cp.template group<SLOT, NARR>(dst + (slot == 0 ? NG - 1 : slot - 1) * (kG * SLOT), base);
-            const uint8_t* sl = rd + slot * (kG * SLOT);
-            Raw<DP> raw[kG];
-            uint32_t p2[kG];
+            cp.template group<SLOT, NARR, KG>(dst + (slot == 0 ? NG - 1 : slot - 1) * (KG * SLOT), base);
+            const uint8_t* sl = rd + slot * (KG * SLOT);
+            // everything the group reads from the ring first: the sums' stores below may not be
+            // reordered with later loads
+            Raw<DP> raw[KG];
+            Deltas<DP, NIN, PS> de[KG];
+            uint32_t p2[KG];
+            p2_group<KG>(sm, u0, p2);
 #pragma unroll
-            for (int v = 0; v < kG; ++v) {
+            for (int v = 0; v < KG; ++v) {
                 raw[v] = load_raw<DP>(sl + v * SLOT);
-                p2[v] = __shfl_sync(0xffffffffu, p2v, u0 + v);
+                de[v] = load_deltas<DP, NIN, PS>(sl + v * SLOT + 2 * DP);
             }
 #pragma unroll
-            for (int v = 0; v < kG; ++v) {
+            for (int v = 0; v < KG; ++v) {
                 uint32_t c[W], dl[W], sum[W];
                 path_step<DP, decltype(clean)::value>(st, raw[v], pad, p1x2, p2[v], lane, c, dl);
 #pragma unroll
                 for (int k = 0; k < W; ++k) sum[k] = c[k] * (uint32_t)(NIN + 1) + dl[k];
-                add_deltas<DP, NIN, PS>(sl + v * SLOT + 2 * DP, sum);
+                add_deltas<DP, NIN, PS>(de[v], sum);
                 put_sums<DP, NIN>(a, q, s_wta, (u0 + v) & 15, tb + v, lane, act, sum);
             }
             slot = slot == NG - 1 ? 0 : slot + 1;
-            if ((u0 & 15) == 12 || tb + kG >= q.maxlen) {
+            if (((u0 + KG) & 15) == 0 || tb + KG >= q.maxlen) {
                 __syncwarp();
                 wta_block<DP, NIN>(a, q, s_wta, t0 + (u0 & 16), lane);
                 __syncwarp();
@@ -575,14 +633,192 @@ __device__ __forceinline__ void run_last8(const Args8& a, const uint8_t* const* 
         }
     };
     for (int t0 = tb0; t0 < q.maxlen; t0 += 32) {
-        const uint32_t p2v = p2_block(a, q, t0, lane, g);
-        if (clean_block(a, q, dx, t0)) groups(std::true_type(), t0, p2v);
-        else groups(std::false_type(), t0, p2v);
+        p2_block(a, q, t0, lane, sm, g);
+        if (clean_block(a, q, dx, t0)) groups(std::true_type(), t0);
+        else groups(std::false_type(), t0);
     }
     if constexpr (BAND)
         if (carry_out) band_store<DP>(a, s, lane, st);
     cp_wait<0>();
     __syncwarp();
+}
+
+// Two warps per pair of scanlines: warp 0 runs the recurrence and hands each step's n * C + delta to
+// warp 1, which adds the other directions' deltas and runs the WTA.  Steps change hands in segments of
+// KG steps through two shared buffers: warp 0 arrives on FULL[slot] once a segment is written and waits on
+// FREE[slot] before it writes the slot again, warp 1 the other way round.  Both walk the same number of
+// segments (one pair per block), so every barrier generation is completed by one arrival of each warp.
+// Barrier ids are immediates (a register id would make the compiler reserve all sixteen) and the kernel
+// has no other block barrier.
+template <int DP, int NIN, int KG, int NGP, int NGC>
+struct Split8 {
+    static constexpr int ring_p = NGP * KG * 2 * DP + kTail;
+    static constexpr int ring_c = NGC * KG * NIN * 2 * DP + kTail;
+    static constexpr int part = 2 * KG * DP * 4;
+    static constexpr int bytes = (int)sizeof(P2Smem) + Geo<DP>::wta_words * 4 + part + ring_p + ring_c;
+};
+template <int ID>
+__device__ __forceinline__ void nbar_sync() { asm volatile("bar.sync %0, 64;\n" ::"n"(ID) : "memory"); }
+template <int ID>
+__device__ __forceinline__ void nbar_arrive() { asm volatile("bar.arrive %0, 64;\n" ::"n"(ID) : "memory"); }
+// barrier BASE + slot for a slot of two
+template <int BASE, bool SYNC>
+__device__ __forceinline__ void nbar(int slot) {
+    if (slot) {
+        if (SYNC) nbar_sync<BASE + 1>();
+        else nbar_arrive<BASE + 1>();
+    } else {
+        if (SYNC) nbar_sync<BASE>();
+        else nbar_arrive<BASE>();
+    }
+}
+constexpr int kSeg = 2;
+constexpr int kFull = 0, kFree = kSeg;
+
+template <int DP, int NIN, int KG, int NGP, int NGC, bool PS, bool BAND>
+__global__ void __launch_bounds__(64) sgm8_last_split_kernel(Args8 a, In8 in, int dx, int dy, int nscan) {
+    using G = Geo<DP>;
+    using S = Split8<DP, NIN, KG, NGP, NGC>;
+    constexpr int W = G::W;
+    static_assert(16 % KG == 0, "a WTA block is whole segments");
+    extern __shared__ __align__(16) uint8_t s8[];
+    P2Smem* sm = reinterpret_cast<P2Smem*>(s8);
+    uint32_t* s_wta = reinterpret_cast<uint32_t*>(s8 + sizeof(P2Smem));
+    uint32_t* s_part = s_wta + G::wta_words;
+    uint8_t* ring_p = s8 + sizeof(P2Smem) + G::wta_words * 4 + S::part;
+    uint8_t* ring_c = ring_p + S::ring_p;
+    const int lane = threadIdx.x & 31;
+    const int s = 2 * (int)blockIdx.x;
+    Pair q = pair_start(a, dx, dy, s, nscan);
+    int tb0 = 0;
+    bool carry_out = false;
+    if constexpr (BAND) carry_out = band_limits(a, q, tb0);
+    if (q.maxlen <= tb0) return;  // the whole block (one pair)
+    const int nseg = (q.maxlen - tb0 + KG - 1) / KG;
+    const bool act = G::AL == 32 || lane < G::AL;
+    uint32_t* part = s_part + lane * W;
+    Copier<DP> cp;
+    cp.init(q, tb0, lane);
+    if (threadIdx.x < 32) {
+        constexpr int SLOT = 2 * DP;
+        uint8_t* dst = ring_p + Copier<DP>::template place<SLOT>(lane);
+        auto base = [&](int) { return a.vol; };
+#pragma unroll
+        for (int t = 0; t < NGP - 1; ++t) cp.template group<SLOT, 1, KG>(dst + t * KG * SLOT, base);
+        uint32_t pad[W];
+        pad_words<DP>(a, lane, pad);
+        const uint32_t p1x2 = (uint32_t)a.P1 * 0x00010001u;
+        Chain<W> st;
+        chain_init(st);
+        if constexpr (BAND)
+            if (tb0 > 0) band_load<DP>(a, s, lane, p1x2, st);
+        GrayRun g;
+        gray_init(a, q, tb0, lane, sm, g);
+        const uint8_t* rd = ring_p + lane * W;
+        int slot = 0;
+        auto groups = [&](auto clean, int t0) {
+#pragma unroll 1
+            for (int u0 = 0; u0 < 32; u0 += KG) {
+                const int tb = t0 + u0;
+                if (tb >= q.maxlen) break;
+                cp_wait<NGP - 2>();
+                __syncwarp();
+                cp.template group<SLOT, 1, KG>(dst + (slot == 0 ? NGP - 1 : slot - 1) * (KG * SLOT), base);
+                const uint8_t* sl = rd + slot * (KG * SLOT);
+                Raw<DP> raw[KG];
+                uint32_t p2[KG];
+                p2_group<KG>(sm, u0, p2);
+#pragma unroll
+                for (int v = 0; v < KG; ++v) {
+                    raw[v] = load_raw<DP>(sl + v * SLOT);
+                }
+                const int seg = (tb - tb0) / KG, sb = seg % kSeg;
+                if (seg >= kSeg) nbar<kFree, true>(sb);
+#pragma unroll
+                for (int v = 0; v < KG; ++v) {
+                    uint32_t c[W], dl[W];
+                    path_step<DP, decltype(clean)::value>(st, raw[v], pad, p1x2, p2[v], lane, c, dl);
+                    if (act) {
+                        uint32_t* o = part + (sb * KG + v) * DP;
+#pragma unroll
+                        for (int k = 0; k < W; ++k) c[k] = c[k] * (uint32_t)(NIN + 1) + dl[k];
+                        if constexpr (W == 2) *reinterpret_cast<uint2*>(o) = make_uint2(c[0], c[1]);
+                        else {
+#pragma unroll
+                            for (int k = 0; k < W; k += 4)
+                                *reinterpret_cast<uint4*>(o + k) = make_uint4(c[k], c[k + 1], c[k + 2], c[k + 3]);
+                        }
+                    }
+                }
+                __threadfence_block();
+                nbar<kFull, false>(sb);
+                slot = slot == NGP - 1 ? 0 : slot + 1;
+            }
+        };
+        for (int t0 = tb0; t0 < q.maxlen; t0 += 32) {
+            p2_block(a, q, t0, lane, sm, g);
+            if (clean_block(a, q, dx, t0)) groups(std::true_type(), t0);
+            else groups(std::false_type(), t0);
+        }
+        if constexpr (BAND)
+            if (carry_out) band_store<DP>(a, s, lane, st);
+    } else {
+        constexpr int SLOT = NIN * 2 * DP;
+        uint8_t* dst = ring_c + Copier<DP>::template place<SLOT>(lane);
+        auto base = [&](int b) { return in.d[b]; };
+#pragma unroll
+        for (int t = 0; t < NGC - 1; ++t) cp.template group<SLOT, NIN, KG>(dst + t * KG * SLOT, base);
+        const uint8_t* rd = ring_c + lane * W;
+        int slot = 0;
+#pragma unroll 1
+        for (int seg = 0; seg < nseg; ++seg) {
+            const int tb = tb0 + seg * KG, sb = seg % kSeg;
+            cp_wait<NGC - 2>();
+            __syncwarp();
+            cp.template group<SLOT, NIN, KG>(dst + (slot == 0 ? NGC - 1 : slot - 1) * (KG * SLOT), base);
+            const uint8_t* sl = rd + slot * (KG * SLOT);
+            // the segment's reads come first, half a segment at a time: the sums' stores may not be
+            // reordered with later loads
+            constexpr int H = KG >= 4 ? 4 : KG;
+            Deltas<DP, NIN, PS> de[H];
+#pragma unroll
+            for (int v = 0; v < H; ++v) de[v] = load_deltas<DP, NIN, PS>(sl + v * SLOT);
+            nbar<kFull, true>(sb);
+#pragma unroll
+            for (int h = 0; h < KG; h += H) {
+                uint32_t sum[H][W];
+#pragma unroll
+                for (int v = 0; v < H; ++v) {
+                    const uint32_t* o = part + (sb * KG + h + v) * DP;
+                    if constexpr (W == 2) {
+                        const uint2 x = *reinterpret_cast<const uint2*>(o);
+                        sum[v][0] = x.x; sum[v][1] = x.y;
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < W; k += 4) {
+                            const uint4 x = *reinterpret_cast<const uint4*>(o + k);
+                            sum[v][k] = x.x; sum[v][k + 1] = x.y; sum[v][k + 2] = x.z; sum[v][k + 3] = x.w;
+                        }
+                    }
+                    if (h > 0) de[v] = load_deltas<DP, NIN, PS>(sl + (h + v) * SLOT);
+                }
+#pragma unroll
+                for (int v = 0; v < H; ++v) {
+                    add_deltas<DP, NIN, PS>(de[v], sum[v]);
+                    put_sums<DP, NIN>(a, q, s_wta, (tb + h + v) & 15, tb + h + v, lane, act, sum[v]);
+                }
+            }
+            __threadfence_block();
+            if (seg + kSeg < nseg) nbar<kFree, false>(sb);
+            slot = slot == NGC - 1 ? 0 : slot + 1;
+            if (((tb + KG) & 15) == 0 || seg == nseg - 1) {
+                __syncwarp();
+                wta_block<DP, NIN>(a, q, s_wta, tb & ~15, lane);
+                __syncwarp();
+            }
+        }
+    }
+    cp_wait<0>();
 }
 
 // One warp per block: chains of different lengths end independently.
@@ -597,19 +833,38 @@ __global__ void __launch_bounds__(32) sgm8_first_kernel(Args8 a, Dirs8 tab) {
     run_first8<DP>(a, s8, tab.dx[d], tab.dy[d], s, tab.nscan[d], tab.out[d]);
 }
 
-template <int DP, int NIN, int NG, bool PS, bool BAND>
+template <int DP, int NIN, int KG, int NG, bool PS, bool BAND>
 __global__ void __launch_bounds__(32) sgm8_last_kernel(Args8 a, In8 in, int dx, int dy, int nscan) {
     extern __shared__ __align__(16) uint8_t s8[];
-    run_last8<DP, NIN, NG, PS, BAND>(a, in.d, s8, dx, dy, 2 * (int)blockIdx.x, nscan);
+    run_last8<DP, NIN, KG, NG, PS, BAND>(a, in.d, s8, dx, dy, 2 * (int)blockIdx.x, nscan);
 }
 
 int nscan8(int w, int h, int dx, int dy) { return dy == 0 ? h : (dx == 0 ? w : w + h - 1); }
+
+// adaptive_p2 (common.cuh) on the host, the same single-precision steps.
+int host_p2(const SgmPen& p, int dI) {
+    int P2 = p.P2_base;
+    if (p.adaptive) {
+        if (p.piecewise) {
+            if (dI >= p.t2) P2 = p.P2_base / 4;
+            else if (dI >= p.t1) P2 = p.P2_base / 2;
+        } else {
+            const volatile float scaled = p.alpha * (float)dI;
+            const volatile float den = 1.f + scaled;
+            const volatile float quot = (float)p.P2_base / den;
+            const volatile float up = quot + 0.5f;
+            P2 = (int)up;
+        }
+    }
+    return std::max(P2, p.P1 + 1);
+}
 
 Args8 make_args8(const SgmLaunch& l) {
     Args8 a{};
     a.w = l.w; a.h = l.h; a.d0 = l.d0; a.D = l.D; a.dmax = l.d0 + l.D;
     a.def_ranges = l.default_ranges;
-    a.pen = l.pen;
+    a.P1 = l.pen.P1;
+    for (int i = 0; i < 256; ++i) a.p2[i] = (uint8_t)host_p2(l.pen, i);
     a.gray = l.gray;
     a.vol = reinterpret_cast<const uint8_t*>(l.cvol);
     a.wta = WtaOut{l.disp, l.best, l.second, l.subpixel, l.sp_method, l.sp_param, l.sp_tel};
@@ -652,13 +907,39 @@ cudaError_t by_dp(int Dp, F f) {
     }
 }
 
-template <int DP, int NIN, int PF, bool PS, bool BAND>
+// Blocks of `bytes` shared memory the device holds at once.
+int blocks_at_once(size_t bytes) {
+    int dev = 0, nsm = 0, per_sm = 0, reserved = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return nsm * (int)(per_sm / (bytes + reserved));
+}
+
+template <int DP, int NIN, bool PS, bool BAND>
 cudaError_t launch_last_t(const Args8& a, const In8& in, int dx, int dy, int nscan, cudaStream_t st) {
-    auto kern = sgm8_last_kernel<DP, NIN, PF, PS, BAND>;
-    const size_t smem = even_share((nscan + 1) / 2, last_bytes<DP, NIN, PF>(), 4);
+    const int blocks = (nscan + 1) / 2;
+    // two warps per pair where every pair is resident at once in that form, else one
+    constexpr int SG = NIN == 3 && DP <= 128 ? 8 : 4, NGP = DP == 256 ? 2 : 3, NGC = DP == 192 && NIN == 3 ? 3 : 2;
+    using S = Split8<DP, NIN, SG, NGP, NGC>;
+    if (blocks <= blocks_at_once(S::bytes)) {
+        auto kern = sgm8_last_split_kernel<DP, NIN, SG, NGP, NGC, PS, BAND>;
+        const size_t smem = even_share(blocks, S::bytes, 4);
+        const cudaError_t e = allow_dynamic_smem(kern, smem);
+        if (e != cudaSuccess) return e;
+        kern<<<blocks, 64, smem, st>>>(a, in, dx, dy, nscan);
+        return cudaGetLastError();
+    }
+    constexpr int KG = DP == 256 ? (NIN == 3 ? 2 : 1) : (NIN == 3 ? 4 : 2), NG = 3;
+    auto kern = sgm8_last_kernel<DP, NIN, KG, NG, PS, BAND>;
+    const size_t smem = even_share(blocks, last_bytes<DP, NIN, KG, NG>(), 4);
     const cudaError_t e = allow_dynamic_smem(kern, smem);
     if (e != cudaSuccess) return e;
-    kern<<<(nscan + 1) / 2, 32, smem, st>>>(a, in, dx, dy, nscan);
+    kern<<<blocks, 32, smem, st>>>(a, in, dx, dy, nscan);
     return cudaGetLastError();
 }
 
@@ -672,15 +953,12 @@ cudaError_t launch_last_any(const SgmLaunch& l, const Args8& a, int dx, int dy, 
     const bool ps = 2 * max_p2(l.pen) <= 255;
     return by_dp(l.Dp, [&](auto dp) -> cudaError_t {
         constexpr int DP = decltype(dp)::value;
-        constexpr int PF3 = DP == 256 ? 2 : 4;
         if (nin == 3)
-            return ps ? launch_last_t<DP, 3, PF3, true, BAND>(a, t, dx, dy, nscan, st)
-                      : launch_last_t<DP, 3, PF3, false, BAND>(a, t, dx, dy, nscan, st);
-        if constexpr (!BAND) {
-            constexpr int PF7 = DP >= 192 ? 2 : 3;
-            return ps ? launch_last_t<DP, 7, PF7, true, false>(a, t, dx, dy, nscan, st)
-                      : launch_last_t<DP, 7, PF7, false, false>(a, t, dx, dy, nscan, st);
-        }
+            return ps ? launch_last_t<DP, 3, true, BAND>(a, t, dx, dy, nscan, st)
+                      : launch_last_t<DP, 3, false, BAND>(a, t, dx, dy, nscan, st);
+        if constexpr (!BAND)
+            return ps ? launch_last_t<DP, 7, true, false>(a, t, dx, dy, nscan, st)
+                      : launch_last_t<DP, 7, false, false>(a, t, dx, dy, nscan, st);
         return cudaErrorInvalidValue;
     });
 }

@@ -19,79 +19,72 @@ struct WtaOut {
     apg_subpixel_telemetry_t* sp_tel;
 };
 
-// WTA of pixel p from its final sums, W2 u16x2 words in shared memory (16-byte aligned), run by one
-// lane (wta_impl, src/sgm_optimizer.cpp:465-536): the first minimum, the second minimum outside
+// WTA of pixel p from its final sums, W2 u16x2 words in shared memory (16-byte aligned, changed by the
+// scan), run by one lane (wta_impl, src/sgm_optimizer.cpp:465-536): the first minimum, the second minimum outside
 // |d - best| <= 1, the sub-pixel step.  Every sum carries BIAS; sums >= INF are invalid.  A negative
 // winning disparity reads as "none" like the reference's best_d < 0 test (:490-495).
 template <int W2, uint32_t INF, uint32_t BIAS>
-__device__ __forceinline__ void wta_row(const WtaOut& o, int d0, int D, const uint32_t* row, int p) {
-    // one pass over the row keeps the minimum of each chunk of four or eight words in registers; the
-    // first index and the second minimum then read the (at most two) chunks they touch again
-    constexpr int CS = W2 >= 128 ? 8 : 4;  // words per chunk (W2 is a multiple of 32)
-    constexpr int NC = W2 / CS;
+__device__ __forceinline__ void wta_row(const WtaOut& o, int d0, int D, uint32_t* row, int p) {
+    constexpr int NC = W2 / 4;  // chunks of four words
     const auto halves = [](uint32_t v) { return min(v & 0xFFFFu, v >> 16); };
-    uint32_t cmin[NC];
+    // the minimum and the first group of GC chunks that holds it, as one key (minimum << 8 | group)
+    constexpr int GC = NC <= 16 ? 1 : NC / 16 + (NC % 16 != 0), NGR = NC / GC;
+    static_assert(NGR * GC == NC, "groups cover the row");
+    uint32_t key = 0xFFFFFFFFu;
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
+    for (int g = 0; g < NGR; ++g) {
         uint32_t v = 0xFFFFFFFFu;
 #pragma unroll
-        for (int i = 0; i < CS; i += 4) {
-            const uint4 q = *reinterpret_cast<const uint4*>(row + c * CS + i);
-            v = __vminu2(__vimin3_u16x2(v, q.x, q.y), __vminu2(q.z, q.w));
+        for (int c = 0; c < GC; ++c) {
+            const uint4 q = *reinterpret_cast<const uint4*>(row + 4 * (g * GC + c));
+            v = __vimin3_u16x2(__vimin3_u16x2(v, q.x, q.y), q.z, q.w);
         }
-        cmin[c] = v;
+        key = min(key, halves(v) * 256u + g);
     }
-    uint32_t all = cmin[0];
-#pragma unroll
-    for (int c = 1; c < NC; ++c) all = __vminu2(all, cmin[c]);
-    const uint32_t m = halves(all);
+    const uint32_t m = key >> 8;
     float dval = -1.f, fb = __int_as_float(0x7f800000), fs = __int_as_float(0x7f800000);
     if (m < INF) {
-        // the first chunk whose minimum is m, then the first halfword equal to m inside it
-        int fc = 0;
-#pragma unroll
-        for (int c = NC - 1; c >= 0; --c)
-            if (halves(cmin[c]) == m) fc = c;
+        // the first halfword of that group equal to m
+        const uint32_t* gr = row + 4 * GC * (key & 0xFFu);
         int bdi = 0;
 #pragma unroll
-        for (int i = CS - 1; i >= 0; --i) {
-            const uint32_t v = row[fc * CS + i];
-            if ((v >> 16) == m) bdi = 2 * i + 1;
-            if ((v & 0xFFFFu) == m) bdi = 2 * i;
-        }
-        bdi += 2 * fc * CS;
-        if (d0 + bdi >= 0) {
-            const uint16_t* r16 = reinterpret_cast<const uint16_t*>(row);
-            dval = (float)(d0 + bdi);
-            // second minimum outside |d - best| <= 1: chunks without an excluded halfword keep
-            // their minimum; the (at most two) chunks with one are read again with those masked
-            const int klo = bdi > 0 ? (bdi - 1) >> 1 : 0, khi = min((bdi + 1) >> 1, W2 - 1);
-            const int clo = klo / CS, chi = khi / CS;
-            uint32_t sec2 = 0xFFFFFFFFu;
+        for (int c = GC - 1; c >= 0; --c) {
+            const uint4 q = *reinterpret_cast<const uint4*>(gr + 4 * c);
+            const uint32_t v[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-            for (int c = 0; c < NC; ++c)
-                if (c != clo && c != chi) sec2 = __vminu2(sec2, cmin[c]);
-            for (int c = clo; c <= chi; ++c) {
-#pragma unroll
-                for (int i = 0; i < CS; ++i) {
-                    const int k = c * CS + i;
-                    uint32_t v = row[k];
-                    if (abs(2 * k - bdi) <= 1) v |= 0x0000FFFFu;
-                    if (abs(2 * k + 1 - bdi) <= 1) v |= 0xFFFF0000u;
-                    sec2 = __vminu2(sec2, v);
-                }
+            for (int i = 3; i >= 0; --i) {
+                if ((v[i] >> 16) == m) bdi = 8 * c + 2 * i + 1;
+                if ((v[i] & 0xFFFFu) == m) bdi = 8 * c + 2 * i;
             }
-            const uint32_t sec = halves(sec2);
+        }
+        bdi += 8 * GC * (int)(key & 0xFFu);
+        if (d0 + bdi >= 0) {
+            // the second minimum outside |d - best| <= 1: those three sums are read, taken out of the
+            // row, and the row scanned again
+            uint16_t* r16 = reinterpret_cast<uint16_t*>(row);
+            const uint32_t cm = bdi > 0 ? r16[bdi - 1] : 0xFFFFu, cp = bdi + 1 < 2 * W2 ? r16[bdi + 1] : 0xFFFFu;
+            if (bdi > 0) r16[bdi - 1] = 0xFFFFu;
+            r16[bdi] = 0xFFFFu;
+            if (bdi + 1 < 2 * W2) r16[bdi + 1] = 0xFFFFu;
+            uint32_t s0 = 0xFFFFFFFFu, s1 = 0xFFFFFFFFu;
+#pragma unroll
+            for (int c = 0; c < NC; c += 2) {
+                const uint4 q = *reinterpret_cast<const uint4*>(row + 4 * c);
+                const uint4 r = *reinterpret_cast<const uint4*>(row + 4 * c + 4);
+                s0 = __vimin3_u16x2(__vimin3_u16x2(s0, q.x, q.y), q.z, q.w);
+                s1 = __vimin3_u16x2(__vimin3_u16x2(s1, r.x, r.y), r.z, r.w);
+            }
+            const uint32_t sec = halves(__vminu2(s0, s1));
             const uint32_t bv = m - BIAS;
-            if (o.subpixel && bdi > 0 && bdi + 1 < D) {
-                const uint32_t cm = r16[bdi - 1], cp = r16[bdi + 1];
-                if (cm < INF && cp < INF) {
-                    // WTA uniqueness (src/sgm_optimizer.cpp:520-525): (second - best) / max(best, 1)
-                    const float u = sec >= INF ? 1.0f : __fdiv_rn((float)(sec - m), (float)max(bv, 1u));
-                    const float fm = (float)(cm - BIAS), f0 = (float)bv, fp = (float)(cp - BIAS);
-                    dval = __fadd_rn(dval, o.sp_tel ? subpixel_delta_tel(fm, f0, fp, o.sp_method, o.sp_param, u, o.sp_tel)
-                                                    : subpixel_delta(fm, f0, fp, o.sp_method, o.sp_param, u));
-                }
+            dval = (float)(d0 + bdi);
+            if (o.subpixel && bdi > 0 && bdi + 1 < D && cm < INF && cp < INF) {
+                // WTA uniqueness (src/sgm_optimizer.cpp:520-525): (second - best) / max(best, 1), read by
+                // one of the experimental methods only
+                float u = 1.0f;
+                if (o.sp_method == 2 && sec < INF) u = __fdiv_rn((float)(sec - m), (float)max(bv, 1u));
+                const float fm = (float)(cm - BIAS), f0 = (float)bv, fp = (float)(cp - BIAS);
+                dval = __fadd_rn(dval, o.sp_tel ? subpixel_delta_tel(fm, f0, fp, o.sp_method, o.sp_param, u, o.sp_tel)
+                                                : subpixel_delta(fm, f0, fp, o.sp_method, o.sp_param, u));
             }
             fb = (float)bv;
             fs = sec >= INF ? __int_as_float(0x7f800000) : (float)(sec - BIAS);
