@@ -36,7 +36,7 @@ namespace apgcu {
 namespace {
 
 constexpr int kBand = 32;
-constexpr int kPublish = 8;      // steps between progress publications
+constexpr int kChunk = 8;        // steps between exchanges (records, row above, progress)
 constexpr int kMaxRejected = 64;  // rejected outputs tabulated per radius (expected: none)
 
 __global__ void refine_flags_kernel(int w, int h, const uint8_t* __restrict__ reliable, const int16_t* __restrict__ rmin,
@@ -201,19 +201,17 @@ __device__ __forceinline__ float packed_cost(const CostCtx& c, const float* lut,
 }
 
 // Everything about one pixel of a pass that does not depend on the wavefront, computed for all
-// pixels at once before the pass and laid out in pass order (index v * w + u): the value at the
-// start of the pass, its range, and the two static candidates -- the current value and the
-// current value plus the pixel's draw -- with their costs.  The band kernel only costs the two
-// dynamic candidates (left and up neighbours) and keeps the reference's candidate order.
+// pixels at once before the pass and laid out in pass order (index v * w + u): its range and the two
+// static candidates -- the current value and the current value plus the pixel's draw -- with their
+// costs.  The band kernel only costs the two dynamic candidates (left and up neighbours) and keeps
+// the reference's candidate order.  A pixel the pass does not update carries the cost -infinity and
+// its value as a neighbour candidate (roundf(value) when value >= 0, else -1), so the same selection
+// returns it; an updated pixel without a value carries the cost 1e9 and the start of its range.
 struct __align__(16) RStep {
-    float cur;     // value at the start of the pass
-    float c_cur;   // cost of candidate `cur` (when upd bit 1)
-    float c_draw;  // cost of candidate `cur + draw` (when upd bit 2)
+    float c_cur;   // cost of candidate d_cur
+    float c_draw;  // cost of candidate d_draw (1e9: none)
     int d_pack;    // d_cur (low 16, signed) | d_draw (high 16, signed)
-    int range;     // lo (low 16) | hi (high 16)
-    int upd;       // bit 0: unreliable with a non-empty range; bit 1: cur is a candidate; bit 2: cur + draw is
-    int rcur;      // the start value as a neighbour candidate: roundf(cur) when cur >= 0, else -1
-    int pad1;
+    int range;     // lo (low 16) | hi - 1 (high 16)
 };
 
 template <bool C64>
@@ -241,34 +239,36 @@ __global__ void refine_prep_kernel(CostCtx c, int fwd, const uint8_t* __restrict
         const int y = fwd ? v : h - 1 - v;
         const int i = y * w + x;
         RStep st;
-        st.cur = work[i];
+        const float cur = work[i];
         const int lo = c.rmin[i], hi = c.rmax[i];
-        st.range = (lo & 0xFFFF) | (hi << 16);
-        st.upd = (!reliable[i] && hi > lo) ? 1 : 0;
-        int d_cur = 0, d_draw = 0;
-        st.c_cur = st.c_draw = 1e9f;
-        st.rcur = st.cur >= 0.f ? (int)roundf(st.cur) : -1;
-        st.pad1 = 0;
-        if (st.upd && st.cur >= 0.f) {
+        st.range = (lo & 0xFFFF) | ((hi - 1) << 16);
+        st.c_draw = 1e9f;
+        int d_cur, d_draw = 0;
+        if (reliable[i] || hi <= lo) {
+            st.c_cur = __int_as_float(0xff800000);
+            d_cur = cur >= 0.f ? (int)roundf(cur) : -1;
+        } else if (cur >= 0.f) {
             const RPack<C64> l = lp[i];
-            d_cur = min(max((int)roundf(st.cur), lo), hi - 1);
+            d_cur = min(max((int)roundf(cur), lo), hi - 1);
             st.c_cur = cand_cost<C64>(c, s_lut, l, rp, x, y, d_cur, lo, hi);
-            st.upd |= 2;
             const unsigned q = (unsigned)prefix[fwd ? i : n - 1 - i];
-            const float dv = __fadd_rn(st.cur, (float)draw_value[accepted_index(P, q, rej, nrej)]);
+            const float dv = __fadd_rn(cur, (float)draw_value[accepted_index(P, q, rej, nrej)]);
             if (dv >= 0.f) {
                 d_draw = min(max((int)roundf(dv), lo), hi - 1);
                 st.c_draw = cand_cost<C64>(c, s_lut, l, rp, x, y, d_draw, lo, hi);
-                st.upd |= 4;
             }
+        } else {
+            st.c_cur = 1e9f;
+            d_cur = lo;
         }
         st.d_pack = (d_cur & 0xFFFF) | (d_draw << 16);
         steps[j] = st;
     }
 }
 
-constexpr int kRing = 16;  // steps of pixel records in flight per lane
-constexpr int kAhead = 32; // steps ahead the right-image window is prefetched into L1
+constexpr int kSlots = 4;               // chunks of pixel records in flight
+constexpr int kRing = kSlots * kChunk;  // the same in steps
+constexpr int kAhead = 64;              // steps ahead the right-image window is prefetched into L1
 
 __device__ __forceinline__ void prefetch_l1(const void* p) {
     asm volatile("prefetch.global.L1 [%0];\n" ::"l"(p));
@@ -298,7 +298,7 @@ __device__ __forceinline__ void cp16(void* dst, const void* src) {
 // acquire) -> the next band's link warp, which is the order the reference's in-place raster scan
 // implies for the row above.
 constexpr int kUpRing = 128;
-struct BandLink {
+struct __align__(16) BandLink {
     int up[kUpRing];    // row above the band as neighbour candidates (roundf(value) when value >= 0,
                         // else -1): column c at up[c & (kUpRing - 1)]
     int avail;          // columns [0, avail) of the row above are in `up` (link warp)
@@ -439,14 +439,14 @@ template <bool C64>
 struct BandRing {
     RStep rec[kRing][32];       // step t's records in slot t % kRing, one per lane
     RPack<C64> lpk[kRing][32];  // and the lanes' packed left pixels
-    uint64_t full[kRing];       // slot filled (32 loader arrivals, each once its copies landed)
-    uint64_t empty[kRing];      // slot read (one arrival of the compute warp)
+    uint64_t full[kSlots];      // chunk filled (32 loader arrivals, each once its copies landed)
+    uint64_t empty[kSlots];     // chunk read (one arrival of the compute warp)
     int stop;                   // the compute warp has stopped: the loader stops too
 };
 
-// The loader warp: copies step t's records, packed left pixels and (WIN) the window's entering
-// right-image pixels into slot t % kRing and signals full[slot] when they have landed, up to
-// kRing steps ahead of the compute warp, refilling a slot only once the compute warp has released
+// The loader warp: copies a chunk's records, packed left pixels and (WIN) the window's entering
+// right-image pixels into its slot and signals full[slot] when they have landed, up to kSlots
+// chunks ahead of the compute warp, refilling a slot only once the compute warp has released
 // it.  Without WIN it keeps the right-image window warm in L1 instead: every lane misses L1 at a
 // different step and the compute warp waits for the slowest, so the window's first kAhead steps
 // are prefetched first and its entering edge kAhead steps ahead of the copies.
@@ -467,35 +467,57 @@ __device__ void band_loader(const CostCtx& c, const BandRow<C64>& r, BandRing<C6
     if (!WIN && r.ok) {
         for (int k = -c.D; k <= kAhead; k += 8) prefetch_l1(r.right + min(max(r.xb + r.xs * k - r.eoff, 0), w - 1));
     }
-    int pe = r.xb + r.xs * (kAhead - lane) - r.eoff;  // entering pixel kAhead steps ahead
-    const int nsteps = w + kBand - 1;
-    for (int t = 0; t < nsteps; ++t) {
-        const int slot = t % kRing;
-        if (t >= kRing &&
-            !mbar_wait_warp(&ring->empty[slot], ((t / kRing) - 1) & 1, spin_limit, &ring->stop, 64))
+    const int nchunks = (w + kBand - 1 + kChunk - 1) / kChunk;
+    for (int k = 0; k < nchunks; ++k) {
+        const int slot = k % kSlots;
+        if (k >= kSlots &&
+            !mbar_wait_warp(&ring->empty[slot], ((k / kSlots) - 1) & 1, spin_limit, &ring->stop, 32))
             break;  // the compute warp stopped, or never released the slot: it fails the pass itself
-        const int u = t - lane;
-        if (r.ok && u >= 0 && u < w) {
-            const RStep* src = r.steps + u;
-            cp16(&ring->rec[slot][lane], src);
-            cp16(reinterpret_cast<unsigned char*>(&ring->rec[slot][lane]) + 16,
-                 reinterpret_cast<const unsigned char*>(src) + 16);
-            const RPack<C64>* ls = r.left + (r.xb + r.xs * u);
-            if constexpr (C64) {
-                cp16(&ring->lpk[slot][lane], ls);
-            } else {
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(smem_u32(&ring->lpk[slot][lane])),
-                             "l"(ls));
+#pragma unroll
+        for (int i = 0; i < kChunk; ++i) {
+            const int u = k * kChunk + i - lane;
+            RStep* rec = &ring->rec[slot * kChunk + i][lane];
+            RPack<C64>* lpk = &ring->lpk[slot * kChunk + i][lane];
+            if (r.ok && u >= 0 && u < w) {
+                cp16(rec, r.steps + u);
+                const RPack<C64>* ls = r.left + (r.xb + r.xs * u);
+                if constexpr (C64) {
+                    cp16(lpk, ls);
+                } else {
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(smem_u32(lpk)), "l"(ls));
+                }
             }
+            // the window pixel entering at this column (also for the columns before the lane's first)
+            if (WIN && r.ok && u < w) copy_win(u);
+            if (!WIN && r.ok) prefetch_l1(r.right + min(max(r.xb + r.xs * (u + kAhead) - r.eoff, 0), w - 1));
         }
-        // the window pixel entering at this column (also for the columns before the lane's first)
-        if (WIN && r.ok && u < w) copy_win(u);
-        if (!WIN && r.ok) prefetch_l1(r.right + min(max(pe, 0), w - 1));
-        pe += r.xs;
         mbar_arrive_copies(&ring->full[slot]);
     }
     // no copy may land after the block has left
     asm volatile("cp.async.wait_all;\n" ::: "memory");
+}
+
+// A packed pixel taken apart for the step's cost: gray, and |gx|, |gy| as halves.
+template <bool C64>
+struct Split {
+    decltype(RPack<C64>::c) c;
+    int gray;
+    uint32_t gxy;
+    __device__ __forceinline__ explicit Split(const RPack<C64>& p)
+        : c(p.c), gray((int)(p.g & 0xFFu)), gxy(__byte_perm(p.g, 0u, 0x4241)) {}
+};
+// packed_cost with every table read: the entries of a term the configuration leaves out are zero, and
+// adding zero changes no sum.
+template <bool C64>
+__device__ __forceinline__ float split_cost(const float* lut, const Split<C64>& l, const RPack<C64>& rp) {
+    const Split<C64> r(rp);
+    int pop;
+    if constexpr (C64) pop = __popcll(l.c ^ r.c);
+    else pop = __popc(l.c ^ r.c);
+    const uint32_t dg = __vmaxs2(l.gxy, r.gxy) - __vmins2(l.gxy, r.gxy);  // |dgx| | |dgy| << 16
+    const float a = lut[kLutCensus + pop], b = lut[kLutAd + abs(l.gray - r.gray)];
+    const float g = lut[kLutGrad + __dp4a(dg, 0x00010001u, 0u)];
+    return __fadd_rn(__fadd_rn(a, b), g);
 }
 
 // WIN: each lane's right-image window ([x - dmax + 1, x - d0] of its row, sliding one pixel per
@@ -505,6 +527,12 @@ __device__ void band_loader(const CostCtx& c, const BandRow<C64>& r, BandRing<C6
 // Without WIN they are global loads kept warm in L1 by the loader's prefetches.  Three warps per block: warp 0 computes, warp 1
 // links the band to its neighbours (band_link), warp 2 loads the step ring (band_loader), so that
 // no copy or address arithmetic sits in the compute warp's step.
+//
+// Bound: the step's dependent chain -- neighbour shuffle, clamp, window load, table loads, two adds,
+// four selects, about 150 cycles -- times w + h steps a pass.  Everything else is kept off the step:
+// waits, hand-overs and publications come once per chunk of eight steps, the chunk's steps are one
+// straight line of code without divergent branches (a pixel that is not updated takes the same
+// selection, see RStep), and its records load ahead of the chain.
 template <bool C64, bool WIN>
 __global__ void __launch_bounds__(96) refine_band_kernel(CostCtx c, int fwd, const RStep* __restrict__ steps,
                                                          const RPack<C64>* __restrict__ lp,
@@ -512,7 +540,7 @@ __global__ void __launch_bounds__(96) refine_band_kernel(CostCtx c, int fwd, con
                                                          int* progress, int* err, int spin_limit, int wmask) {
     __shared__ float s_lut[kLutSize];
     __shared__ __align__(16) BandRing<C64> s_ring;
-    __shared__ BandLink s_link;
+    __shared__ __align__(16) BandLink s_link;
     for (int i = threadIdx.x; i < kLutSize; i += blockDim.x) s_lut[i] = c.lut[i];
     if (threadIdx.x == 0) {
         s_link.avail = 0;
@@ -520,7 +548,7 @@ __global__ void __launch_bounds__(96) refine_band_kernel(CostCtx c, int fwd, con
         s_link.done = 0;
         s_link.abort = 0;
         s_ring.stop = 0;
-        for (int i = 0; i < kRing; ++i) {
+        for (int i = 0; i < kSlots; ++i) {
             mbar_init(&s_ring.full[i], 32);
             mbar_init(&s_ring.empty[i], 1);
         }
@@ -543,27 +571,29 @@ __global__ void __launch_bounds__(96) refine_band_kernel(CostCtx c, int fwd, con
         return;
     }
     volatile BandLink* link = &s_link;
-    const int lane = r.lane, v = r.v;
-    const bool row_ok = r.ok;
-    float* wrow = r.work;
-    const RPack<C64>* rrow = r.right;
+    const int lane = r.lane;
+    const int wl = r.ok ? w : 0;  // columns of this lane's row
     // Neighbour values travel as candidates: roundf(value) when value >= 0, else -1 (the
-    // reference takes a neighbour only when it is non-negative, rounded).  An updated value is an
-    // integer already; a start value's candidate comes with its record.
+    // reference takes a neighbour only when it is non-negative, rounded).
     int prev = -1;  // candidate of this lane's previous column (its left neighbour)
     int avail = band > 0 ? 0 : w;  // columns of the row above known to be in the link's ring
     bool abort = false;
-    for (int t = 0; t < w + kBand - 1; ++t) {
-        int up_first = -1;  // the row above at column t (lane 0's up neighbour)
-        if (band > 0 && t < w) {
-            if (t >= avail) {
-                // wait until the link warp has the row above at least up to column t (lane 0
-                // polls, so that the warp decides together)
+    const int nchunks = (w + kBand - 1 + kChunk - 1) / kChunk;
+    for (int k = 0; k < nchunks; ++k) {
+        const int t0 = k * kChunk;
+        int up_first[kChunk];  // the row above at columns t0 .. (lane 0's up neighbours)
+#pragma unroll
+        for (int i = 0; i < kChunk; ++i) up_first[i] = -1;
+        if (band > 0 && t0 < w) {
+            const int need = min(t0 + kChunk, w);
+            if (avail < need) {
+                // wait until the link warp has the chunk's columns of the row above (lane 0 polls, so
+                // that the warp decides together)
                 int spins = 0, state = 0;  // 1: available, 2: gave up
                 for (;;) {
                     if (lane == 0) {
                         const int a = link->avail;
-                        state = a > t ? 1 : ((link->abort || ++spins > spin_limit) ? 2 : 0);
+                        state = a >= need ? 1 : ((link->abort || ++spins > spin_limit) ? 2 : 0);
                         if (state == 1) avail = a;
                     }
                     state = __shfl_sync(0xffffffffu, state, 0);
@@ -578,62 +608,66 @@ __global__ void __launch_bounds__(96) refine_band_kernel(CostCtx c, int fwd, con
                 }
                 __threadfence_block();
             }
-            if (lane == 0) up_first = s_link.up[t & (kUpRing - 1)];
+            const int4* up4 = reinterpret_cast<const int4*>(&s_link.up[t0 & (kUpRing - 1)]);
+#pragma unroll
+            for (int i = 0; i < kChunk; i += 4) {
+                const int4 q = up4[i / 4];
+                up_first[i] = q.x; up_first[i + 1] = q.y; up_first[i + 2] = q.z; up_first[i + 3] = q.w;
+            }
         }
-        // step t's slot has landed
-        const int slot = t % kRing;
-        if (!mbar_wait_warp(&s_ring.full[slot], (t / kRing) & 1, spin_limit, nullptr, 0)) {
+        // the chunk's slot has landed
+        const int slot = k % kSlots;
+        if (!mbar_wait_warp(&s_ring.full[slot], (k / kSlots) & 1, spin_limit, nullptr, 0)) {
             abort = true;
             if (lane == 0) atomicExch(err, 1);
             break;
         }
-        const int up_lane = __shfl_up_sync(0xffffffffu, prev, 1);
-        const int u = t - lane;
-        if (row_ok && u >= 0 && u < w) {
-            const RStep st = s_ring.rec[slot][lane];
-            int cand = st.rcur;
-            if (st.upd & 1) {
-                const int x = r.xb + r.xs * u;
-                const int lo = (int)(short)(st.range & 0xFFFF), hi = st.range >> 16;
-                const int d_cur = (int)(short)(st.d_pack & 0xFFFF), d_draw = st.d_pack >> 16;
-                const bool has_cur = (st.upd & 2) != 0, has_draw = (st.upd & 4) != 0;
-                const RPack<C64> l = s_ring.lpk[slot][lane];
-                // dynamic candidates: left (forward) / right (backward) and up / down
-                const int left = u > 0 ? prev : -1;
-                const int up = v > 0 ? (lane > 0 ? up_lane : up_first) : -1;
-                const bool has_l = left >= 0, has_u = up >= 0;
-                // clamped into [lo, hi - 1] (hi > lo for an updated pixel), so only x - d needs a test
-                const int dl = has_l ? min(max(left, lo), hi - 1) : 0;
-                const int du = has_u ? min(max(up, lo), hi - 1) : 0;
-                const int xl = x - dl, xu = x - du;
-                const float cl = (has_l && (unsigned)xl < (unsigned)w)
-                                     ? packed_cost<C64>(c, s_lut, l, WIN ? s_win[(xl & wmask) * kBand] : rrow[xl])
-                                     : 1e6f;
-                const float cu = (has_u && (unsigned)xu < (unsigned)w)
-                                     ? packed_cost<C64>(c, s_lut, l, WIN ? s_win[(xu & wmask) * kBand] : rrow[xu])
-                                     : 1e6f;
-                // the reference's order: cur, left, up, cur + draw; the first strict minimum wins
-                float best_c = 1e9f;
-                int best_d = st.cur >= 0.f ? d_cur : lo;
-                if (has_cur && st.c_cur < best_c) { best_c = st.c_cur; best_d = d_cur; }
-                if (has_l && cl < best_c) { best_c = cl; best_d = dl; }
-                if (has_u && cu < best_c) { best_c = cu; best_d = du; }
-                if (has_draw && st.c_draw < best_c) { best_c = st.c_draw; best_d = d_draw; }
-                wrow[x] = (float)best_d;
-                cand = best_d >= 0 ? best_d : -1;
+        const RStep* recs = &s_ring.rec[slot * kChunk][lane];
+        const RPack<C64>* lpks = &s_ring.lpk[slot * kChunk][lane];
+        const int u0 = t0 - lane, x0 = r.xb + r.xs * u0;
+#pragma unroll
+        for (int i = 0; i < kChunk; ++i) {
+            const int up_lane = __shfl_up_sync(0xffffffffu, prev, 1);
+            const int up = lane > 0 ? up_lane : up_first[i];
+            const RStep st = recs[i * 32];
+            const Split<C64> l(lpks[i * 32]);
+            const int x = x0 + r.xs * i;
+            const int lo = (int)(short)(st.range & 0xFFFF), hi1 = st.range >> 16;
+            // dynamic candidates: left (forward) / right (backward) and up / down, clamped into the
+            // range, so only x - d needs a test
+            const int dl = min(max(prev, lo), hi1), du = min(max(up, lo), hi1);
+            const int xl = x - dl, xu = x - du;
+            const bool in_l = (unsigned)xl < (unsigned)w, in_u = (unsigned)xu < (unsigned)w;
+            RPack<C64> pl, pu;
+            if constexpr (WIN) {
+                pl = s_win[(xl & wmask) * kBand];
+                pu = s_win[(xu & wmask) * kBand];
+            } else {
+                pl = r.right[in_l ? xl : 0];
+                pu = r.right[in_u ? xu : 0];
             }
-            prev = cand;
+            float cl = in_l ? split_cost<C64>(s_lut, l, pl) : 1e6f;
+            float cu = in_u ? split_cost<C64>(s_lut, l, pu) : 1e6f;
+            cl = prev >= 0 ? cl : 1e30f;
+            cu = up >= 0 ? cu : 1e30f;
+            // the reference's order: cur, left, up, cur + draw; the first strict minimum wins
+            float best_c = st.c_cur;
+            int best_d = (int)(short)(st.d_pack & 0xFFFF);
+            if (cl < best_c) { best_c = cl; best_d = dl; }
+            if (cu < best_c) { best_c = cu; best_d = du; }
+            if (st.c_draw < best_c) best_d = st.d_pack >> 16;
+            const bool on = (unsigned)(u0 + i) < (unsigned)wl;
+            if (on && st.c_cur != __int_as_float(0xff800000)) r.work[x] = (float)best_d;
+            prev = on ? max(best_d, -1) : -1;
         }
         // every lane has read the slot (and its window pixels): the loader may refill it
         __syncwarp();
         if (lane == 0) mbar_arrive(&s_ring.empty[slot]);
-        if ((t % kPublish) == kPublish - 1) {
-            // release to the link warp (CTA scope): how far the last row (lane 31, column t - 31)
-            // is final, and that the ring's columns up to t are read
-            __threadfence_block();
-            if (lane == kBand - 1) link->done = max(0, min(t - (kBand - 1) + 1, w));
-            if (lane == 0) link->used = min(t + 1, w);
-        }
+        // release to the link warp (CTA scope): how far the last row (lane 31, column t - 31) is
+        // final, and that the ring's columns of this chunk are read
+        __threadfence_block();
+        if (lane == kBand - 1) link->done = max(0, min(t0 + kChunk - (kBand - 1), w));
+        if (lane == 0) link->used = min(t0 + kChunk, w);
     }
     if (abort) *(volatile int*)&s_ring.stop = 1;
     __syncwarp();
