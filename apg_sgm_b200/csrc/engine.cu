@@ -270,7 +270,7 @@ Layout Engine::make_layout(const apg_pipeline_config_t& c, int w, int h, int ch,
         L.rf_scan_tmp = take(L.rf_scan_tmp_bytes);
         L.rf_state = take((size_t)(kRefineProgWord + refine_band_count(h)) * 4);
         L.rf_pack = take(refine_pack_bytes((int)n, c.census_type == APG_CENSUS_9X7));
-        L.rf_steps = take(refine_steps_bytes((int)n));
+        L.rf_steps = take(refine_steps_bytes(w, h, L.D, c.census_type == APG_CENSUS_9X7));
     }
     L.total = o;
     return L;

@@ -321,7 +321,7 @@ cudaError_t launch_refine_count(const Layout& L, unsigned char* arena, const flo
 cudaError_t launch_refine_pack(const CostCtx& c, const Layout& L, unsigned char* arena, cudaStream_t s,
                                unsigned* launches);
 size_t refine_pack_bytes(int n, bool c64);
-size_t refine_steps_bytes(int n);
+size_t refine_steps_bytes(int w, int h, int D, bool c64);
 cudaError_t launch_refine_pass(const CostCtx& c, const Layout& L, unsigned char* arena, const RefineTables& tab,
                                int it, float* work, const RefineTuning& tune, cudaStream_t s, unsigned* launches);
 size_t refine_scan_temp_bytes(int n);

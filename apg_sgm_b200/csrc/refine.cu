@@ -8,11 +8,15 @@
 // (pass-order) rows, lane i row i, and walks the columns with lane i one column behind lane i-1:
 // at step t lane i updates column t - i, so its up neighbour is what lane i-1 produced at step
 // t-1 (one shuffle) and its left neighbour is its own previous value.  The first row of a band
-// reads the row above from global memory once the band above has published, through a progress
-// counter, that its last row is final that far; the bands therefore run as a wavefront about 40
-// columns apart and a pass takes about w + h steps.  Every wait is bounded: on timeout the band
-// sets an error flag (read by the host) and stops.  This is exactly the reference's
-// read-after-write order.
+// takes the row above from the band above, eight columns at a time: through the shared memory of the
+// thread-block cluster the two bands run in, or between clusters through global memory and a progress
+// counter.  The bands run as a wavefront about 48 steps apart and a pass takes about w + 1.5 h steps.
+// Every wait is bounded: on timeout the band sets an error flag (read by the host) and stops.  This is
+// exactly the reference's read-after-write order.
+//
+// Measured (one B200, all three passes of HighQuality with their per-pixel kernels): 1920x1080 D256
+// 1.97 ms, 1280x720 D128 1.27 ms, where steps with divergent branches, per-step hand-overs by polling
+// and per-lane copies took 5.61 and 3.70 ms; a step costs about 300 cycles.
 //
 // Random draws: a pixel consumes a draw when it is unreliable, has a non-empty range and holds a
 // non-negative value at the start of the pass, so its draw index is an exclusive prefix count of
@@ -201,18 +205,22 @@ __device__ __forceinline__ float packed_cost(const CostCtx& c, const float* lut,
 }
 
 // Everything about one pixel of a pass that does not depend on the wavefront, computed for all
-// pixels at once before the pass and laid out in pass order (index v * w + u): its range and the two
-// static candidates -- the current value and the current value plus the pixel's draw -- with their
+// pixels at once before the pass and laid out in wavefront order: its range and the two static
+// candidates -- the current value and the current value plus the pixel's draw -- with their
 // costs.  The band kernel only costs the two dynamic candidates (left and up neighbours) and keeps
 // the reference's candidate order.  A pixel the pass does not update carries the cost -infinity and
 // its value as a neighbour candidate (roundf(value) when value >= 0, else -1), so the same selection
 // returns it; an updated pixel without a value carries the cost 1e9 and the start of its range.
+// The pixel's packed left image rides along.
+template <bool C64>
 struct __align__(16) RStep {
     float c_cur;   // cost of candidate d_cur
     float c_draw;  // cost of candidate d_draw (1e9: none)
-    int d_pack;    // d_cur (low 16, signed) | d_draw (high 16, signed)
-    int range;     // lo (low 16) | hi - 1 (high 16)
+    int lo, hi1;   // the range's first and last disparity
+    int d_cur, d_draw;
+    RPack<C64> left;
 };
+static_assert(sizeof(RStep<false>) == 32 && sizeof(RStep<true>) == 48, "bulk copies of whole records");
 
 template <bool C64>
 __device__ __forceinline__ float cand_cost(const CostCtx& c, const float* lut, const RPack<C64>& l,
@@ -222,52 +230,82 @@ __device__ __forceinline__ float cand_cost(const CostCtx& c, const float* lut, c
     return 1e6f;
 }
 
-template <bool C64>
-__global__ void refine_prep_kernel(CostCtx c, int fwd, const uint8_t* __restrict__ reliable,
+// Wavefront order: the records and right-image pixels of a band's step lie together, lane
+// by lane ([band][step][lane]), so a chunk of steps is one contiguous bulk copy each.  The right pixels
+// start wave_lead(D) steps before the first step: the window of the first columns.
+__host__ __device__ inline int wave_chunks(int w) { return (w + kBand - 1 + kChunk - 1) / kChunk; }
+__host__ __device__ inline int wave_lead(int D) { return (D - 1 + kChunk - 1) / kChunk * kChunk; }
+
+// A window pixel outside the image: its byte 3 against a left pixel's 0 takes the gradient index past
+// kGradIn, where the table holds 1e30.
+constexpr uint32_t kOutside = 0xFF000000u;
+constexpr uint32_t kGradWeights = 0x03010100u;  // index = |dgx| + |dgy| + 3 * byte 3
+constexpr int kGradIn = 511, kGradAll = 3 * 255 + kGradIn;
+
+// One pixel record per (band, step, lane), neutral where the lane has no pixel at that step, and the
+// right-image pixel that enters its window at that step (column u of a row brings image column
+// x(u) - eoff).
+template <bool C64, bool WIN>
+__global__ void __launch_bounds__(256) refine_prep_kernel(CostCtx c, int fwd, const uint8_t* __restrict__ reliable,
                                    const int* __restrict__ prefix, const int16_t* __restrict__ draw_value,
                                    const unsigned* __restrict__ rej, int nrej, const unsigned* __restrict__ P_ptr,
                                    const RPack<C64>* __restrict__ lp, const RPack<C64>* __restrict__ rp,
-                                   const float* __restrict__ work, RStep* __restrict__ steps) {
+                                   const float* __restrict__ work, RStep<C64>* __restrict__ steps,
+                                   RPack<C64>* __restrict__ wr) {
     __shared__ float s_lut[kLutSize];
     for (int i = threadIdx.x; i < kLutSize; i += blockDim.x) s_lut[i] = c.lut[i];
     __syncthreads();
     const int w = c.w, h = c.h, n = w * h;
     const unsigned P = *P_ptr;
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-        const int v = j / w, u = j - v * w;
+    const int lead = WIN ? wave_lead(c.D) : 0, nstep = wave_chunks(w) * kChunk, tt = lead + nstep;
+    const int nbands = (h + kBand - 1) / kBand;
+    const int eoff = fwd ? c.d0 : c.d0 + c.D - 1;
+    const int lane = threadIdx.x & 31, per = blockDim.x >> 5;
+    for (int j = blockIdx.x * per + (threadIdx.x >> 5); j < nbands * tt; j += gridDim.x * per) {
+        const int band = j / tt, t = j - band * tt - lead;
+        const int v = band * kBand + lane, u = t - lane;
         const int x = fwd ? u : w - 1 - u;
         const int y = fwd ? v : h - 1 - v;
-        const int i = y * w + x;
-        RStep st;
-        const float cur = work[i];
-        const int lo = c.rmin[i], hi = c.rmax[i];
-        st.range = (lo & 0xFFFF) | ((hi - 1) << 16);
-        st.c_draw = 1e9f;
-        int d_cur, d_draw = 0;
-        if (reliable[i] || hi <= lo) {
-            st.c_cur = __int_as_float(0xff800000);
-            d_cur = cur >= 0.f ? (int)roundf(cur) : -1;
-        } else if (cur >= 0.f) {
-            const RPack<C64> l = lp[i];
-            d_cur = min(max((int)roundf(cur), lo), hi - 1);
-            st.c_cur = cand_cost<C64>(c, s_lut, l, rp, x, y, d_cur, lo, hi);
-            const unsigned q = (unsigned)prefix[fwd ? i : n - 1 - i];
-            const float dv = __fadd_rn(cur, (float)draw_value[accepted_index(P, q, rej, nrej)]);
-            if (dv >= 0.f) {
-                d_draw = min(max((int)roundf(dv), lo), hi - 1);
-                st.c_draw = cand_cost<C64>(c, s_lut, l, rp, x, y, d_draw, lo, hi);
-            }
-        } else {
-            st.c_cur = 1e9f;
-            d_cur = lo;
+        if constexpr (WIN) {
+            const int pe = x - eoff;
+            RPack<C64> e = {};
+            e.g = kOutside;
+            if (v < h && (unsigned)pe < (unsigned)w) e = rp[(size_t)y * w + pe];
+            wr[(size_t)j * 32 + lane] = e;
+            if (t < 0) continue;
         }
-        st.d_pack = (d_cur & 0xFFFF) | (d_draw << 16);
-        steps[j] = st;
+        RStep<C64> st = {};
+        st.c_cur = __int_as_float(0xff800000);
+        st.c_draw = 1e9f;
+        st.d_cur = -1;
+        if (v < h && (unsigned)u < (unsigned)w) {
+            const int i = y * w + x;
+            const float cur = work[i];
+            const int lo = c.rmin[i], hi = c.rmax[i];
+            st.left = lp[i];
+            st.lo = lo;
+            st.hi1 = hi - 1;
+            if (reliable[i] || hi <= lo) {
+                if (cur >= 0.f) st.d_cur = (int)roundf(cur);
+            } else if (cur >= 0.f) {
+                st.d_cur = min(max((int)roundf(cur), lo), hi - 1);
+                st.c_cur = cand_cost<C64>(c, s_lut, st.left, rp, x, y, st.d_cur, lo, hi);
+                const unsigned q = (unsigned)prefix[fwd ? i : n - 1 - i];
+                const float dv = __fadd_rn(cur, (float)draw_value[accepted_index(P, q, rej, nrej)]);
+                if (dv >= 0.f) {
+                    st.d_draw = min(max((int)roundf(dv), lo), hi - 1);
+                    st.c_draw = cand_cost<C64>(c, s_lut, st.left, rp, x, y, st.d_draw, lo, hi);
+                }
+            } else {
+                st.c_cur = 1e9f;
+                st.d_cur = lo;
+            }
+        }
+        steps[((size_t)band * nstep + t) * 32 + lane] = st;
     }
 }
 
-constexpr int kSlots = 4;               // chunks of pixel records in flight
-constexpr int kRing = kSlots * kChunk;  // the same in steps
+constexpr int kRing = 4 * kChunk;       // steps of pixel records in flight, at most
 constexpr int kAhead = 64;              // steps ahead the right-image window is prefetched into L1
 
 __device__ __forceinline__ void prefetch_l1(const void* p) {
@@ -279,101 +317,24 @@ __device__ __forceinline__ void prefetch_l1(const void* p) {
 // counter and fences before reading the row above.
 __device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;\n" ::: "memory"); }
 
-// The loader warp's copies into the step ring carry no compiler memory clobber: their order
-// against the compute warp's reads is set by the ring's mbarriers (a slot is refilled only after
-// the wait for its empty barrier, and read only after the wait for its full barrier).
-__device__ __forceinline__ void cp16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
-                 "l"(src));
-}
+// The row above a band, as neighbour candidates (roundf(value) when value >= 0, else -1): column u at
+// up[u + kUpShift], with one single-use mbarrier per kChunk positions.  The shift puts the columns a
+// band's last lane finishes in one chunk (column t - 31 at step t) on one barrier and one 32-byte line.
+constexpr int kUpShift = (kBand - 1) % kChunk;
+__host__ __device__ inline int up_blocks(int w) { return (w + kUpShift - 1) / kChunk + 1; }
 
-// Shared state of one band's two warps.  The compute warp (warp 0) walks the band; the link warp
-// (warp 1) carries every exchange with the other bands, so that no GPU-scope fence or L2 round
-// trip sits in the compute warp's step loop:
-//   * it polls the band above's progress counter and copies the newly final columns of that
-//     band's last row into `up` (a ring of kUpRing columns), then raises `avail`;
-//   * it publishes how far this band's last row is final (`done`, raised by the compute warp at
-//     CTA scope) to this band's progress counter, behind a GPU-scope fence.
-// Causality runs compute warp -> (CTA-scope release / acquire) -> link warp -> (GPU-scope release /
-// acquire) -> the next band's link warp, which is the order the reference's in-place raster scan
-// implies for the row above.
-constexpr int kUpRing = 128;
-struct __align__(16) BandLink {
-    int up[kUpRing];    // row above the band as neighbour candidates (roundf(value) when value >= 0,
-                        // else -1): column c at up[c & (kUpRing - 1)]
-    int avail;          // columns [0, avail) of the row above are in `up` (link warp)
-    int used;           // columns [0, used) of `up` are no longer read (compute warp)
-    int done;           // columns [0, done) of the band's last row are final in `work` (compute warp)
-    int abort;          // the link warp gave up waiting (or saw the error word): the compute warp stops
+// Shared state between the compute warp (warp 0) and the link warp (warp 1) of a band at the edge of a
+// cluster.  Inside a cluster a band's compute warp sends its last row straight into the next band's
+// shared memory (st.async, which completes on the receiver's barriers).  Between clusters the link warps
+// carry the exchange, so that no GPU-scope fence or L2 round trip sits in the compute warp's steps:
+//   * the link warp of a cluster's first band polls the band above's progress counter, copies the newly
+//     final columns of that band's last row into `up` and arrives on their barriers;
+//   * that of a cluster's last band publishes how far the last row is final (`done`, raised by the
+//     compute warp at CTA scope) to the band's progress counter, behind a GPU-scope fence.
+struct BandLink {
+    int done;   // columns [0, done) of the band's last row are final in `work` (compute warp)
+    int abort;  // the link warp gave up waiting (or saw the error word): the compute warp stops
 };
-
-// The link warp of band `band` (see BandLink).  Every wait is bounded: after spin_limit polls in
-// which nothing moved it sets the error word and `abort`, and after as many again it leaves.
-__device__ void band_link(BandLink* s_link, int band, int w, int h, int fwd, const float* work, int* progress,
-                          int* err, int spin_limit) {
-    const int lane = threadIdx.x & 31;
-    volatile BandLink* L = s_link;
-    volatile int* vprog = progress;
-    const int xs = fwd ? 1 : -1, xb = fwd ? 0 : w - 1;
-    const int y_above = band > 0 ? (fwd ? band * kBand - 1 : h - band * kBand) : 0;
-    const float* above = work + (size_t)y_above * w;
-    int fetched = band > 0 ? 0 : w;  // columns of the row above copied into the ring
-    int published = 0;
-    int idle = 0;
-    bool gave_up = false;
-    for (;;) {
-        bool moved = false;
-        // this band's last row, as far as the compute warp has released it
-        const int done = L->done;
-        if (done > published) {
-            if (lane == 0) {
-                fence_acq_rel();
-                vprog[band] = done;
-            }
-            published = done;
-            moved = true;
-        }
-        if (published >= w) break;
-        // the row above, as far as the band above has published it and the ring has room
-        if (fetched < w && !gave_up) {
-            int prog = 0;
-            if (lane == 0) prog = vprog[band - 1];
-            prog = __shfl_sync(0xffffffffu, prog, 0);
-            const int upto = min(min(prog, L->used + kUpRing), w);
-            if (upto > fetched) {
-                if (lane == 0) fence_acq_rel();
-                __syncwarp();
-                for (int col = fetched + lane; col < upto; col += 32) {
-                    const float a = __ldcg(above + (xb + xs * col));
-                    s_link->up[col & (kUpRing - 1)] = a >= 0.f ? (int)roundf(a) : -1;
-                }
-                __syncwarp();
-                if (lane == 0) {
-                    __threadfence_block();
-                    L->avail = upto;
-                }
-                fetched = upto;
-                moved = true;
-            }
-        }
-        if (moved) {
-            idle = 0;
-            continue;
-        }
-        ++idle;
-        if (!gave_up && (idle > spin_limit || *(volatile int*)err)) {
-            if (lane == 0) {
-                atomicExch(err, 1);
-                L->abort = 1;
-            }
-            gave_up = true;
-            idle = 0;
-        } else if (gave_up && idle > spin_limit) {
-            break;  // the compute warp did not finish either: leave (the frame is already failed)
-        }
-        __nanosleep(64);
-    }
-}
 
 // ---- the band kernel's step ring: mbarriers between the loader warp and the compute warp
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -382,10 +343,6 @@ __device__ __forceinline__ void mbar_init(uint64_t* b, unsigned count) {
 }
 __device__ __forceinline__ void mbar_arrive(uint64_t* b) {
     asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n}\n" ::"r"(smem_u32(b)) : "memory");
-}
-// arrives once every cp.async this thread issued before it has landed
-__device__ __forceinline__ void mbar_arrive_copies(uint64_t* b) {
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(smem_u32(b)) : "memory");
 }
 __device__ __forceinline__ bool mbar_done(uint64_t* b, unsigned parity) {
     unsigned ok;
@@ -407,273 +364,358 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* b, unsigned parity, int
     }
 }
 
-// Per-lane view of a band's row for one pass: pass-order column u of the lane's row is image
-// column xb + xs * u.
-template <bool C64>
-struct BandRow {
-    int lane, v, xs, xb, eoff;
-    bool ok;
-    const RStep* steps;       // this lane's records, pass order
-    const RPack<C64>* left;   // this lane's left pixels
-    const RPack<C64>* right;  // this lane's right-image row
-    float* work;
-    __device__ BandRow(const CostCtx& c, int band, int fwd, const RStep* all_steps, const RPack<C64>* lp,
-                       const RPack<C64>* rp, float* all_work) {
-        lane = threadIdx.x & 31;
-        v = band * kBand + lane;
-        ok = v < c.h;
-        xs = fwd ? 1 : -1;
-        xb = fwd ? 0 : c.w - 1;
-        const int yrow = fwd ? v : c.h - 1 - v;
-        const size_t rowoff = (size_t)(ok ? yrow : 0) * c.w;
-        steps = all_steps + (size_t)(ok ? v : 0) * c.w;
-        left = lp + rowoff;
-        right = rp + rowoff;
-        work = all_work + rowoff;
-        eoff = fwd ? c.d0 : c.d0 + c.D - 1;  // entering window pixel of column u: x(u) - eoff
-    }
-};
+__device__ __forceinline__ void mbar_expect(uint64_t* b, unsigned bytes) {
+    asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n}\n" ::"r"(smem_u32(b)), "r"(bytes)
+                 : "memory");
+}
+// contiguous copy of this GPU's global memory to shared memory, completing on b (16-byte multiples)
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned bytes, uint64_t* b) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(smem_u32(b))
+                 : "memory");
+}
+// the same shared-memory address in CTA `rank` of the cluster
+__device__ __forceinline__ unsigned peer_smem(unsigned addr, unsigned rank) {
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void st_async4(unsigned addr, int a, int b, int c, int d, unsigned bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];\n" ::"r"(addr),
+                 "r"(a), "r"(b), "r"(c), "r"(d), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;\n" ::: "memory");
+}
 
-// Shared memory of the band kernel besides the link state.
+// The link warp of a band that receives from (recv) or publishes to (send) another cluster.  Every wait
+// is bounded: after spin_limit polls in which nothing moved it sets the error word and `abort`, and after
+// as many again it leaves.
+__device__ void band_link(BandLink* s_link, int* s_up, uint64_t* upbar, int band, int w, int h, int fwd,
+                          const float* work, int* progress, int* err, int spin_limit, bool recv, bool send) {
+    const int lane = threadIdx.x & 31;
+    volatile BandLink* L = s_link;
+    volatile int* vprog = progress;
+    const int xs = fwd ? 1 : -1, xb = fwd ? 0 : w - 1;
+    const int y_above = recv ? (fwd ? band * kBand - 1 : h - band * kBand) : 0;
+    const float* above = work + (size_t)y_above * w;
+    int fetched = recv ? 0 : w;      // columns of the row above copied
+    int blocks = 0;                  // barriers arrived on
+    int published = send ? 0 : w;
+    int idle = 0;
+    bool gave_up = false;
+    for (;;) {
+        bool moved = false;
+        // this band's last row, as far as the compute warp has released it
+        const int done = L->done;
+        if (done > published) {
+            if (lane == 0) {
+                fence_acq_rel();
+                vprog[band] = done;
+            }
+            published = done;
+            moved = true;
+        }
+        if (published >= w && (fetched >= w || gave_up)) break;
+        // the row above, as far as the band above has published it
+        if (fetched < w && !gave_up) {
+            int prog = 0;
+            if (lane == 0) prog = vprog[band - 1];
+            prog = min(__shfl_sync(0xffffffffu, prog, 0), w);
+            if (prog > fetched) {
+                if (lane == 0) fence_acq_rel();
+                __syncwarp();
+                for (int col = fetched + lane; col < prog; col += 32) {
+                    const float a = __ldcg(above + (xb + xs * col));
+                    s_up[col + kUpShift] = a >= 0.f ? (int)roundf(a) : -1;
+                }
+                __syncwarp();
+                fetched = prog;
+                const int upto = fetched >= w ? up_blocks(w) : (fetched + kUpShift) / kChunk;
+                if (lane == 0) {
+                    __threadfence_block();
+                    for (int b = blocks; b < upto; ++b) mbar_arrive(&upbar[b]);
+                }
+                blocks = upto;
+                moved = true;
+            }
+        }
+        if (moved) {
+            idle = 0;
+            continue;
+        }
+        ++idle;
+        if (!gave_up && (idle > spin_limit || *(volatile int*)err)) {
+            if (lane == 0) {
+                atomicExch(err, 1);
+                L->abort = 1;
+            }
+            gave_up = true;
+            idle = 0;
+        } else if (gave_up && idle > spin_limit) {
+            break;  // the compute warp did not finish either: leave (the frame is already failed)
+        }
+        __nanosleep(32);
+    }
+}
+
+// Shared memory of the band kernel besides the row above and the window.
 template <bool C64>
 struct BandRing {
-    RStep rec[kRing][32];       // step t's records in slot t % kRing, one per lane
-    RPack<C64> lpk[kRing][32];  // and the lanes' packed left pixels
-    uint64_t full[kSlots];      // chunk filled (32 loader arrivals, each once its copies landed)
+    static constexpr int kSlots = C64 ? 2 : 4;    // chunks in flight
+    static_assert(kSlots * kChunk <= kRing, "the window ring covers the steps copied ahead");
+    RStep<C64> rec[kSlots * kChunk][32];          // chunk k's records in slot k % kSlots, one per step and lane
+    uint64_t full[kSlots];      // chunk filled (its bulk copies landed)
     uint64_t empty[kSlots];     // chunk read (one arrival of the compute warp)
     int stop;                   // the compute warp has stopped: the loader stops too
 };
 
-// The loader warp: copies a chunk's records, packed left pixels and (WIN) the window's entering
-// right-image pixels into its slot and signals full[slot] when they have landed, up to kSlots
-// chunks ahead of the compute warp, refilling a slot only once the compute warp has released
-// it.  Without WIN it keeps the right-image window warm in L1 instead: every lane misses L1 at a
-// different step and the compute warp waits for the slowest, so the window's first kAhead steps
-// are prefetched first and its entering edge kAhead steps ahead of the copies.
+// The loader warp: bulk copies of a chunk's records and (WIN) the right-image pixels that enter the window, which land on full[slot], up to kSlots chunks ahead of the compute warp, refilling a
+// slot only once the compute warp has released it.  Without WIN it keeps the right-image window warm in L1
+// instead: every lane misses L1 at a different step and the compute warp waits for the slowest, so the
+// window's first kAhead steps are prefetched first and its entering edge kAhead steps ahead of the copies.
 template <bool C64, bool WIN>
-__device__ void band_loader(const CostCtx& c, const BandRow<C64>& r, BandRing<C64>* ring, RPack<C64>* s_win,
-                            int wmask, int spin_limit) {
-    const int w = c.w, lane = r.lane;
-    auto copy_win = [&](int u) {
-        const int pe = r.xb + r.xs * u - r.eoff;
-        if ((unsigned)pe < (unsigned)w)
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(smem_u32(&s_win[(pe & wmask) * kBand])),
-                         "l"(r.right + pe));
-    };
-    if (WIN && r.ok) {
-        // the rest of the window of the lane's first column: columns -(D - 1) .. -lane - 1
-        for (int u = -(c.D - 1); u < -lane; ++u) copy_win(u);
-    }
-    if (!WIN && r.ok) {
-        for (int k = -c.D; k <= kAhead; k += 8) prefetch_l1(r.right + min(max(r.xb + r.xs * k - r.eoff, 0), w - 1));
-    }
-    const int nchunks = (w + kBand - 1 + kChunk - 1) / kChunk;
+__device__ void band_loader(const CostCtx& c, int band, int fwd, BandRing<C64>* ring, RPack<C64>* s_win, int wmask,
+                            const RStep<C64>* steps, const RPack<C64>* wr, const RPack<C64>* rp, int spin_limit) {
+    const int w = c.w, lane = threadIdx.x & 31;
+    const int nchunks = wave_chunks(w), nstep = nchunks * kChunk;
+    const int lead = WIN ? wave_lead(c.D) : 0;
+    const RStep<C64>* gs = steps + (size_t)band * nstep * 32;
+    const RPack<C64>* gr = wr + ((size_t)band * (lead + nstep) + lead) * 32;
+    constexpr int kSlots = BandRing<C64>::kSlots;
+    constexpr unsigned bs = kChunk * 32 * sizeof(RStep<C64>), bp = kChunk * 32 * sizeof(RPack<C64>);
+    const int v = band * kBand + lane, y = fwd ? v : c.h - 1 - v;
+    const int xs = fwd ? 1 : -1, xb = fwd ? 0 : w - 1, eoff = fwd ? c.d0 : c.d0 + c.D - 1;
+    const RPack<C64>* rrow = rp + (size_t)(v < c.h ? y : 0) * w;
+    if (!WIN)
+        for (int k = -c.D; k <= kAhead; k += 8) prefetch_l1(rrow + min(max(xb + xs * k - eoff, 0), w - 1));
+    int issued = 0;
     for (int k = 0; k < nchunks; ++k) {
         const int slot = k % kSlots;
         if (k >= kSlots &&
             !mbar_wait_warp(&ring->empty[slot], ((k / kSlots) - 1) & 1, spin_limit, &ring->stop, 32))
             break;  // the compute warp stopped, or never released the slot: it fails the pass itself
-#pragma unroll
-        for (int i = 0; i < kChunk; ++i) {
-            const int u = k * kChunk + i - lane;
-            RStep* rec = &ring->rec[slot * kChunk + i][lane];
-            RPack<C64>* lpk = &ring->lpk[slot * kChunk + i][lane];
-            if (r.ok && u >= 0 && u < w) {
-                cp16(rec, r.steps + u);
-                const RPack<C64>* ls = r.left + (r.xb + r.xs * u);
-                if constexpr (C64) {
-                    cp16(lpk, ls);
-                } else {
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(smem_u32(lpk)), "l"(ls));
-                }
+        if (lane == 0) {
+            const unsigned first = WIN && k == 0 ? (unsigned)lead * 32 * (unsigned)sizeof(RPack<C64>) : 0u;
+            mbar_expect(&ring->full[slot], bs + (WIN ? bp + first : 0u));
+            const size_t o = (size_t)k * kChunk * 32;
+            bulk_load(&ring->rec[slot * kChunk][0], gs + o, bs, &ring->full[slot]);
+            if (WIN) {
+                // the window ring holds step t's entering pixels at t & wmask
+                if (first) bulk_load(s_win + (size_t)(wmask + 1 - lead) * 32, gr - (size_t)lead * 32, first, &ring->full[slot]);
+                bulk_load(s_win + (size_t)((k * kChunk) & wmask) * 32, gr + o, bp, &ring->full[slot]);
             }
-            // the window pixel entering at this column (also for the columns before the lane's first)
-            if (WIN && r.ok && u < w) copy_win(u);
-            if (!WIN && r.ok) prefetch_l1(r.right + min(max(r.xb + r.xs * (u + kAhead) - r.eoff, 0), w - 1));
         }
-        mbar_arrive_copies(&ring->full[slot]);
+        issued = k + 1;
+        if (!WIN) {
+#pragma unroll
+            for (int i = 0; i < kChunk; ++i)
+                prefetch_l1(rrow + min(max(xb + xs * (k * kChunk + i - lane + kAhead) - eoff, 0), w - 1));
+        }
+        __syncwarp();
     }
-    // no copy may land after the block has left
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    // no copy may land after the block has left: wait for the chunks still in flight
+    for (int k = max(0, issued - kSlots); k < issued; ++k)
+        mbar_wait_warp(&ring->full[k % kSlots], (k / kSlots) & 1, 1 << 23, nullptr, 0);
 }
 
-// A packed pixel taken apart for the step's cost: gray, and |gx|, |gy| as halves.
+// packed_cost for the wavefront's steps: one byte-difference instruction for the three differences, every
+// table read (the entries of a term the configuration leaves out are zero, and adding zero changes no
+// sum), the gradient table extended to kGradAll entries so that a pixel outside the image costs 1e30.
 template <bool C64>
-struct Split {
-    decltype(RPack<C64>::c) c;
-    int gray;
-    uint32_t gxy;
-    __device__ __forceinline__ explicit Split(const RPack<C64>& p)
-        : c(p.c), gray((int)(p.g & 0xFFu)), gxy(__byte_perm(p.g, 0u, 0x4241)) {}
-};
-// packed_cost with every table read: the entries of a term the configuration leaves out are zero, and
-// adding zero changes no sum.
-template <bool C64>
-__device__ __forceinline__ float split_cost(const float* lut, const Split<C64>& l, const RPack<C64>& rp) {
-    const Split<C64> r(rp);
+__device__ __forceinline__ float step_cost(const float* lut, const RPack<C64>& l, const RPack<C64>& r) {
     int pop;
     if constexpr (C64) pop = __popcll(l.c ^ r.c);
     else pop = __popc(l.c ^ r.c);
-    const uint32_t dg = __vmaxs2(l.gxy, r.gxy) - __vmins2(l.gxy, r.gxy);  // |dgx| | |dgy| << 16
-    const float a = lut[kLutCensus + pop], b = lut[kLutAd + abs(l.gray - r.gray)];
-    const float g = lut[kLutGrad + __dp4a(dg, 0x00010001u, 0u)];
-    return __fadd_rn(__fadd_rn(a, b), g);
+    const uint32_t dd = __vabsdiffu4(l.g, r.g);
+    return __fadd_rn(__fadd_rn(lut[kLutCensus + pop], lut[kLutAd + (dd & 0xFFu)]),
+                     lut[kLutGrad + __dp4a(dd, kGradWeights, 0u)]);
 }
 
-// WIN: each lane's right-image window ([x - dmax + 1, x - d0] of its row, sliding one pixel per
-// step) lives in shared memory, a ring of wmask + 1 records per lane (a power of two holding the
-// window plus the kRing steps copied ahead; the lanes' rings interleaved); the loader copies the
-// entering pixel with the step's record, so the candidates' right pixels are shared-memory loads.
-// Without WIN they are global loads kept warm in L1 by the loader's prefetches.  Three warps per block: warp 0 computes, warp 1
-// links the band to its neighbours (band_link), warp 2 loads the step ring (band_loader), so that
-// no copy or address arithmetic sits in the compute warp's step.
+// WIN: the lanes' right-image windows ([x - dmax + 1, x - d0] of each row, sliding one pixel per step)
+// live in shared memory, a ring of wmask + 1 steps (a power of two holding the window plus the kRing
+// steps copied ahead): the pixels entering at step t lie at t & wmask, lane by lane, so a candidate's
+// right pixel is a conflict-free shared-memory load a known number of steps back.  Without WIN they are
+// global loads kept warm in L1 by the loader's prefetches.  Three warps per block: warp 0 computes,
+// warp 1 links the band to other clusters (band_link), warp 2 loads the rings (band_loader).
 //
 // Bound: the step's dependent chain -- neighbour shuffle, clamp, window load, table loads, two adds,
-// four selects, about 150 cycles -- times w + h steps a pass.  Everything else is kept off the step:
-// waits, hand-overs and publications come once per chunk of eight steps, the chunk's steps are one
-// straight line of code without divergent branches (a pixel that is not updated takes the same
-// selection, see RStep), and its records load ahead of the chain.
-template <bool C64, bool WIN>
-__global__ void __launch_bounds__(96) refine_band_kernel(CostCtx c, int fwd, const RStep* __restrict__ steps,
-                                                         const RPack<C64>* __restrict__ lp,
+// four selects -- times about w + 40 bands steps a pass.  Everything else is kept off the step: waits
+// and hand-overs come once per chunk of eight steps, the chunk's steps are one straight line of code
+// without divergent branches (a pixel that is not updated takes the same selection, see RStep), its
+// records come by bulk copies that use no issue slot or load path of the SM, and a band hands its last
+// row to the next one through the cluster's shared memory.
+template <bool C64, bool WIN, bool FWD>
+__global__ void __launch_bounds__(96) refine_band_kernel(CostCtx c, int nbands, int csize,
+                                                         const RStep<C64>* __restrict__ steps,
+                                                         const RPack<C64>* __restrict__ wr,
                                                          const RPack<C64>* __restrict__ rp, float* work,
                                                          int* progress, int* err, int spin_limit, int wmask) {
-    __shared__ float s_lut[kLutSize];
-    __shared__ __align__(16) BandRing<C64> s_ring;
-    __shared__ __align__(16) BandLink s_link;
-    for (int i = threadIdx.x; i < kLutSize; i += blockDim.x) s_lut[i] = c.lut[i];
+    constexpr int fwd = FWD ? 1 : 0;
+    constexpr int kSlots = BandRing<C64>::kSlots;
+    __shared__ float s_lut[kLutGrad + kGradAll];
+    __shared__ __align__(128) BandRing<C64> s_ring;
+    __shared__ BandLink s_link;
+    extern __shared__ __align__(128) unsigned char s_dyn[];
+    const int w = c.w;
+    const int ublk = up_blocks(w);
+    RPack<C64>* s_win = reinterpret_cast<RPack<C64>*>(s_dyn);
+    int* s_up = reinterpret_cast<int*>(s_dyn + (WIN ? (size_t)(wmask + 1) * 32 * sizeof(RPack<C64>) : 0));
+    uint64_t* s_upbar = reinterpret_cast<uint64_t*>(s_up + ublk * kChunk);
+    const int band = blockIdx.x;
+    const int rank = band % csize;
+    const bool live = band < nbands;
+    // the row above comes from the cluster's previous band, from another cluster, or (band 0) nowhere
+    const bool from_peer = live && rank > 0, from_link = live && band > 0 && rank == 0;
+    const bool to_peer = live && rank + 1 < csize && band + 1 < nbands;
+    const bool to_link = live && rank + 1 == csize && band + 1 < nbands;
+    for (int i = threadIdx.x; i < kLutGrad + kGradAll; i += blockDim.x) s_lut[i] = i < kLutGrad + kGradIn ? c.lut[i] : 1e30f;
+    for (int i = threadIdx.x; i < ublk; i += blockDim.x) mbar_init(&s_upbar[i], 1);
     if (threadIdx.x == 0) {
-        s_link.avail = 0;
-        s_link.used = 0;
         s_link.done = 0;
         s_link.abort = 0;
         s_ring.stop = 0;
         for (int i = 0; i < kSlots; ++i) {
-            mbar_init(&s_ring.full[i], 32);
+            mbar_init(&s_ring.full[i], 1);
             mbar_init(&s_ring.empty[i], 1);
         }
     }
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     __syncthreads();
-    const int band = blockIdx.x;
-    const int w = c.w;
+    if (from_peer)
+        for (int i = threadIdx.x; i < ublk; i += blockDim.x) mbar_expect(&s_upbar[i], kChunk * 4);
+    __syncthreads();
+    cluster_sync();  // every band's barriers are armed before a peer sends
     const int warp = threadIdx.x >> 5;
-    if (warp == 1) {
-        band_link(&s_link, band, w, c.h, fwd, work, progress, err, spin_limit);
-        return;
-    }
-    const BandRow<C64> r(c, band, fwd, steps, lp, rp, work);
-    extern __shared__ __align__(16) unsigned char s_dyn[];
-    // the lanes' window rings interleaved, record i of lane l at i * kBand + l: a step's loads of
-    // the 32 lanes fall in distinct banks whatever their offsets
-    RPack<C64>* s_win = reinterpret_cast<RPack<C64>*>(s_dyn) + r.lane;
-    if (warp == 2) {
-        band_loader<C64, WIN>(c, r, &s_ring, s_win, wmask, spin_limit);
-        return;
-    }
-    volatile BandLink* link = &s_link;
-    const int lane = r.lane;
-    const int wl = r.ok ? w : 0;  // columns of this lane's row
-    // Neighbour values travel as candidates: roundf(value) when value >= 0, else -1 (the
-    // reference takes a neighbour only when it is non-negative, rounded).
-    int prev = -1;  // candidate of this lane's previous column (its left neighbour)
-    int avail = band > 0 ? 0 : w;  // columns of the row above known to be in the link's ring
-    bool abort = false;
-    const int nchunks = (w + kBand - 1 + kChunk - 1) / kChunk;
-    for (int k = 0; k < nchunks; ++k) {
-        const int t0 = k * kChunk;
-        int up_first[kChunk];  // the row above at columns t0 .. (lane 0's up neighbours)
-#pragma unroll
-        for (int i = 0; i < kChunk; ++i) up_first[i] = -1;
-        if (band > 0 && t0 < w) {
-            const int need = min(t0 + kChunk, w);
-            if (avail < need) {
-                // wait until the link warp has the chunk's columns of the row above (lane 0 polls, so
-                // that the warp decides together)
-                int spins = 0, state = 0;  // 1: available, 2: gave up
-                for (;;) {
-                    if (lane == 0) {
-                        const int a = link->avail;
-                        state = a >= need ? 1 : ((link->abort || ++spins > spin_limit) ? 2 : 0);
-                        if (state == 1) avail = a;
-                    }
-                    state = __shfl_sync(0xffffffffu, state, 0);
-                    if (state) break;
-                    __nanosleep(32);
-                }
-                avail = __shfl_sync(0xffffffffu, avail, 0);
-                if (state == 2) {
+    const int lane = threadIdx.x & 31;
+    if (live && warp == 1) {
+        if (from_link || to_link)
+            band_link(&s_link, s_up, s_upbar, band, w, c.h, fwd, work, progress, err, spin_limit, from_link, to_link);
+    } else if (live && warp == 2) {
+        band_loader<C64, WIN>(c, band, fwd, &s_ring, s_win, wmask, steps, wr, rp, spin_limit);
+    } else if (live) {
+        volatile BandLink* link = &s_link;
+        const int v = band * kBand + lane;
+        const int yrow = fwd ? v : c.h - 1 - v;
+        const int xs = fwd ? 1 : -1, xb = fwd ? 0 : w - 1;
+        const size_t rowoff = (size_t)(v < c.h ? yrow : 0) * w;
+        float* wrow = work + rowoff;
+        const RPack<C64>* rrow = rp + rowoff;
+        const unsigned peer_up = to_peer ? peer_smem(smem_u32(s_up), rank + 1) : 0u;
+        const unsigned peer_bar = to_peer ? peer_smem(smem_u32(s_upbar), rank + 1) : 0u;
+        // steps back to a candidate's window pixel: back_0 + d forward, back_0 - d backward (the entering
+        // pixel has the lowest disparity forward, the highest backward)
+        const int back_0 = fwd ? -c.d0 : c.d0 + c.D - 1;
+        // Neighbour values travel as candidates: roundf(value) when value >= 0, else -1 (the
+        // reference takes a neighbour only when it is non-negative, rounded), or any negative value.
+        int prev = -1;  // candidate of this lane's previous column (its left neighbour)
+        bool abort = false;
+        const int nchunks = wave_chunks(w);
+        int upc = band > 0 ? 0 : ublk;  // barriers of the row above known to be complete
+        int sent = 0;                   // blocks of this band's last row sent to the peer
+        for (int k = 0; k < nchunks && !abort; ++k) {
+            const int t0 = k * kChunk;
+            // the row above up to column t0 + kChunk - 1 (lane 0's up neighbours)
+            const int need = min((t0 + kChunk - 1 + kUpShift) / kChunk + 1, ublk);
+            while (upc < need) {
+                if (!mbar_wait_warp(&s_upbar[upc], 0, spin_limit, &s_link.abort, 0)) {
                     abort = true;
-                    if (lane == 0) atomicExch(err, 1);
                     break;
                 }
+                ++upc;
+            }
+            // the chunk's slot has landed
+            const int slot = k % kSlots;
+            if (abort || !mbar_wait_warp(&s_ring.full[slot], (k / kSlots) & 1, spin_limit, nullptr, 0)) {
+                abort = true;
+                break;
+            }
+            int up_first[kChunk];
+#pragma unroll
+            for (int i = 0; i < kChunk; ++i)
+                up_first[i] = band > 0 ? s_up[min(t0 + i + kUpShift, ublk * kChunk - 1)] : -1;
+            const RStep<C64>* recs = &s_ring.rec[slot * kChunk][lane];
+            const int x0 = xb + xs * (t0 - lane);
+            int last[kChunk];
+#pragma unroll
+            for (int i = 0; i < kChunk; ++i) {
+                const int up_lane = __shfl_up_sync(0xffffffffu, prev, 1);
+                const int up = lane > 0 ? up_lane : up_first[i];
+                const RStep<C64> st = recs[i * 32];
+                // dynamic candidates: left (forward) / right (backward) and up / down, clamped into the
+                // range
+                const int dl = min(max(prev, st.lo), st.hi1), du = min(max(up, st.lo), st.hi1);
+                RPack<C64> pl, pu;
+                if constexpr (WIN) {
+                    // byte offsets into the ring, 32 pixels a step
+                    constexpr int B = 32 * (int)sizeof(RPack<C64>);
+                    const int base = (t0 + i - back_0) * B, m = wmask * B;
+                    const unsigned char* win = reinterpret_cast<const unsigned char*>(s_win + lane);
+                    pl = *reinterpret_cast<const RPack<C64>*>(win + ((FWD ? base - dl * B : base + dl * B) & m));
+                    pu = *reinterpret_cast<const RPack<C64>*>(win + ((FWD ? base - du * B : base + du * B) & m));
+                } else {
+                    const int xl = x0 + xs * i - dl, xu = x0 + xs * i - du;
+                    const bool in_l = (unsigned)xl < (unsigned)w, in_u = (unsigned)xu < (unsigned)w;
+                    pl = rrow[in_l ? xl : 0];
+                    pu = rrow[in_u ? xu : 0];
+                    pl.g = in_l ? pl.g : kOutside;
+                    pu.g = in_u ? pu.g : kOutside;
+                }
+                // a neighbour outside the image costs 1e6 like the reference's; no neighbour never wins
+                const float vl = step_cost<C64>(s_lut, st.left, pl), vu = step_cost<C64>(s_lut, st.left, pu);
+                const float il = vl < 1e29f ? vl : 1e6f, iu = vu < 1e29f ? vu : 1e6f;
+                const float cl = prev >= 0 ? il : 1e30f, cu = up >= 0 ? iu : 1e30f;
+                // the reference's order: cur, left, up, cur + draw; the first strict minimum wins (as two
+                // pairs, the second winning only if strictly below the first)
+                const int da = cl < st.c_cur ? dl : st.d_cur, db = st.c_draw < cu ? st.d_draw : du;
+                const float ca = fminf(cl, st.c_cur), cb = fminf(st.c_draw, cu);
+                prev = cb < ca ? db : da;
+                if (st.c_cur != __int_as_float(0xff800000)) wrow[x0 + xs * i] = (float)prev;
+                last[i] = prev;
+            }
+            // every lane has read the slot (and its window pixels): the loader may refill it
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&s_ring.empty[slot]);
+            // hand on the last row's columns of this chunk (lane 31, column t - 31)
+            if (to_peer) {
+                const int pos = t0 - (kBand - 1) + kUpShift;  // a multiple of kChunk
+                if (pos >= 0 && pos < ublk * kChunk) {
+                    if (lane == kBand - 1) {
+                        const unsigned dst = peer_up + pos * 4, bar = peer_bar + pos / kChunk * 8;
+                        st_async4(dst, last[0], last[1], last[2], last[3], bar);
+                        st_async4(dst + 16, last[4], last[5], last[6], last[7], bar);
+                    }
+                    sent = pos / kChunk + 1;
+                }
+            } else if (to_link) {
                 __threadfence_block();
-            }
-            const int4* up4 = reinterpret_cast<const int4*>(&s_link.up[t0 & (kUpRing - 1)]);
-#pragma unroll
-            for (int i = 0; i < kChunk; i += 4) {
-                const int4 q = up4[i / 4];
-                up_first[i] = q.x; up_first[i + 1] = q.y; up_first[i + 2] = q.z; up_first[i + 3] = q.w;
+                if (lane == kBand - 1) link->done = max(0, min(t0 + kChunk - (kBand - 1), w));
             }
         }
-        // the chunk's slot has landed
-        const int slot = k % kSlots;
-        if (!mbar_wait_warp(&s_ring.full[slot], (k / kSlots) & 1, spin_limit, nullptr, 0)) {
-            abort = true;
+        if (abort) {
             if (lane == 0) atomicExch(err, 1);
-            break;
+            *(volatile int*)&s_ring.stop = 1;
         }
-        const RStep* recs = &s_ring.rec[slot * kChunk][lane];
-        const RPack<C64>* lpks = &s_ring.lpk[slot * kChunk][lane];
-        const int u0 = t0 - lane, x0 = r.xb + r.xs * u0;
-#pragma unroll
-        for (int i = 0; i < kChunk; ++i) {
-            const int up_lane = __shfl_up_sync(0xffffffffu, prev, 1);
-            const int up = lane > 0 ? up_lane : up_first[i];
-            const RStep st = recs[i * 32];
-            const Split<C64> l(lpks[i * 32]);
-            const int x = x0 + r.xs * i;
-            const int lo = (int)(short)(st.range & 0xFFFF), hi1 = st.range >> 16;
-            // dynamic candidates: left (forward) / right (backward) and up / down, clamped into the
-            // range, so only x - d needs a test
-            const int dl = min(max(prev, lo), hi1), du = min(max(up, lo), hi1);
-            const int xl = x - dl, xu = x - du;
-            const bool in_l = (unsigned)xl < (unsigned)w, in_u = (unsigned)xu < (unsigned)w;
-            RPack<C64> pl, pu;
-            if constexpr (WIN) {
-                pl = s_win[(xl & wmask) * kBand];
-                pu = s_win[(xu & wmask) * kBand];
-            } else {
-                pl = r.right[in_l ? xl : 0];
-                pu = r.right[in_u ? xu : 0];
-            }
-            float cl = in_l ? split_cost<C64>(s_lut, l, pl) : 1e6f;
-            float cu = in_u ? split_cost<C64>(s_lut, l, pu) : 1e6f;
-            cl = prev >= 0 ? cl : 1e30f;
-            cu = up >= 0 ? cu : 1e30f;
-            // the reference's order: cur, left, up, cur + draw; the first strict minimum wins
-            float best_c = st.c_cur;
-            int best_d = (int)(short)(st.d_pack & 0xFFFF);
-            if (cl < best_c) { best_c = cl; best_d = dl; }
-            if (cu < best_c) { best_c = cu; best_d = du; }
-            if (st.c_draw < best_c) best_d = st.d_pack >> 16;
-            const bool on = (unsigned)(u0 + i) < (unsigned)wl;
-            if (on && st.c_cur != __int_as_float(0xff800000)) r.work[x] = (float)best_d;
-            prev = on ? max(best_d, -1) : -1;
-        }
-        // every lane has read the slot (and its window pixels): the loader may refill it
         __syncwarp();
-        if (lane == 0) mbar_arrive(&s_ring.empty[slot]);
-        // release to the link warp (CTA scope): how far the last row (lane 31, column t - 31) is
-        // final, and that the ring's columns of this chunk are read
         __threadfence_block();
-        if (lane == kBand - 1) link->done = max(0, min(t0 + kChunk - (kBand - 1), w));
-        if (lane == 0) link->used = min(t0 + kChunk, w);
+        // the whole band is final (or the pass was abandoned: let the next band finish).  Every block of
+        // the row is sent whatever happened, and every band takes all of its own before it leaves, so no
+        // store is under way to a block that has ended.
+        if (lane == kBand - 1) {
+            link->done = w;
+            if (to_peer)
+                for (int b = sent; b < ublk; ++b) {
+                    st_async4(peer_up + b * (kChunk * 4), -1, -1, -1, -1, peer_bar + b * 8);
+                    st_async4(peer_up + b * (kChunk * 4) + 16, -1, -1, -1, -1, peer_bar + b * 8);
+                }
+        }
+        __syncwarp();
+        if (from_peer)
+            for (; upc < ublk; ++upc) mbar_wait_warp(&s_upbar[upc], 0, 1 << 23, nullptr, 0);
     }
-    if (abort) *(volatile int*)&s_ring.stop = 1;
     __syncwarp();
-    __threadfence_block();
-    // the whole band is final (or the pass was abandoned: let the next band finish)
-    if (lane == kBand - 1) link->done = w;
+    cluster_sync();  // a peer's last stores have a block to land in
 }
 
 // ---- host: the engine stream, its draw values and rejected indices per radius
@@ -803,8 +845,18 @@ cudaError_t launch_refine_pack(const CostCtx& c, const Layout& L, unsigned char*
 
 size_t refine_pack_bytes(int n, bool c64) { return (size_t)n * 2 * (c64 ? sizeof(RPack<true>) : sizeof(RPack<false>)); }
 
-cudaError_t launch_refine_pass(const CostCtx& c, const Layout& L, unsigned char* arena, const RefineTables& tab,
-                               int it, float* work, const RefineTuning& tune, cudaStream_t s, unsigned* launches) {
+size_t refine_steps_bytes(int w, int h, int D, bool c64) {
+    const size_t nb = refine_band_count(h), nstep = (size_t)wave_chunks(w) * kChunk;
+    const size_t pk = c64 ? sizeof(RPack<true>) : sizeof(RPack<false>);
+    return nb * 32 * (nstep * (c64 ? sizeof(RStep<true>) : sizeof(RStep<false>)) + (c64 ? 0 : (nstep + wave_lead(D)) * pk));
+}
+
+namespace {
+
+template <bool C64, bool WIN>
+cudaError_t launch_pass_t(const CostCtx& c, const Layout& L, unsigned char* arena, const RefineTables& tab, int it,
+                          float* work, int spin_limit, int wmask, size_t smem, int csize, cudaStream_t s,
+                          unsigned* launches) {
     const int fwd = (it % 2) == 0;
     const int n = L.w * L.h;
     const int nbands = refine_band_count(L.h);
@@ -813,64 +865,98 @@ cudaError_t launch_refine_pass(const CostCtx& c, const Layout& L, unsigned char*
     unsigned* P = reinterpret_cast<unsigned*>(arena + L.rf_state);
     int* err = reinterpret_cast<int*>(arena + L.rf_state) + kRefineErrWord;
     int* progress = reinterpret_cast<int*>(arena + L.rf_state) + kRefineProgWord;
-    RStep* steps = reinterpret_cast<RStep*>(arena + L.rf_steps);
-    const int blocks = min((n + 255) / 256, 148 * 8);
-    if (c.census64) {
-        const RPack<true>* lpk = reinterpret_cast<const RPack<true>*>(arena + L.rf_pack);
-        refine_prep_kernel<true><<<blocks, 256, 0, s>>>(c, fwd, rel, prefix, tab.value[it], tab.rejected[it], tab.nrej[it],
-                                                        P + it, lpk, lpk + n, work, steps);
-    } else {
-        const RPack<false>* lpk = reinterpret_cast<const RPack<false>*>(arena + L.rf_pack);
-        refine_prep_kernel<false><<<blocks, 256, 0, s>>>(c, fwd, rel, prefix, tab.value[it], tab.rejected[it],
-                                                         tab.nrej[it], P + it, lpk, lpk + n, work, steps);
-    }
+    const RPack<C64>* lpk = reinterpret_cast<const RPack<C64>*>(arena + L.rf_pack);
+    const RPack<C64>* rpk = lpk + n;
+    const size_t ns = (size_t)nbands * wave_chunks(L.w) * kChunk * 32;
+    RStep<C64>* steps = reinterpret_cast<RStep<C64>*>(arena + L.rf_steps);
+    RPack<C64>* wr = reinterpret_cast<RPack<C64>*>(steps + ns);
+    const size_t items = ns / 32 + (WIN ? (size_t)nbands * wave_lead(c.D) : 0);
+    const int blocks = (int)std::min<size_t>((items + 7) / 8, 148 * 8);
+    refine_prep_kernel<C64, WIN><<<blocks, 256, 0, s>>>(c, fwd, rel, prefix, tab.value[it], tab.rejected[it],
+                                                        tab.nrej[it], P + it, lpk, rpk, work, steps, wr);
     ++*launches;
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    // about a second of waiting at most per wait (spins of ~128 ns sleep plus the poll), unless the
-    // engine's tuning sets a smaller poll budget
-    int spin_limit = tune.spin_limit > 0 ? tune.spin_limit : 1 << 23;
-    CostCtx cc = c;
-    const void* lpk = arena + L.rf_pack;
-    const void* rpk = c.census64 ? (const void*)(reinterpret_cast<const RPack<true>*>(lpk) + n)
-                                 : (const void*)(reinterpret_cast<const RPack<false>*>(lpk) + n);
-    const RStep* csteps = steps;
-    int fwd_arg = fwd;
-    // the right-image window in shared memory (32-bit census): a power-of-two ring per lane holding
-    // the D window pixels plus the kRing copied ahead, when every band still fits on the device at once
-    int wmask = 0;
-    size_t wbytes = 0;
-    const void* kern = c.census64 ? (const void*)refine_band_kernel<true, false> : (const void*)refine_band_kernel<false, false>;
-    if (!c.census64 && tune.window == 0) {
-        int rs = 1;
-        while (rs < c.D + kRing) rs <<= 1;
-        const size_t bytes = (size_t)kBand * (rs + 1) * sizeof(RPack<false>);
-        auto wk = refine_band_kernel<false, true>;
-        if (rs <= 512 && allow_dynamic_smem(wk, bytes) == cudaSuccess) {
-            int per_sm = 0, dev = 0, nsm = 0;
-            if (cudaGetDevice(&dev) == cudaSuccess &&
-                cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wk, 3 * kBand, bytes) == cudaSuccess &&
-                per_sm * nsm >= nbands) {
-                wmask = rs - 1;
-                wbytes = bytes;
-                kern = (const void*)wk;
-            }
-        }
-        cudaGetLastError();
-    }
-    void* args[] = {&cc, &fwd_arg, (void*)&csteps, (void*)&lpk, (void*)&rpk, &work, &progress, &err, &spin_limit,
-                    &wmask};
-    e = cudaLaunchCooperativeKernel(kern, dim3(nbands), dim3(3 * kBand), args, wbytes, s);
+    // every band at once (a band waits for the one above): a cooperative launch in clusters of csize
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((nbands + csize - 1) / csize * csize);
+    cfg.blockDim = dim3(3 * kBand);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = csize;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+    e = cudaLaunchKernelEx(&cfg, fwd ? refine_band_kernel<C64, WIN, true> : refine_band_kernel<C64, WIN, false>, c, nbands,
+                           csize, (const RStep<C64>*)steps, (const RPack<C64>*)wr, rpk, work, progress, err, spin_limit,
+                           wmask);
     if (e != cudaSuccess) return e;
     ++*launches;
     // start of the next pass, and cleared progress counters
-    const int* count = prefix + n;
-    refine_advance_kernel<<<1, 64, 0, s>>>(P, it, count, tab.rejected[it], tab.nrej[it], progress, nbands);
+    refine_advance_kernel<<<1, 64, 0, s>>>(P, it, prefix + n, tab.rejected[it], tab.nrej[it], progress, nbands);
     ++*launches;
     return cudaGetLastError();
 }
 
-size_t refine_steps_bytes(int n) { return (size_t)n * sizeof(RStep); }
+// The largest cluster (8, 4, 2, 1 bands) in which every band of the frame is resident at once with
+// `smem` bytes each, or 0.
+template <bool C64, bool WIN, bool FWD>
+int cluster_size(int nbands, size_t smem) {
+    auto kern = refine_band_kernel<C64, WIN, FWD>;
+    if (allow_dynamic_smem(kern, smem) != cudaSuccess) return 0;
+    for (int cs = 8; cs >= 1; cs >>= 1) {
+        if (cs > 1 && cs > nbands) continue;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((nbands + cs - 1) / cs * cs);
+        cfg.blockDim = dim3(3 * kBand);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = cs;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int nc = 0;
+        if (cudaOccupancyMaxActiveClusters(&nc, kern, &cfg) == cudaSuccess && nc * cs >= (int)cfg.gridDim.x) return cs;
+        cudaGetLastError();
+    }
+    return 0;
+}
+template <bool C64, bool WIN>
+int cluster_size_of(bool fwd, int nbands, size_t smem) {
+    return fwd ? cluster_size<C64, WIN, true>(nbands, smem) : cluster_size<C64, WIN, false>(nbands, smem);
+}
+
+}  // namespace
+
+cudaError_t launch_refine_pass(const CostCtx& c, const Layout& L, unsigned char* arena, const RefineTables& tab,
+                               int it, float* work, const RefineTuning& tune, cudaStream_t s, unsigned* launches) {
+    const int nbands = refine_band_count(L.h);
+    const bool fwd = (it % 2) == 0;
+    // about a second of waiting at most per wait, unless the engine's tuning sets a smaller poll budget
+    const int spin_limit = tune.spin_limit > 0 ? tune.spin_limit : 1 << 23;
+    const size_t up = (size_t)up_blocks(L.w) * (kChunk * 4 + 8);
+    // the right-image window in shared memory (32-bit census): a power-of-two ring of steps holding the
+    // window (rounded up to whole chunks) plus the kRing steps copied ahead, when every band still fits
+    // on the device at once
+    if (!c.census64 && tune.window == 0) {
+        int rs = 1;
+        while (rs < wave_lead(c.D) + kRing + kChunk) rs <<= 1;
+        const size_t smem = (size_t)rs * 32 * sizeof(RPack<false>) + up;
+        if (rs <= 512) {
+            const int cs = cluster_size_of<false, true>(fwd, nbands, smem);
+            if (cs) return launch_pass_t<false, true>(c, L, arena, tab, it, work, spin_limit, rs - 1, smem, cs, s, launches);
+        }
+        cudaGetLastError();
+    }
+    const int cs = c.census64 ? cluster_size_of<true, false>(fwd, nbands, up) : cluster_size_of<false, false>(fwd, nbands, up);
+    if (!cs) return cudaErrorCooperativeLaunchTooLarge;
+    return c.census64 ? launch_pass_t<true, false>(c, L, arena, tab, it, work, spin_limit, 0, up, cs, s, launches)
+                      : launch_pass_t<false, false>(c, L, arena, tab, it, work, spin_limit, 0, up, cs, s, launches);
+}
 
 }  // namespace apgcu
