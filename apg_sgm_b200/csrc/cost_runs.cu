@@ -339,13 +339,23 @@ __device__ __forceinline__ void run_steps(const CostCtx& c, const RunGeom& g, in
     if (CROSS && PRIOR) store_counts<WPL>(s_totc + run * W2 + WPL * lane, cnt);
 }
 
+// floor(s / n) of a window sum and its count, by the table's reciprocal m of n: 2^32 / n (div_by_magic),
+// or, for the byte output (costs of at most 254), 2^24 / n, the quotient in the product's top byte (the
+// bound is derived in cross8.cu).
+template <bool U8>
+__device__ __forceinline__ uint32_t window_div(uint32_t s, uint32_t n, uint32_t m) {
+    if constexpr (U8) return (s * m) >> 24;
+    else return div_by_magic(s, n, m);
+}
+
 // Aggregated word kk at pixel x from its packed window sum s (cost.cu's tile kernel, same rules).
+template <bool U8>
 __device__ __forceinline__ uint32_t agg_word(const CostCtx& c, uint32_t s, int kk, int x, int l, int r,
                                              const uint32_t* s_magic) {
     const int dw = c.d0 + 2 * kk;
     if (2 * kk + 1 < c.D && x - l >= dw + 1 && x + r <= c.w - 1 + dw) {
         const uint32_t len = (uint32_t)(l + r + 1), mg = s_magic[len];
-        return div_by_magic(s & 0xFFFFu, len, mg) | (div_by_magic(s >> 16, len, mg) << 16);
+        return window_div<U8>(s & 0xFFFFu, len, mg) | (window_div<U8>(s >> 16, len, mg) << 16);
     }
     uint32_t word = 0;
 #pragma unroll
@@ -355,7 +365,7 @@ __device__ __forceinline__ uint32_t agg_word(const CostCtx& c, uint32_t s, int k
         const uint32_t sh = (s >> (16 * hs)) & 0xFFFFu;
         const int nh = min(x + r, c.w - 1 + d) - max(x - l, d) + 1;  // valid x' in the window
         const bool ok = di < c.D && d <= x && nh > 0;
-        const uint32_t q = ok ? div_by_magic(sh, (uint32_t)nh, s_magic[nh]) : kInvalidCost;
+        const uint32_t q = ok ? window_div<U8>(sh, (uint32_t)nh, s_magic[nh]) : kInvalidCost;
         word |= q << (16 * hs);
     }
     return word;
@@ -364,6 +374,7 @@ __device__ __forceinline__ uint32_t agg_word(const CostCtx& c, uint32_t s, int k
 // Aggregated word kk from its window sum s and its two 8-bit valid counts n, with per-pixel ranges
 // (cost.cu's tile kernel, same rule): a half is valid when its disparity is inside the centre
 // pixel's range and its window holds a valid voxel.
+template <bool U8>
 __device__ __forceinline__ uint32_t prior_word(const CostCtx& c, uint32_t s, uint32_t n, int kk, int lo, int hi,
                                                const uint32_t* s_magic) {
     uint32_t word = 0;
@@ -373,7 +384,7 @@ __device__ __forceinline__ uint32_t prior_word(const CostCtx& c, uint32_t s, uin
         const int d = c.d0 + di;
         const uint32_t sh = (s >> (16 * hs)) & 0xFFFFu, nh = (n >> (8 * hs)) & 0xFFu;
         const bool ok = di < c.D && d >= lo && d < hi && nh > 0;
-        const uint32_t q = ok ? div_by_magic(sh, nh, s_magic[nh]) : kInvalidCost;
+        const uint32_t q = ok ? window_div<U8>(sh, nh, s_magic[nh]) : kInvalidCost;
         word |= q << (16 * hs);
     }
     return word;
@@ -417,7 +428,7 @@ __global__ void __launch_bounds__(CROSS ? 512 : 256, CROSS ? (WPL > 2 ? 1 : 2) :
         for (int i = tid; i < 65; i += nt) s_q[i] = c.qlut[i];
     }
     if (CROSS)
-        for (int i = tid; i < 2 * g.ha + 2; i += nt) s_magic[i] = magic[i];
+        for (int i = tid; i < 2 * g.ha + 2; i += nt) s_magic[i] = U8 ? (i ? (1u << 24) / (uint32_t)i + 1u : 0u) : magic[i];
 
     const int xs = min(run * g.rl, g.nx), xe = min(xs + g.rl, g.nx);
 
@@ -529,19 +540,36 @@ __global__ void __launch_bounds__(CROSS ? 512 : 256, CROSS ? (WPL > 2 ? 1 : 2) :
                     const uint32_t rg = s_rng[sxi];
                     const int lo = (int)(int16_t)(rg & 0xFFFFu), hi = (int)(int16_t)(rg >> 16);
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) wd[q] = prior_word(c, sum[q], cw[q] & 0xFFFFu, k4 + q, lo, hi, s_magic);
-                } else if (c.D == c.Dp && len > 1 && x - l >= c.d0 + c.Dp - 1 && x + r <= c.w - 1 + c.d0) {
-                    // every word of the pixel has its whole window valid (no padded words, x - d inside
-                    // the image over the window for every d): one count, no per-word tests
+                    for (int q = 0; q < 4; ++q) wd[q] = prior_word<U8>(c, sum[q], cw[q] & 0xFFFFu, k4 + q, lo, hi, s_magic);
+                } else if (2 * k4 + 8 <= c.D && len > 1 && x - l >= c.d0 + 2 * k4 + 7 && x + r <= c.w - 1 + c.d0 + 2 * k4) {
+                    // these eight disparities have their whole window valid (inside the range, x - d inside
+                    // the image over the window): one count, no per-word tests
                     const uint32_t mg = s_magic[len];
+                    if constexpr (U8) {
+                        // the quotients are the products' top bytes
+                        uint32_t o[2];
+#pragma unroll
+                        for (int q = 0; q < 4; q += 2) {
+                            const uint32_t e = __byte_perm((sum[q] & 0xFFFFu) * mg, (sum[q] >> 16) * mg, 0x0073);
+                            const uint32_t f = __byte_perm((sum[q + 1] & 0xFFFFu) * mg, (sum[q + 1] >> 16) * mg, 0x0073);
+                            o[q / 2] = __byte_perm(e, f, 0x5410);
+                        }
+                        *reinterpret_cast<uint2*>(reinterpret_cast<uint8_t*>(out_vol) + ((size_t)row + x) * (2 * W2) + 2 * k4) =
+                            make_uint2(o[0], o[1]);
+                        continue;
+                    }
 #pragma unroll
                     for (int q = 0; q < 4; ++q)
                         wd[q] = __byte_perm(__umulhi(sum[q] & 0xFFFFu, mg), __umulhi(sum[q] >> 16, mg), 0x5410);
                 } else {
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) wd[q] = agg_word(c, sum[q], k4 + q, x, l, r, s_magic);
+                    for (int q = 0; q < 4; ++q) wd[q] = agg_word<U8>(c, sum[q], k4 + q, x, l, r, s_magic);
                 }
-                *reinterpret_cast<uint4*>(out_vol + ((size_t)row + x) * W2 + k4) = make_uint4(wd[0], wd[1], wd[2], wd[3]);
+                if constexpr (U8)
+                    *reinterpret_cast<uint2*>(reinterpret_cast<uint8_t*>(out_vol) + ((size_t)row + x) * (2 * W2) + 2 * k4) =
+                        make_uint2(__byte_perm(wd[0], wd[1], 0x6420), __byte_perm(wd[2], wd[3], 0x6420));
+                else
+                    *reinterpret_cast<uint4*>(out_vol + ((size_t)row + x) * W2 + k4) = make_uint4(wd[0], wd[1], wd[2], wd[3]);
             }
         }
     }
@@ -605,8 +633,8 @@ cudaError_t launch_runs_w(const CostCtx& c, int txc, int lmax, int tau, uint32_t
 template <bool CROSS, bool STORE, bool FULL, bool PRIOR>
 cudaError_t launch_runs_p(const CostCtx& c, int txc, int lmax, int tau, uint32_t* vol, uint32_t* rkey,
                           const uint32_t* magic, cudaStream_t s) {
-    if constexpr (STORE && !CROSS && !FULL) {
-        // the byte volume (Fast census-only costs below 255)
+    if constexpr (STORE && (CROSS || !FULL)) {
+        // the byte volume (costs below 255): census-only, or aggregated
         if (c.vol8) {
             switch (c.Dp) {
                 case 64: return launch_runs_w<CROSS, STORE, FULL, 1, PRIOR, true>(c, txc, lmax, tau, vol, rkey, magic, s);

@@ -775,7 +775,14 @@ int Engine::run_pre(const uint8_t* dl, int lstride, const uint8_t* dr, int rstri
     const uint32_t* magic = ptr<uint32_t>(L.magic);
     if (L.raw_cost) RUN(launch_cost(cc, 0, lmax, cfg_.color_threshold, ptr<uint32_t>(L.volRaw), ptr<uint32_t>(L.rkey), magic, s), "cost(raw)");
     const uint32_t* sgm_src = nullptr;
-    if (L.cross) {
+    // T, the horizontally aggregated volume, at one byte per voxel too where the pixel-run cost kernel
+    // writes it and the byte form of the vertical pass takes its arms
+    const bool t8 = L.cross && L.bytes && cross_v8_supported(Dp, lmax) && cost_runs_supported(cc, 1, lmax);
+    if (t8) {
+        CostCtx cv = cc;
+        cv.vol8 = 1;
+        RUN(launch_cost(cv, 1, lmax, cfg_.color_threshold, ptr<uint32_t>(L.volA), ptr<uint32_t>(L.rkey), magic, s), "cost+crossH");
+    } else if (L.cross) {
         RUN(launch_cost(cc, 1, lmax, cfg_.color_threshold, ptr<uint32_t>(L.volA), ptr<uint32_t>(L.rkey), magic, s), "cost+crossH");
     } else if (L.fused_fast) {
         if (!L.raw_cost) RUN(launch_cost(cc, 2, lmax, 0, nullptr, ptr<uint32_t>(L.rkey), magic, s), "right argmin");
@@ -802,7 +809,11 @@ int Engine::run_pre(const uint8_t* dl, int lstride, const uint8_t* dr, int rstri
     cudaEventRecord(ev_[4], s);
     if (L.cross) {
         const int tau = cfg_.color_threshold;
-        RUN(launch_cross_v(w, h, d0, D, Dp, lmax, tau, ptr<uint8_t>(L.lgray), ptr<int16_t>(L.rmin), ptr<int16_t>(L.rmax),
+        if (t8)
+            RUN(launch_cross_v8(w, h, d0, D, Dp, lmax, tau, ptr<uint8_t>(L.lgray), ptr<int16_t>(L.rmin), ptr<int16_t>(L.rmax),
+                                ptr<uint8_t>(L.volA), ptr<uint8_t>(L.volB), !ranged(), s), "crossV");
+        else
+            RUN(launch_cross_v(w, h, d0, D, Dp, lmax, tau, ptr<uint8_t>(L.lgray), ptr<int16_t>(L.rmin), ptr<int16_t>(L.rmax),
                            ptr<uint32_t>(L.volA), ptr<uint32_t>(L.volB), magic, !ranged(), L.bytes, s), "crossV");
         const int iters = std::max(1, cfg_.agg_iterations);
         for (int it = 1; it < iters; ++it) {

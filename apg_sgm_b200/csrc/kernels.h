@@ -51,6 +51,11 @@ cudaError_t launch_hier_range(const apg_pipeline_config_t& c, int w, int h, cons
 cudaError_t launch_cross_v(int w, int h, int d0, int D, int Dp, int lmax, int tau, const uint8_t* gray,
                            const int16_t* rmin, const int16_t* rmax, const uint32_t* tin, uint32_t* cout,
                            const uint32_t* magic, bool default_ranges, bool out8, cudaStream_t s);
+// cross8.cu: the same with T and the result at one byte per voxel (every quantised cost below 255).
+bool cross_v8_supported(int Dp, int lmax);
+cudaError_t launch_cross_v8(int w, int h, int d0, int D, int Dp, int lmax, int tau, const uint8_t* gray,
+                            const int16_t* rmin, const int16_t* rmax, const uint8_t* tin, uint8_t* cout,
+                            bool default_ranges, cudaStream_t s);
 cudaError_t launch_cross_h(int w, int h, int d0, int D, int Dp, int lmax, int tau, const uint8_t* gray,
                            const int16_t* rmin, const int16_t* rmax, const uint32_t* vin, uint32_t* vout,
                            const uint32_t* magic, cudaStream_t s);
