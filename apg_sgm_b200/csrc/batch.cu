@@ -4,14 +4,16 @@
 // one engine (device workspace + stream) per pair slot.  A call runs:
 //   * every pair's phases before the SGM (aux, range, cost + cross-H + right argmin, cross-V) on
 //     its own stream, so the pairs' kernels overlap on the device;
-//   * ONE persistent SGM launch per phase for the pairs of ALL buckets, whatever their sizes and
+//   * the sweeps of every pair on that stream too where they run over byte volumes (every preset: a
+//     pair's whole frame is then one chain of launches, and pairs overlap in all stages); else
+//     ONE persistent SGM launch per phase for the pairs of ALL buckets, whatever their sizes and
 //     disparity ranges (sgm_batch_mixed_kernel: warps pull (pair, direction, scanline) units,
 //     longest chains first, from one work queue, each unit running with its own pair's words per
 //     lane), so the latency-bound sweeps of every pair fill the GPU together;
 //   * every pair's phases after the SGM (confidence, LR, fill, median, frame counters) on its
 //     stream again.
 // The whole sequence is captured once into a CUDA graph per batch composition (the buckets and
-// their pair counts) and replayed; inputs are copied into the slots' fixed input buffers before
+// their pair counts; per bucket and pair count with byte sweeps) and replayed; inputs are copied into the slots' fixed input buffers before
 // the replay and the outputs copied out after it.  The option "unified_sgm" 0 (or 16 lanes per
 // chain from the tuner) runs each bucket on its own stream instead, with one SGM launch per phase
 // per bucket, captured per (bucket, pair count).
@@ -134,6 +136,7 @@ private:
     Bucket& bucket_for(const BucketKey& k);
     int ensure_slots(Bucket& b, int m);
     int ensure_plan(Bucket& b, int m);
+    bool byte_sweeps(const Bucket& b) const;
     int enqueue(Bucket& b, int m, bool batched_sgm);
     int run_bucket(Bucket& b, int m, bool batched_sgm);
     int autotune(Bucket& b, const apgcu_pair_t& sample, bool device_buffers);
@@ -199,7 +202,6 @@ int Batch::ensure_slots(Bucket& b, int m) {
         }
         e->set_sgm_lanes(b.tune.sgm_lanes);
         e->set_cost_tile(b.tune.cost_tile);
-        e->set_cost8(1);  // the batched SGM kernels read two-byte volumes
         b.slots.push_back(std::move(e));
         cudaEvent_t ev;
         if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) {
@@ -218,6 +220,15 @@ void drop_plans(Bucket& b) {
     b.graphs.clear();
     for (auto& p : b.plans) sgm_batch_plan_destroy(&p.second);
     b.plans.clear();
+}
+
+// Whether the bucket's pairs run the byte sweeps: those run pair by pair on the slots' streams (every
+// pair's whole frame in one captured graph, so pairs overlap in all stages), the persistent launch over
+// many pairs serves the 16-bit sweeps.  Twelve uneven Balanced pairs (four each of 640x480 D64, 1242x375
+// D192, 1280x720 D128): 5.15 ms a call, against 7.23 with 16-bit sweeps in one launch per phase.
+bool Batch::byte_sweeps(const Bucket& b) const {
+    return forced_lanes_ != 16 &&
+           Engine::make_layout(b.cfg, b.key.w, b.key.h, b.key.ch, 0).bytes;
 }
 
 int Batch::ensure_plan(Bucket& b, int m) {
@@ -448,11 +459,13 @@ int Batch::autotune(Bucket& b, const apgcu_pair_t& sample, bool device_buffers) 
     }
     const int Dp = round_up(b.key.dmax - b.cfg.min_disparity, 64);
     std::vector<Tuning> cand;
+    const bool bytes = byte_sweeps(b);
     const int alt_tile = Dp <= 128 ? 256 : 128;
     for (int tile : {0, alt_tile})
         for (int lanes : {32, 16})
             for (int mb : {0, 2}) {
                 if (lanes == 16 && Dp > 256) continue;
+                if (bytes && (lanes != 32 || mb != 0)) continue;  // the byte sweeps have neither choice
                 // one launch serves every bucket: 32 lanes per chain, the occupancy-limited grid
                 if (use_unified_ && (lanes != 32 || mb != 0)) continue;
                 Tuning t;
@@ -477,13 +490,13 @@ int Batch::autotune(Bucket& b, const apgcu_pair_t& sample, bool device_buffers) 
         e.set_sgm_lanes(t.sgm_lanes);
         e.set_cost_tile(t.cost_tile);
         drop_plans(b);
-        rc = ensure_plan(b, 1);
+        rc = bytes ? kOk : ensure_plan(b, 1);
         if (rc) break;
-        rc = enqueue(b, 1, true);  // warm-up
+        rc = enqueue(b, 1, !bytes);  // warm-up
         if (rc) break;
         cudaStreamSynchronize(b.stream);
         cudaEventRecord(t0, b.stream);
-        for (int rep = 0; rep < 2 && rc == kOk; ++rep) rc = enqueue(b, 1, true);
+        for (int rep = 0; rep < 2 && rc == kOk; ++rep) rc = enqueue(b, 1, !bytes);
         cudaEventRecord(t1, b.stream);
         cudaEventSynchronize(t1);
         float total = 0.f;
@@ -594,7 +607,7 @@ int Batch::process(int n, const apgcu_pair_t* pairs, bool device_buffers) {
         SgmLaunch probe;
         uint32_t* s7[7];
         b.slots[0]->sgm_launch(&probe, s7);
-        const bool batched = use_batched_sgm_ && sgm_batch_supported(Dp) && probe.cvol != nullptr;
+        const bool batched = use_batched_sgm_ && sgm_batch_supported(Dp) && probe.cvol != nullptr && !probe.cost8;
         if (!batched || b.tune.sgm_lanes != 32) unified = false;
         batched_of.push_back(batched);
         comp.emplace_back(g.first, m);

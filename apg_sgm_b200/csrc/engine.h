@@ -255,7 +255,7 @@ private:
     bool ranges_written_ = false;  // the last frame wrote the range planes (else: default ranges)  // the last download() wrote the caller's page-locked (or device) outputs
     std::vector<float> lut_host_;
     std::vector<uint16_t> qlut_host_;
-    cudaEvent_t ev_[12] = {};
+    cudaEvent_t ev_[10] = {};
     bool have_times_ = false;
     // per-launch profile (APGCU_DEBUG_PROFILE): event after every launch, on the engine stream
     static constexpr int kMaxProf = 64;
@@ -280,8 +280,6 @@ private:
     // host path: confidence / reliability (and reason, without refine) are final after the
     // confidence kernel; their device-to-host copies run on copy_stream_ while the rest finishes
     cudaStream_t copy_stream_ = nullptr;
-    cudaStream_t side_stream_ = nullptr;  // the right-image WTA finalize, beside aggregation and SGM
-    bool rwta_forked_ = false;            // the last frame finalized it there (join before confidence)
     cudaEvent_t ev_maps_ = nullptr, ev_copied_ = nullptr;
     // banded host path: the post-processing stream and the per-band events (sweep done, rows done)
     cudaStream_t post_stream_ = nullptr;

@@ -1592,7 +1592,7 @@ cudaError_t sgm_batch_plan_create(const SgmLaunch* pl, uint32_t* const* sbufs, i
     int Dp = 0;
     bool mixed = false;
     for (int i = 0; i < npairs; ++i) {
-        if (!sgm_batch_supported(pl[i].Dp) || !pl[i].cvol) return cudaErrorInvalidValue;
+        if (!sgm_batch_supported(pl[i].Dp) || !pl[i].cvol || pl[i].cost8) return cudaErrorInvalidValue;
         if (i > 0 && pl[i].Dp != pl[0].Dp) mixed = true;
         Dp = std::max(Dp, pl[i].Dp);
     }

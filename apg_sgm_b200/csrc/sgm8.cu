@@ -890,26 +890,6 @@ Args8 make_args8(const SgmLaunch& l) {
     return a;
 }
 
-// Shared memory of a one-warp block, rounded up so that an SM takes no more than its even share of the
-// launch's blocks (at least `least`).  Every chain of a launch is resident at once, so where a block
-// lands decides how many chains its SM steps: without the cap, blocks placed while another stream's
-// kernel (the right-image finalize) still held most SMs crowded onto the others (Fast 1280x720 D128
-// 0.622 ms per frame with the cap, 0.787 without).
-size_t even_share(int blocks, size_t need, int least) {
-    int dev = 0, nsm = 0, per_sm = 0, reserved = 0, optin = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
-        cudaGetLastError();
-        return need;
-    }
-    const int share = std::max(least, (blocks + nsm - 1) / nsm);
-    const long long cap = std::min<long long>(per_sm / share - reserved, optin) / 128 * 128;
-    return std::max<long long>((long long)need, cap);
-}
-
 int max_p2(const SgmPen& p) { return p.P2_base > p.P1 + 1 ? p.P2_base : p.P1 + 1; }
 
 template <typename F>
@@ -944,7 +924,7 @@ cudaError_t launch_last_t(const Args8& a, const In8& in, int dx, int dy, int nsc
     using S = Split8<DP, NIN, SG, NGP, NGC>;
     if (blocks <= blocks_at_once(S::bytes)) {
         auto kern = sgm8_last_split_kernel<DP, NIN, SG, NGP, NGC, PS, BAND>;
-        const size_t smem = even_share(blocks, S::bytes, 4);
+        const size_t smem = S::bytes;
         const cudaError_t e = allow_dynamic_smem(kern, smem);
         if (e != cudaSuccess) return e;
         kern<<<blocks, 64, smem, st>>>(a, in, dx, dy, nscan);
@@ -952,7 +932,7 @@ cudaError_t launch_last_t(const Args8& a, const In8& in, int dx, int dy, int nsc
     }
     constexpr int KG = DP == 256 ? (NIN == 3 ? 2 : 1) : (NIN == 3 ? 4 : 2), NG = 3;
     auto kern = sgm8_last_kernel<DP, NIN, KG, NG, PS, BAND>;
-    const size_t smem = even_share(blocks, last_bytes<DP, NIN, KG, NG>(), 4);
+    const size_t smem = last_bytes<DP, NIN, KG, NG>();
     const cudaError_t e = allow_dynamic_smem(kern, smem);
     if (e != cudaSuccess) return e;
     kern<<<blocks, 32, smem, st>>>(a, in, dx, dy, nscan);
@@ -1000,10 +980,7 @@ cudaError_t launch_sgm8_first(const SgmLaunch& l, int ndir, const int (*dirs)[2]
     }
     return by_dp(l.Dp, [&](auto dp) -> cudaError_t {
         constexpr int DP = decltype(dp)::value;
-        const size_t smem = even_share(tab.warp_begin[ndir], first_bytes<DP>(), 8);
-        const cudaError_t e = allow_dynamic_smem(sgm8_first_kernel<DP>, smem);
-        if (e != cudaSuccess) return e;
-        sgm8_first_kernel<DP><<<tab.warp_begin[ndir], 32, smem, st>>>(a, tab);
+        sgm8_first_kernel<DP><<<tab.warp_begin[ndir], 32, first_bytes<DP>(), st>>>(a, tab);
         return cudaGetLastError();
     });
 }
