@@ -60,6 +60,7 @@ __global__ void __launch_bounds__(TX * BY) aux_kernel(AuxImage im0, AuxImage im1
         const int gxv = (int)g[cy][cx + 1] - (int)g[cy][cx - 1];
         const int gyv = (int)g[cy + 1][cx] - (int)g[cy - 1][cx];
         const size_t o = (size_t)y * w + x;
+        if (im.keys) im.keys[o] = kInvalidWord;
         gray[o] = g[cy][cx];
         gx[o] = (uint8_t)min(abs(gxv), 255);
         gy[o] = (uint8_t)min(abs(gyv), 255);

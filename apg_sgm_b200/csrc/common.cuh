@@ -144,6 +144,37 @@ __device__ __forceinline__ float subpixel_delta_tel(float cm, float c0, float cp
     return delta;
 }
 
+// The right-image disparity of pixel (xr, y) from its argmin key (cost << 16 | disparity index): the
+// disparity, with the parabola through the raw costs of its diagonal neighbours C(xr+d-1, d-1), C(xr+d, d),
+// C(xr+d+1, d+1) (src/pipeline.cpp:53-82), recomputed from the aux planes.  lut: the kLutSize tables.
+template <bool C64>
+__device__ __forceinline__ float right_disparity(const CostCtx& c, const float* lut, uint32_t key, int y, int xr,
+                                                 int subpixel) {
+    // best_d = -1 is the reference's "none" marker, tested as best_d >= 0: a negative winning
+    // disparity is reported as -1 too (src/pipeline.cpp:40-53).
+    if (key == kInvalidWord || c.d0 + (int)(key & 0xFFFFu) < 0) return -1.f;
+    const int di = (int)(key & 0xFFFFu);
+    const int bd = c.d0 + di;
+    const float dv = (float)bd;
+    const int xm = xr + bd - 1, xp = xr + bd + 1;
+    if (!(subpixel && xm >= 0 && xp < c.w && di > 0 && di + 1 < c.D)) return dv;
+    const int row = y * c.w;
+    // C(xl, d) is valid iff d is inside range(xl) and xl - d is inside the image; here xl - d == xr for
+    // all three, so only the range test remains, and with the default ranges it always holds (d >= d0,
+    // d < dmax, d <= xl).  The right pixel's descriptors are the same for the three costs
+    // (src/cost_computer.cpp:247-264).
+    if (c.prior_ranges)
+        for (int k = -1; k <= 1; ++k)
+            if (bd + k < c.rmin[row + xr + bd + k] || bd + k >= c.rmax[row + xr + bd + k]) return dv;
+    float q[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float v = __fadd_rn(__fmul_rn(raw_cost<C64>(c, lut, xm + k, y, xr), c.scale), 0.5f);
+        q[k] = (float)min(max(__float2int_rz(v), 0), c.cost_max);
+    }
+    return __fadd_rn(dv, subpixel_delta(q[0], q[1], q[2], c.sp_method, c.sp_param, 1.0f));
+}
+
 // Exact q = n / d for n < 2^16 and 1 <= d < 2^16 with one high multiply:
 // m = floor(2^32 / d) + 1 gives n*m/2^32 = n/d + e with 0 < e < 2^-16 <= 1/d, so the floor is
 // exact (tests/test_host_logic.py checks every n, d used by the cross aggregation).

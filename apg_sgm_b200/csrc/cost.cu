@@ -402,45 +402,8 @@ __global__ void right_wta_finalize_kernel(CostCtx c, const uint32_t* __restrict_
     __syncthreads();
     const int n = c.w * c.h;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
-        const uint32_t key = rkey[p];
-        float dv = -1.f;
-        // best_d = -1 is the reference's "none" marker, tested as best_d >= 0: a negative
-        // winning disparity is reported as -1 too (src/pipeline.cpp:40-53).
-        if (key != kInvalidWord && c.d0 + (int)(key & 0xFFFFu) >= 0) {
-            const int di = (int)(key & 0xFFFFu);
-            const int bd = c.d0 + di;
-            dv = (float)bd;
-            const int y = p / c.w, xr = p - y * c.w;
-            const int xm = xr + bd - 1, xp = xr + bd + 1;
-            if (subpixel && xm >= 0 && xp < c.w && di > 0 && di + 1 < c.D) {
-                const int row = y * c.w;
-                // C(xl, d) is valid iff d is inside range(xl) and xl - d is inside the image; here
-                // xl - d == xr for all three, so only the range test remains, and with the default
-                // ranges it always holds (d >= d0, d < dmax, d <= xl).  The right pixel's
-                // descriptors are the same for the three costs (src/cost_computer.cpp:247-264).
-                const int rg = c.rgray[row + xr], rgx = c.rgx[row + xr], rgy = c.rgy[row + xr];
-                uint32_t rc32 = 0;
-                unsigned long long rc64 = 0;
-                if (C64) rc64 = c.cr64[row + xr];
-                else rc32 = c.cr[row + xr];
-                auto cost_at = [&](int xl, int d, uint32_t& out) -> bool {
-                    if (c.prior_ranges && (d < c.rmin[row + xl] || d >= c.rmax[row + xl])) return false;
-                    const int pop = C64 ? __popcll(c.cl64[row + xl] ^ rc64) : __popc(c.cl[row + xl] ^ rc32);
-                    float v = s_lut[kLutCensus + pop];
-                    if (c.use_ad) v = __fadd_rn(v, s_lut[kLutAd + abs((int)c.lgray[row + xl] - rg)]);
-                    if (c.use_grad)
-                        v = __fadd_rn(v, s_lut[kLutGrad + abs((int)c.lgx[row + xl] - rgx) + abs((int)c.lgy[row + xl] - rgy)]);
-                    int q = __float2int_rz(__fadd_rn(__fmul_rn(v, c.scale), 0.5f));
-                    q = q < 0 ? 0 : (q > c.cost_max ? c.cost_max : q);
-                    out = (uint32_t)q;
-                    return true;
-                };
-                uint32_t cm, c0v, cp;
-                if (cost_at(xm, bd - 1, cm) && cost_at(xm + 1, bd, c0v) && cost_at(xp, bd + 1, cp))
-                    dv = __fadd_rn(dv, subpixel_delta((float)cm, (float)c0v, (float)cp, c.sp_method, c.sp_param, 1.0f));
-            }
-        }
-        disp_right[p] = dv;
+        const int y = p / c.w;
+        disp_right[p] = right_disparity<C64>(c, s_lut, rkey[p], y, p - y * c.w, subpixel);
     }
 }
 

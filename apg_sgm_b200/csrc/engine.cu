@@ -724,7 +724,8 @@ int Engine::run_pre(const uint8_t* dl, int lstride, const uint8_t* dr, int rstri
     }
     {
         const AuxImage li{dl, lstride, ptr<uint8_t>(L.lgray), ptr<uint8_t>(L.lgx), ptr<uint8_t>(L.lgy),
-                          ptr<uint32_t>(L.cl), ptr<unsigned long long>(L.cl)};
+                          ptr<uint32_t>(L.cl), ptr<unsigned long long>(L.cl),
+                          ptr<uint32_t>(L.rkey)};
         const AuxImage ri{dr, rstride, ptr<uint8_t>(L.rgray), ptr<uint8_t>(L.rgx), ptr<uint8_t>(L.rgy),
                           ptr<uint32_t>(L.cr), ptr<unsigned long long>(L.cr)};
         if (right_on_copy_) {
@@ -764,7 +765,6 @@ int Engine::run_pre(const uint8_t* dl, int lstride, const uint8_t* dr, int rstri
     if (cfg_.hier_enable && !hier_ran_) RUNC(cudaMemsetAsync(arena_ + L.hstats, 0, 32, s), "hier stats init");
     cudaEventRecord(ev_[2], s);
     // cost (+ cross-H, + right argmin)
-    RUNC(cudaMemsetAsync(ptr<uint32_t>(L.rkey), 0xFF, n * 4, s), "rkey init");
     const int lmax = std::max(1, cfg_.max_arm_length);
     const uint32_t* magic = ptr<uint32_t>(L.magic);
     if (L.raw_cost) RUN(launch_cost(cc, 0, lmax, cfg_.color_threshold, ptr<uint32_t>(L.volRaw), ptr<uint32_t>(L.rkey), magic, s), "cost(raw)");
@@ -787,11 +787,13 @@ int Engine::run_pre(const uint8_t* dl, int lstride, const uint8_t* dr, int rstri
         sgm_src = ptr<uint32_t>(L.volA);
     }
     cudaEventRecord(ev_[3], s);
-    // (in line: beside the sweeps' one-warp blocks, whose chains are all resident at once, another stream's
-    // blocks decide how many chains each SM steps; Fast 1280x720 D128 0.520 ms per frame with this kernel on
-    // a side stream and an even share of shared memory forced on the sweeps' blocks, 0.667 without the
-    // share, 0.490 in line)
-    RUN(launch_right_wta_finalize(cc, ptr<uint32_t>(L.rkey), cfg_.subpixel, ptr<float>(L.disp_right), s), "right wta");
+    // the right-image map is a launch of its own where more than the confidence stage reads it (the check
+    // after the refiner, the stage dumps); it runs in line: beside the sweeps' one-warp blocks, whose chains
+    // are all resident at once, another stream's blocks decide how many chains each SM steps (Fast 1280x720
+    // D128 0.520 ms per frame with it on a side stream, 0.490 in line)
+    right_written_ = refine_enabled() || debug_;
+    if (right_written_)
+        RUN(launch_right_wta_finalize(cc, ptr<uint32_t>(L.rkey), cfg_.subpixel, ptr<float>(L.disp_right), s), "right wta");
     cudaEventRecord(ev_[4], s);
     if (L.cross) {
         const int tau = cfg_.color_threshold;
@@ -986,7 +988,11 @@ int Engine::run_post(float* d_disp, float* d_conf, uint8_t* d_reason, uint8_t* d
     const bool refine = cfg_.refine_enable && cfg_.refine_iterations > 0;
     ConfLrArgs ca;
     ca.w = w; ca.h = h;
-    ca.disp = ptr<float>(L.disp_wta); ca.disp_right = ptr<float>(L.disp_right);
+    const CostCtx cc = cost_ctx();
+    ca.disp = ptr<float>(L.disp_wta);
+    ca.disp_right = right_written_ ? ptr<float>(L.disp_right) : nullptr;
+    ca.rkey = ptr<uint32_t>(L.rkey); ca.y0 = 0; ca.ctx = &cc; ca.subpixel = cfg_.subpixel;
+    ca.confidence2 = nullptr; ca.reliable2 = nullptr; ca.reason2 = nullptr;
     ca.best = ptr<float>(L.best); ca.second = ptr<float>(L.second);
     ca.lgx = ptr<uint8_t>(L.lgx); ca.lgy = ptr<uint8_t>(L.lgy);
     ca.uniqueness_ratio = cfg_.conf_uniqueness_ratio; ca.min_texture = cfg_.conf_min_texture;
@@ -998,6 +1004,12 @@ int Engine::run_post(float* d_disp, float* d_conf, uint8_t* d_reason, uint8_t* d
     ca.lr_check = cfg_.lr_check;
     ca.post_lr_max_diff = cfg_.post_lr_max_diff;
     ca.disp_out = ptr<float>(L.disp_lr);
+    // the caller's device buffers take their copies from the kernels that write the maps (an unaligned
+    // float buffer from a copy)
+    const bool conf_direct = d_conf && (reinterpret_cast<uintptr_t>(d_conf) & 3) == 0;
+    ca.confidence2 = conf_direct ? d_conf : nullptr;
+    ca.reliable2 = d_reliable;
+    ca.reason2 = refine && cfg_.lr_check ? nullptr : d_reason;
     RUN(launch_conf_lr(ca, s), "confidence");
     if (debug_) RUNC(cudaMemcpyAsync(ptr<uint8_t>(L.reason_conf), ptr<uint8_t>(L.reason), n, cudaMemcpyDeviceToDevice, s), "dbg");
     if (early_conf_ || early_rel_ || early_reason_) {
@@ -1025,7 +1037,7 @@ int Engine::run_post(float* d_disp, float* d_conf, uint8_t* d_reason, uint8_t* d
         cudaEventRecord(ev_[8], s);
         if (cfg_.lr_check) {
             RUN(launch_lr(w, h, cfg_.post_lr_max_diff, ptr<float>(L.disp_right), ptr<float>(L.disp_ref), ptr<float>(L.disp_lr),
-                          ptr<uint8_t>(L.reason), s), "lr");
+                          ptr<uint8_t>(L.reason), d_reason, s), "lr");
         } else {
             post_in = ptr<float>(L.disp_ref);
         }
@@ -1052,16 +1064,14 @@ int Engine::run_post(float* d_disp, float* d_conf, uint8_t* d_reason, uint8_t* d
     } else {
         RUNC(cudaMemcpyAsync(final_out, med_in, n * 4, cudaMemcpyDeviceToDevice, s), "copy");
     }
-    if (d_reason) RUNC(cudaMemcpyAsync(d_reason, ptr<uint8_t>(L.reason), n, cudaMemcpyDeviceToDevice, s), "reason out");
-    if (d_conf) RUNC(cudaMemcpyAsync(d_conf, ptr<float>(L.confidence), n * 4, cudaMemcpyDeviceToDevice, s), "conf out");
-    if (d_reliable) RUNC(cudaMemcpyAsync(d_reliable, ptr<uint8_t>(L.reliable), n, cudaMemcpyDeviceToDevice, s), "rel out");
+    if (d_conf && !conf_direct) RUNC(cudaMemcpyAsync(d_conf, ptr<float>(L.confidence), n * 4, cudaMemcpyDeviceToDevice, s), "conf out");
     if (d_disp && d_disp != ptr<float>(L.disp_out) && debug_)
         RUNC(cudaMemcpyAsync(ptr<float>(L.disp_out), d_disp, n * 4, cudaMemcpyDeviceToDevice, s), "dbg");
     // PipelineStats counters (src/pipeline.cpp:650-707); refine_changed compares the WTA map with
     // the refined one, prior_support_count is the prior's selected-support count
     unsigned long long* st = ptr<unsigned long long>(L.stats);
-    RUNC(cudaMemsetAsync(st, 0, 64, s), "stats init");
     const bool planes = range_planes_needed();
+    RUNC(cudaMemsetAsync(st, 0, 64, s), "stats init");
     RUN(launch_frame_stats((int)n, final_out, ptr<uint8_t>(L.reliable), ptr<uint8_t>(L.reason),
                            refine ? ptr<float>(L.disp_wta) : nullptr, refine ? ptr<float>(L.disp_ref) : nullptr,
                            planes ? ptr<int16_t>(L.rmin) : nullptr, planes ? ptr<int16_t>(L.rmax) : nullptr,
@@ -1118,7 +1128,11 @@ int Engine::run_banded(int nb, float* hdisp, float* hconf, uint8_t* hreason, uin
     RUNC(cudaStreamWaitEvent(ss, ev_fork_, 0), "event");
     ConfLrArgs ca;
     ca.w = w; ca.h = h;
-    ca.disp = ptr<float>(L.disp_wta); ca.disp_right = ptr<float>(L.disp_right);
+    const CostCtx cc = cost_ctx();
+    ca.disp = ptr<float>(L.disp_wta);
+    ca.disp_right = right_written_ ? ptr<float>(L.disp_right) : nullptr;
+    ca.rkey = ptr<uint32_t>(L.rkey); ca.y0 = 0; ca.ctx = &cc; ca.subpixel = cfg_.subpixel;
+    ca.confidence2 = nullptr; ca.reliable2 = nullptr; ca.reason2 = nullptr;
     ca.best = ptr<float>(L.best); ca.second = ptr<float>(L.second);
     ca.lgx = ptr<uint8_t>(L.lgx); ca.lgy = ptr<uint8_t>(L.lgy);
     ca.uniqueness_ratio = cfg_.conf_uniqueness_ratio; ca.min_texture = cfg_.conf_min_texture;
@@ -1170,7 +1184,9 @@ int Engine::run_banded(int nb, float* hdisp, float* hconf, uint8_t* hreason, uin
         const size_t o = (size_t)ylo * w, rows = (size_t)(yhi - ylo) * w;
         ConfLrArgs cb = ca;
         cb.h = yhi - ylo;
-        cb.disp += o; cb.disp_right += o; cb.best += o; cb.second += o; cb.lgx += o; cb.lgy += o;
+        cb.y0 = ylo;
+        if (cb.disp_right) cb.disp_right += o;
+        cb.disp += o; cb.best += o; cb.second += o; cb.lgx += o; cb.lgy += o;
         cb.confidence += o; cb.reliable += o; cb.reason += o; cb.disp_out += o;
         RUN(launch_conf_lr(cb, ps), "confidence");
         if (fill) {
@@ -1200,8 +1216,8 @@ int Engine::run_banded(int nb, float* hdisp, float* hconf, uint8_t* hreason, uin
     cudaEventRecord(ev_[8], ps);
     // PipelineStats counters over the whole map (src/pipeline.cpp:650-707)
     unsigned long long* st = ptr<unsigned long long>(L.stats);
-    RUNC(cudaMemsetAsync(st, 0, 64, ps), "stats init");
     const bool planes = range_planes_needed();
+    RUNC(cudaMemsetAsync(st, 0, 64, ps), "stats init");
     RUN(launch_frame_stats((int)n, final_map, ptr<uint8_t>(L.reliable), ptr<uint8_t>(L.reason), nullptr, nullptr,
                            planes ? ptr<int16_t>(L.rmin) : nullptr, planes ? ptr<int16_t>(L.rmax) : nullptr,
                            planes ? 0ull : default_range_width_sum(), st, ps),
@@ -1442,7 +1458,16 @@ int Engine::dump(int what, void* dst, size_t bytes) {
         case 13: off = L.disp_wta; sz = n * 4; break;
         case 14: off = L.best; sz = n * 4; break;
         case 15: off = L.second; sz = n * 4; break;
-        case 16: off = L.disp_right; sz = n * 4; break;
+        case 16:
+            off = L.disp_right;
+            sz = n * 4;
+            // without the refiner the confidence stage works the right disparities out itself: write the map
+            // now (the same values where the frame wrote it)
+            if (const cudaError_t e = launch_right_wta_finalize(cost_ctx(), ptr<uint32_t>(L.rkey), cfg_.subpixel,
+                                                                ptr<float>(L.disp_right), stream_);
+                e != cudaSuccess)
+                return cuda_fail(e, "right disparity");
+            break;
         case 17: off = L.confidence; sz = n * 4; break;
         case 18: off = L.reliable; sz = n; break;
         case 19: off = L.reason_conf; sz = n; break;

@@ -298,6 +298,7 @@ private:
     bool early_issued_ = false, early_reason_done_ = false;
     int* refine_err_host_ = nullptr;      // pinned copy of the refine error flag
     bool refine_pending_ = false;
+    bool right_written_ = false;  // the last frame wrote the right-image map (else its keys alone)
     bool counts_fresh_ = false;
     std::string err_;
 };

@@ -20,6 +20,7 @@ struct AuxImage {
     uint8_t *gray, *gx, *gy;
     uint32_t* census;
     unsigned long long* census64;
+    uint32_t* keys = nullptr;  // the argmin keys, set to 0xFFFFFFFF per pixel, or null
 };
 cudaError_t launch_aux(const AuxImage& left, const AuxImage& right, int ch, int w, int h, int census64,
                        cudaStream_t s);
@@ -138,7 +139,11 @@ cudaError_t launch_sgm_batch(const SgmBatchPlan& plan, int max_blocks_per_sm, cu
 struct ConfLrArgs {
     int w, h;
     const float* disp;
-    const float* disp_right;
+    const float* disp_right;    // the right-image map, or null: each pixel works it out from its right
+    const uint32_t* rkey;       // pixel's argmin key (the whole frame's keys and planes of `ctx`; the other
+    int y0;                     // pointers start at row y0)
+    const CostCtx* ctx;
+    int subpixel;
     const float* best;
     const float* second;
     const uint8_t* lgx;
@@ -150,10 +155,15 @@ struct ConfLrArgs {
     uint8_t* reason;
     int fuse_lr, lr_check, post_lr_max_diff;
     float* disp_out;
+    // second copies of the maps (the caller's device buffers), or null
+    float* confidence2;
+    uint8_t* reliable2;
+    uint8_t* reason2;
 };
 cudaError_t launch_conf_lr(const ConfLrArgs& a, cudaStream_t s);
+// reason2 (nullable): a second copy of the final reasons.
 cudaError_t launch_lr(int w, int h, int lr_max_diff, const float* dr, const float* din, float* dout,
-                      uint8_t* reason, cudaStream_t s);
+                      uint8_t* reason, uint8_t* reason2, cudaStream_t s);
 cudaError_t launch_fill(int w, int h, int gap, int shadow, apg_inpaint_telemetry_t* tel, const float* in,
                         const uint8_t* reason, const uint8_t* gray,
                         const float* d_prior, float* out, cudaStream_t s);

@@ -16,8 +16,18 @@ namespace {
 
 __device__ __forceinline__ float clampf(float v, float lo, float hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
-// Confidence (+ optional fused LR check when no refinement sits between them).
-__global__ void conf_lr_kernel(ConfLrArgs a) {
+// Confidence (+ optional fused LR check when no refinement sits between them).  KEYS 0: the right-image
+// disparity comes from its map; 1, 2: it is worked out here from the argmin keys (32- or 64-bit census),
+// once per left pixel that looks at it, which saves the map's own launch, write and read (a 1280x720 D128
+// frame: 5 us of the map's 20, the rest is the costs' own loads).  A second copy of each map goes to the
+// caller's buffer from here: the three device copies after the median took 18 us of every frame.
+template <int KEYS>
+__global__ void __launch_bounds__(256) conf_lr_kernel(ConfLrArgs a, CostCtx c) {
+    __shared__ float s_lut[KEYS ? kLutSize : 1];
+    if (KEYS) {
+        for (int i = threadIdx.x; i < kLutSize; i += blockDim.x) s_lut[i] = c.lut[i];
+        __syncthreads();
+    }
     const int n = a.w * a.h;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int y = i / a.w, x = i - y * a.w;
@@ -28,37 +38,36 @@ __global__ void conf_lr_kernel(ConfLrArgs a) {
             uniq = clampf(uniq, 0.f, 1.f);
         }
         const float d = a.disp[i];
-        float lr = 1.f;
-        {
-            const int xr = (int)roundf(__fsub_rn((float)x, d));
-            if (xr < 0 || xr >= a.w || d < 0.f) {
-                lr = 0.f;
-            } else {
-                const float dr = a.disp_right[y * a.w + xr];
-                if (dr < 0.f || fabsf(__fsub_rn(d, dr)) > __fadd_rn((float)a.conf_lr_max_diff, 0.5f)) lr = 0.f;
-            }
+        const int xr = (int)roundf(__fsub_rn((float)x, d));
+        const bool seen = d >= 0.f && xr >= 0 && xr < a.w;
+        float dr = -1.f;
+        if (seen) {
+            if constexpr (KEYS == 0) dr = a.disp_right[y * a.w + xr];
+            else dr = right_disparity<KEYS == 2>(c, s_lut, a.rkey[(size_t)(y + a.y0) * a.w + xr], y + a.y0, xr, a.subpixel);
         }
+        float lr = 1.f;
+        if (!seen || dr < 0.f || fabsf(__fsub_rn(d, dr)) > __fadd_rn((float)a.conf_lr_max_diff, 0.5f)) lr = 0.f;
         const float tex = (float)((int)a.lgx[i] + (int)a.lgy[i]);
         const float tex_term = clampf(__fdiv_rn(tex, 16.f), 0.f, 1.f);
         float conf = clampf(uniq, 0.f, 4.f);
         conf = __fmul_rn(conf, __fadd_rn(0.5f, __fmul_rn(0.5f, tex_term)));
         if (lr < 0.5f) conf = __fmul_rn(conf, 0.25f);
         a.confidence[i] = conf;
+        if (a.confidence2) a.confidence2[i] = conf;
         const bool lr_ok = lr >= 0.5f;
         const bool rel = lr_ok && conf >= a.reliable_threshold && uniq >= a.uniqueness_ratio &&
                          tex >= a.min_texture && d >= 0.f;
         a.reliable[i] = rel ? 1 : 0;
+        if (a.reliable2) a.reliable2[i] = rel ? 1 : 0;
         uint8_t reason = rel ? kValid : (lr_ok ? kLowConfidence : kMismatch);
         if (a.fuse_lr) {
             float dout = d;
             if (a.lr_check && d >= 0.f) {
                 const float tol = __fadd_rn((float)a.post_lr_max_diff, 0.5f);
-                const int xr = (int)roundf(__fsub_rn((float)x, d));
-                if (xr < 0 || xr >= a.w) {
+                if (!seen) {
                     dout = -1.f;
                     reason = kOcclusion;
                 } else {
-                    const float dr = a.disp_right[y * a.w + xr];
                     if (dr < 0.f || fabsf(__fsub_rn(d, dr)) > tol) {
                         dout = -1.f;
                         reason = (dr > __fadd_rn(d, tol)) ? kOcclusion : kMismatch;
@@ -68,31 +77,34 @@ __global__ void conf_lr_kernel(ConfLrArgs a) {
             a.disp_out[i] = dout;
         }
         a.reason[i] = reason;
+        if (a.reason2) a.reason2[i] = reason;
     }
 }
 
 // Stand-alone LR check (after refinement), src/postprocess.cpp:10-40.
 __global__ void lr_kernel(int w, int h, int lr_max_diff, const float* __restrict__ dr_img,
-                          const float* __restrict__ din, float* __restrict__ dout, uint8_t* __restrict__ reason) {
+                          const float* __restrict__ din, float* __restrict__ dout, uint8_t* reason, uint8_t* reason2) {
     const int n = w * h;
     const float tol = __fadd_rn((float)lr_max_diff, 0.5f);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int y = i / w, x = i - y * w;
         const float d = din[i];
         float o = d;
+        int fail = -1;
         if (d >= 0.f) {
             const int xr = (int)roundf(__fsub_rn((float)x, d));
             if (xr < 0 || xr >= w) {
-                o = -1.f;
-                reason[i] = kOcclusion;
+                fail = kOcclusion;
             } else {
                 const float dr = dr_img[y * w + xr];
-                if (dr < 0.f || fabsf(__fsub_rn(d, dr)) > tol) {
-                    o = -1.f;
-                    reason[i] = (dr > __fadd_rn(d, tol)) ? kOcclusion : kMismatch;
-                }
+                if (dr < 0.f || fabsf(__fsub_rn(d, dr)) > tol) fail = (dr > __fadd_rn(d, tol)) ? kOcclusion : kMismatch;
+            }
+            if (fail >= 0) {
+                o = -1.f;
+                reason[i] = (uint8_t)fail;
             }
         }
+        if (reason2) reason2[i] = fail >= 0 ? (uint8_t)fail : reason[i];
         dout[i] = o;
     }
 }
@@ -489,13 +501,16 @@ inline int grid_for(int n) {
 }  // namespace
 
 cudaError_t launch_conf_lr(const ConfLrArgs& a, cudaStream_t s) {
-    conf_lr_kernel<<<grid_for(a.w * a.h), 256, 0, s>>>(a);
+    const int blocks = grid_for(a.w * a.h);
+    if (a.disp_right) conf_lr_kernel<0><<<blocks, 256, 0, s>>>(a, CostCtx{});
+    else if (!a.ctx->census64) conf_lr_kernel<1><<<blocks, 256, 0, s>>>(a, *a.ctx);
+    else conf_lr_kernel<2><<<blocks, 256, 0, s>>>(a, *a.ctx);
     return cudaGetLastError();
 }
 
 cudaError_t launch_lr(int w, int h, int lr_max_diff, const float* dr, const float* din, float* dout,
-                      uint8_t* reason, cudaStream_t s) {
-    lr_kernel<<<grid_for(w * h), 256, 0, s>>>(w, h, lr_max_diff, dr, din, dout, reason);
+                      uint8_t* reason, uint8_t* reason2, cudaStream_t s) {
+    lr_kernel<<<grid_for(w * h), 256, 0, s>>>(w, h, lr_max_diff, dr, din, dout, reason, reason2);
     return cudaGetLastError();
 }
 
