@@ -25,12 +25,19 @@
 //     r = x - d0 - di receives (x, di) at step x in lane di/P.  Each lane keeps the running minimum
 //     keys (cost << 16 | di: lowest cost first, then lowest d) of its P right pixels; every step
 //     the oldest moves one lane up (a shuffle), and the one leaving lane 31 -- complete over this
-//     run -- goes to a per-warp buffer that is merged into rkey with atomicMin at the end of the
-//     run, together with the partial minima still held.  min is idempotent, so a halo pixel seen
-//     by two tiles changes nothing.
+//     run -- goes to a per-warp buffer; at the end of the run these and the partial minima still
+//     held are merged into the tile's keys in shared memory, and those into rkey with one coalesced
+//     atomicMin per right pixel of the tile.  min is idempotent, so a halo pixel seen by two tiles
+//     changes nothing.
+//
+// Bound: issue slots and the shared-memory gathers (two table entries per voxel, 3.5 and 2.4 bank passes a
+// warp on textured frames), then the population count (eight cycles a warp instruction).  Merging the keys in
+// shared memory, testing validity by two packed compares per word and walking the tiles by columns took the
+// kernel from 439 to 239 us (Fast 1920x1080 D256), 267 to 250 (Balanced 1280x720 D128), 264 to 235 (997x611).
 //
 // Blocks are persistent: each builds its tables once and then walks (row, column tile) items.
 #include <algorithm>
+#include <cmath>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -45,7 +52,7 @@ constexpr int kT2Rows = 33;
 
 struct RunGeom {
     int txc, ha, nx, nr, roff, rl, nrun, ntx, ntiles;
-    size_t t2, lgt, q, magic, arm, lc, lg, rc, rg, rng, pre, cnt, tot, totc, emit, total;
+    size_t t2, lgt, q, magic, arm, lc, lg, rc, rg, rng, pre, cnt, tot, totc, emit, key, total;
 };
 
 inline size_t a16(size_t v) { return (v + 15) & ~size_t(15); }
@@ -54,8 +61,8 @@ inline int run_warps(bool cross) { return cross ? 16 : 8; }
 
 // Staging and table layout of one block for a tile of txc columns with halo ha.  nx (staged left
 // pixels) and rl (run length) are multiples of 4 (16-byte loads of four left descriptors); roff
-// shifts the staged right row so that each step group's right descriptors start at an even index
-// (8-byte loads) and every lane with a disparity inside the range finds its whole window staged.
+// shifts the staged right row so that each step group's right descriptors start at a multiple of four
+// (16-byte loads) or, with 64 or 192 padded disparities, an even index (8-byte loads) and every lane with a disparity inside the range finds its whole window staged.
 // One run per warp.
 RunGeom run_geom(const CostCtx& c, int txc, int ha, bool cross, bool full, bool prior) {
     RunGeom g{};
@@ -65,9 +72,11 @@ RunGeom run_geom(const CostCtx& c, int txc, int ha, bool cross, bool full, bool 
     g.nrun = run_warps(cross);
     g.nx = round_up(txc + 2 * ha, 4);
     g.rl = round_up((g.nx + g.nrun - 1) / g.nrun, 4);
-    // even start for every step group, plus P entries so that a lane holding any disparity of the
-    // range loads its own window without clamping
-    g.roff = ((c.D - 1) % 2 == 0 ? 2 : 1) + c.Dp / 32;
+    // aligned start for every step group (of four entries where P is a multiple of four, else of two),
+    // plus P entries so that a lane holding any disparity of the range loads its own window without
+    // clamping
+    const int P = c.Dp / 32;
+    g.roff = (P % 4 == 0 ? (4 - (c.D - 1) % 4) % 4 : ((c.D - 1) % 2 == 0 ? 2 : 1)) + P;
     g.nr = round_up(g.nx + c.D - 1 + g.roff, 4);
     g.ntx = (c.w + txc - 1) / txc;
     g.ntiles = g.ntx * c.h;
@@ -88,6 +97,7 @@ RunGeom run_geom(const CostCtx& c, int txc, int ha, bool cross, bool full, bool 
     g.tot = o; o = a16(o + (cross ? (size_t)g.nrun * W2 * 4 : 0));
     g.totc = o; o = a16(o + (cross && prior ? (size_t)g.nrun * W2 * 2 : 0));
     g.emit = o; o = a16(o + (size_t)g.nrun * g.rl * 4);
+    g.key = o; o = a16(o + (size_t)(g.nx + c.Dp) * 4);  // argmin keys of the tile's right pixels
     g.total = o;
     return g;
 }
@@ -118,6 +128,13 @@ __device__ __forceinline__ unsigned long long f2mul_rn(unsigned long long a, uns
 }
 __device__ __forceinline__ unsigned long long f2pack(float lo, float hi) {
     return (unsigned long long)__float_as_uint(lo) | ((unsigned long long)__float_as_uint(hi) << 32);
+}
+
+// 0xFFFF in each half whose top bit is set (the permute's sign mode: bytes 1 and 3), else 0
+__device__ __forceinline__ uint32_t spread_top_bits(uint32_t v) {
+    uint32_t r;
+    asm("prmt.b32 %0, %1, 0, 0xBB99;" : "=r"(r) : "r"(v));
+    return r;
 }
 
 template <bool FULL>
@@ -177,18 +194,21 @@ __device__ __forceinline__ void run_steps(const CostCtx& c, const RunGeom& g, in
                                           const uint32_t* s_rg, const float* s_t2, const float* s_lgt,
                                           const uint32_t* s_q, const uint32_t* s_rng, uint32_t* s_pre,
                                           uint16_t* s_cnt, uint32_t* s_tot, uint16_t* s_totc, uint32_t* s_em,
-                                          int run, uint32_t* __restrict__ out_vol, uint32_t* __restrict__ rkey) {
+                                          uint32_t* s_key, int run, uint32_t* __restrict__ out_vol) {
     constexpr int P = 2 * WPL;
     constexpr int W2 = 32 * WPL;
     const int lane = threadIdx.x & 31;
     const int dbase = P * lane;  // first disparity index of this lane
     const unsigned long long scale2 = f2pack(c.scale, c.scale);
     const uint32_t cmax2 = (uint32_t)c.cost_max * 0x00010001u;
-    // lanes wholly past the range load at the last in-bounds even base (dl + P <= D + roff keeps
-    // every window entry inside the staged row; even keeps the 8-byte loads aligned) and are
-    // masked; a lane with any disparity below D has dbase <= D - 1 < D + roff - P, so keeps its own
-    const int dl = V ? dbase : min(dbase, (c.D + g.roff - P) & ~1);
-    int ri = xs - dl + c.D - 1 + g.roff;  // staged right descriptor of (xs, dl); even
+    // a step group's four right descriptors in one load where the lanes' windows allow it: at a stride of
+    // P words, two 8-byte loads would hit every bank twice as often
+    constexpr bool kWide = P % 4 == 0;
+    // lanes wholly past the range load at the last in-bounds aligned base (dl + P <= D + roff keeps
+    // every window entry inside the staged row) and are masked; a lane with any disparity below D has
+    // dbase <= D - 1 < D + roff - P (rounded down to the alignment too), so keeps its own
+    const int dl = V ? dbase : min(dbase, (c.D + g.roff - P) & (kWide ? ~3 : ~1));
+    int ri = xs - dl + c.D - 1 + g.roff;  // staged right descriptor of (xs, dl); aligned
     uint32_t wc[P], wg[P], acc[P], pre[WPL], cnt[WPL];
 #pragma unroll
     for (int j = 0; j < P; ++j) {
@@ -208,13 +228,25 @@ __device__ __forceinline__ void run_steps(const CostCtx& c, const RunGeom& g, in
         const uint4 lc4 = *reinterpret_cast<const uint4*>(s_lc + xi);
         uint4 lg4 = make_uint4(0, 0, 0, 0);
         if (FULL) lg4 = *reinterpret_cast<const uint4*>(s_lg + xi);
-        const uint2 na = *reinterpret_cast<const uint2*>(s_rc + ri);
-        const uint2 nb = *reinterpret_cast<const uint2*>(s_rc + ri + 2);
-        uint2 ga = make_uint2(0, 0), gb = make_uint2(0, 0);
-        if (FULL) {
-            ga = *reinterpret_cast<const uint2*>(s_rg + ri);
-            gb = *reinterpret_cast<const uint2*>(s_rg + ri + 2);
+        uint2 na, nb, ga = make_uint2(0, 0), gb = make_uint2(0, 0);
+        if constexpr (kWide) {
+            const uint4 nc = *reinterpret_cast<const uint4*>(s_rc + ri);
+            na = make_uint2(nc.x, nc.y);
+            nb = make_uint2(nc.z, nc.w);
+            if (FULL) {
+                const uint4 ng = *reinterpret_cast<const uint4*>(s_rg + ri);
+                ga = make_uint2(ng.x, ng.y);
+                gb = make_uint2(ng.z, ng.w);
+            }
+        } else {
+            na = *reinterpret_cast<const uint2*>(s_rc + ri);
+            nb = *reinterpret_cast<const uint2*>(s_rc + ri + 2);
+            if (FULL) {
+                ga = *reinterpret_cast<const uint2*>(s_rg + ri);
+                gb = *reinterpret_cast<const uint2*>(s_rg + ri + 2);
+            }
         }
+        uint32_t em[4];
         const uint32_t L[4] = {lc4.x, lc4.y, lc4.z, lc4.w};
         const uint32_t LG[4] = {lg4.x, lg4.y, lg4.z, lg4.w};
         const uint32_t NC[4] = {na.x, na.y, nb.x, nb.y};
@@ -231,47 +263,46 @@ __device__ __forceinline__ void run_steps(const CostCtx& c, const RunGeom& g, in
             wg[0] = NG[s];
             uint32_t qp[WPL];  // quantised costs of disparities 2w | 2w + 1 << 16
             uint32_t vm[WPL];  // their validity: 0xFFFF per valid half
-            uint32_t rmask = 0xFFFFu;  // this lane's disparities inside the left pixel's range
-            if (PRIOR) {
-                const uint32_t rg = s_rng[xi + s];
-                const int base = c.d0 + dbase;
-                const int a0 = min(max((int)(int16_t)(rg & 0xFFFFu) - base, 0), P);
-                const int a1 = min(max((int)(int16_t)(rg >> 16) - base, 0), P);
-                rmask = ((1u << a1) - 1u) & ~((1u << a0) - 1u);
+            // this lane's valid disparities [lo, hi) of the pixel: inside its own range (PRIOR), inside
+            // the image and the range (!V).  Both bounds in both halves, biased so that a difference's
+            // top bit is the comparison's outcome
+            uint32_t lo2 = 0, hi2 = 0;
+            if (!V || PRIOR) {
+                int lo = 0, hi = P;
+                if (PRIOR) {
+                    const uint32_t rg = s_rng[xi + s];
+                    const int base = c.d0 + dbase;
+                    lo = (int)(int16_t)(rg & 0xFFFFu) - base;
+                    hi = (int)(int16_t)(rg >> 16) - base;
+                }
+                if (!V) {
+                    const int xd = x - c.d0 - dbase;  // right column of the lane's first disparity
+                    lo = max(lo, xd - (c.w - 1));
+                    hi = min(min(hi, xd + 1), c.D - dbase);
+                    if (x < 0 || x >= c.w) hi = 0;
+                }
+                lo2 = (uint32_t)min(max(lo, 0), P) * 0x00010001u;
+                hi2 = (uint32_t)min(max(hi, 0), P) * 0x00010001u + 0x7FFF7FFFu;
             }
 #pragma unroll
             for (int w = 0; w < WPL; ++w) {
                 qp[w] = run_cost2<FULL>(L[s], LG[s], wc[2 * w], wg[2 * w], wc[2 * w + 1], wg[2 * w + 1], s_t2, s_lgt,
                                         s_q, scale2, cmax2);
                 vm[w] = 0xFFFFFFFFu;
+                uint32_t qk = qp[w];
                 if (!V || PRIOR) {
-                    uint32_t m = 0;
-#pragma unroll
-                    for (int hs = 0; hs < 2; ++hs) {
-                        const int j = 2 * w + hs;
-                        bool ok = true;
-                        if (!V) {
-                            const int di = dbase + j, xr = x - c.d0 - di;
-                            ok = x >= 0 && x < c.w && di < c.D && xr >= 0 && xr < c.w;
-                        }
-                        if (PRIOR) ok = ok && ((rmask >> j) & 1u);
-                        if (ok) m |= 0xFFFFu << (16 * hs);
-                    }
-                    vm[w] = m;
+                    const uint32_t jp = (uint32_t)(2 * w) | ((uint32_t)(2 * w + 1) << 16);
+                    // top bit of each half: j >= lo and j < hi, spread over the half
+                    vm[w] = spread_top_bits(((jp | 0x80008000u) - lo2) & (hi2 - jp));
+                    qk |= ~vm[w];
                 }
-#pragma unroll
-                for (int hs = 0; hs < 2; ++hs) {
-                    const int j = 2 * w + hs;
-                    // key (cost << 16 | disparity index), or the invalid word
-                    const uint32_t key = hs == 0 ? ((qp[w] << 16) | (uint32_t)(dbase + j))
-                                                 : ((qp[w] & 0xFFFF0000u) | (uint32_t)(dbase + j));
-                    const bool ok = (V && !PRIOR) || ((vm[w] >> (16 * hs)) & 1u);
-                    acc[j] = min(acc[j], ok ? key : kInvalidWord);
-                }
+                // keys (cost << 16 | disparity index); an invalid voxel's is 0xFFFF0000 or more, above any cost
+                acc[2 * w] = min(acc[2 * w], (qk << 16) | (uint32_t)(dbase + 2 * w));
+                acc[2 * w + 1] = min(acc[2 * w + 1], (qk & 0xFFFF0000u) | (uint32_t)(dbase + 2 * w + 1));
             }
             // the oldest minimum moves one lane up; lane 31's is complete for this run
             const uint32_t out = acc[P - 1];
-            if (lane == 31) s_em[xi - xs + s] = out;
+            em[s] = out;
             const uint32_t in = __shfl_up_sync(0xFFFFFFFFu, out, 1);
 #pragma unroll
             for (int j = P - 1; j > 0; --j) acc[j] = acc[j - 1];
@@ -310,6 +341,7 @@ __device__ __forceinline__ void run_steps(const CostCtx& c, const RunGeom& g, in
                 }
             }
         }
+        if (lane == 31) *reinterpret_cast<uint4*>(s_em + (xi - xs)) = make_uint4(em[0], em[1], em[2], em[3]);
         ri += 4;
         pp += 4 * W2;
         cp += 4 * W2;
@@ -318,21 +350,15 @@ __device__ __forceinline__ void run_steps(const CostCtx& c, const RunGeom& g, in
     }
     __syncwarp();
     if (xe > xs) {
-        // minima that left lane 31 at step xs + e: right pixel xbase + xs + e - d0 - (Dp - 1)
+        // into the tile's keys (index 0: right pixel xbase - d0 - (Dp - 1)): the minima that left lane 31 at
+        // step xs + e, and the partial ones still held (acc[j] is of right pixel xbase + xe - d0 - dbase - j)
         const int n = xe - xs;
-        const int r0 = xbase + xs - c.d0 - (2 * W2 - 1);
-        for (int e = lane; e < n; e += 32) {
-            const uint32_t m = s_em[e];
-            const int r = r0 + e;
-            if (m != kInvalidWord && r >= 0 && r < c.w) atomicMin(rkey + row + r, m);
-        }
-        // partial minima still held: acc[j] is for right pixel xl + 1 - d0 - dbase - j
-        const int r1 = xbase + xe - c.d0 - dbase;
+        for (int e = lane; e < n; e += 32)
+            if (s_em[e] < 0xFFFF0000u) atomicMin(s_key + xs + e, s_em[e]);
+        uint32_t* kp = s_key + xe - dbase + 2 * W2 - 1;
 #pragma unroll
-        for (int j = 0; j < P; ++j) {
-            const int r = r1 - j;
-            if (acc[j] != kInvalidWord && r >= 0 && r < c.w) atomicMin(rkey + row + r, acc[j]);
-        }
+        for (int j = 0; j < P; ++j)
+            if (acc[j] < 0xFFFF0000u) atomicMin(kp - j, acc[j]);
     }
     __syncwarp();
     if (CROSS) store_words<WPL>(s_tot + run * W2 + WPL * lane, pre);
@@ -415,6 +441,7 @@ __global__ void __launch_bounds__(CROSS ? 512 : 256, CROSS ? (WPL > 2 ? 1 : 2) :
     uint16_t* s_totc = reinterpret_cast<uint16_t*>(smem + g.totc);
     const int tid = threadIdx.x, nt = blockDim.x, run = tid >> 5, lane = tid & 31;
     uint32_t* s_em = reinterpret_cast<uint32_t*>(smem + g.emit) + run * g.rl;
+    uint32_t* s_key = reinterpret_cast<uint32_t*>(smem + g.key);
 
     if (FULL) {
         for (int i = tid; i < 256 * kT2Rows; i += nt) {
@@ -433,12 +460,17 @@ __global__ void __launch_bounds__(CROSS ? 512 : 256, CROSS ? (WPL > 2 ? 1 : 2) :
     const int xs = min(run * g.rl, g.nx), xe = min(xs + g.rl, g.nx);
 
     for (int tile = blockIdx.x; tile < g.ntiles; tile += gridDim.x) {
-        const int y = tile / g.ntx;
-        const int x0 = (tile - y * g.ntx) * g.txc;
+        // column by column: the left ones, whose voxels reach out of the image and are tested one by one,
+        // then fall on every block alike (row by row, a number of blocks divisible by the tiles of a row
+        // gave them all to the same blocks: Fast 1920x1080 D256 in four tiles, 287 us)
+        const int col = tile / c.h;
+        const int y = tile - col * c.h;
+        const int x0 = col * g.txc;
         const int xbase = x0 - g.ha;
         const int rbase = xbase - (c.d0 + c.D - 1) - g.roff;  // image column of staged right 0
         const int row = y * c.w;
         __syncthreads();  // the previous item's readers are done with the staging
+        for (int i = tid; i < g.nx + c.Dp; i += nt) s_key[i] = kInvalidWord;
         for (int i = tid; i < g.nx; i += nt) {
             const int x = xbase + i;
             const bool in = x >= 0 && x < c.w;
@@ -478,14 +510,23 @@ __global__ void __launch_bounds__(CROSS ? 512 : 256, CROSS ? (WPL > 2 ? 1 : 2) :
             if (__all_sync(0xFFFFFFFFu, ok))
                 run_steps<true, CROSS, STORE, FULL, WPL, PRIOR, U8>(c, g, row, xbase, xs, xe, s_lc, s_lg, s_rc, s_rg, s_t2,
                                                                 s_lgt, s_q, s_rng, s_pre, s_cnt, s_tot, s_totc, s_em,
-                                                                run, out_vol, rkey);
+                                                                s_key, run, out_vol);
             else
                 run_steps<false, CROSS, STORE, FULL, WPL, PRIOR, U8>(c, g, row, xbase, xs, xe, s_lc, s_lg, s_rc, s_rg,
                                                                  s_t2, s_lgt, s_q, s_rng, s_pre, s_cnt, s_tot, s_totc,
-                                                                 s_em, run, out_vol, rkey);
+                                                                 s_em, s_key, run, out_vol);
+        }
+        __syncthreads();
+        {
+            // the tile's keys (from the last thread down: the first ones scan the run offsets)
+            const int r0 = xbase - c.d0 - (c.Dp - 1);
+            for (int i = nt - 1 - tid; i < g.nx + c.Dp; i += nt) {
+                const uint32_t m = s_key[i];
+                const int r = r0 + i;
+                if (m != kInvalidWord && r >= 0 && r < c.w) atomicMin(rkey + row + r, m);
+            }
         }
         if (CROSS) {
-            __syncthreads();
             // run offsets: the run totals become an exclusive prefix over the runs, per word, so a
             // window's sum is two lookups whatever number of runs it spans (sums wrap modulo 2^32
             // and counts modulo 2^16; the window differences are exact, as for the prefixes)
@@ -519,8 +560,12 @@ __global__ void __launch_bounds__(CROSS ? 512 : 256, CROSS ? (WPL > 2 ? 1 : 2) :
                 const int rlo = (int)((arm >> 16) & 0xFFu), rhi = (int)(arm >> 24);
                 const int sxi = xi + g.ha, a = sxi - l, b = sxi + r;
                 const uint4 pb = *reinterpret_cast<const uint4*>(s_pre + b * W2 + k4);
-                const uint4 ob = *reinterpret_cast<const uint4*>(s_tot + rhi * W2 + k4);
-                const uint4 oa = *reinterpret_cast<const uint4*>(s_tot + rlo * W2 + k4);
+                // the offsets of the runs at the window's ends cancel where it lies in one run
+                uint4 ob = make_uint4(0, 0, 0, 0), oa = ob;
+                if (rhi != rlo) {
+                    ob = *reinterpret_cast<const uint4*>(s_tot + rhi * W2 + k4);
+                    oa = *reinterpret_cast<const uint4*>(s_tot + rlo * W2 + k4);
+                }
                 const uint4 pa = a > 0 ? *reinterpret_cast<const uint4*>(s_pre + (a - 1) * W2 + k4) : make_uint4(0, 0, 0, 0);
                 const uint32_t sum[4] = {(pb.x + ob.x) - (pa.x + oa.x), (pb.y + ob.y) - (pa.y + oa.y),
                                          (pb.z + ob.z) - (pa.z + oa.z), (pb.w + ob.w) - (pa.w + oa.w)};
@@ -611,10 +656,33 @@ int cross_tile(const CostCtx& c, int lmax, bool full) {
     return 32;
 }
 
+// Tile width without aggregation (no halo): eight runs of up to kMaxRun pixels.  A run's end costs its warp
+// about kRunEnd steps more (the partial minima, the barrier), blocks walk the tiles in rounds whose last is
+// partly empty, and warps past the row's end idle: the run length with the least rounds (half counted whole,
+// half as the fraction used) times run, times the square of the padding.  Over run lengths of 20 to 120 at
+// 640x480 to 1920x1080, D 64 to 256, the choice was within 9% of the best one (Fast 1920x1080 D256: 80 pixels
+// 239 us, 32 pixels 276; 1280x720 D128: 80 pixels 67 us, 60 pixels 78).
+constexpr int kMaxRun = 96, kRunEnd = 8;
+int plain_tile(const CostCtx& c, int blocks) {
+    const int nrun = run_warps(false);
+    int best = 0;
+    double best_cost = 0;
+    for (int rl = 4; rl <= kMaxRun; rl += 4) {
+        const int txc = rl * nrun, ntx = (c.w + txc - 1) / txc;
+        const double rounds = (double)ntx * c.h / blocks, pad = (double)ntx * txc / c.w;
+        const double cost = (std::ceil(rounds) + rounds) * (rl + kRunEnd) * pad * pad;
+        if (!best || cost < best_cost) {
+            best_cost = cost;
+            best = txc;
+        }
+    }
+    return best;
+}
+
 template <bool CROSS, bool STORE, bool FULL, int WPL, bool PRIOR, bool U8>
 cudaError_t launch_runs_w(const CostCtx& c, int txc, int lmax, int tau, uint32_t* vol, uint32_t* rkey,
                           const uint32_t* magic, cudaStream_t s) {
-    const RunGeom g = run_geom(c, txc, CROSS ? lmax : 0, CROSS, FULL, PRIOR);
+    RunGeom g = run_geom(c, txc, CROSS ? lmax : 0, CROSS, FULL, PRIOR);
     const int nt = 32 * g.nrun;
     auto kern = cost_run_kernel<CROSS, STORE, FULL, WPL, PRIOR, U8>;
     cudaError_t e = allow_dynamic_smem(kern, g.total);
@@ -624,6 +692,8 @@ cudaError_t launch_runs_w(const CostCtx& c, int txc, int lmax, int tau, uint32_t
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nt, g.total);
     if (e != cudaSuccess) return e;
+    // the widest tile's staging decided the occupancy; a narrower one needs less
+    if (!CROSS) g = run_geom(c, plain_tile(c, std::max(1, per_sm) * nsm), 0, CROSS, FULL, PRIOR);
     const int blocks = std::max(1, std::min(g.ntiles, std::max(1, per_sm) * nsm));
     kern<<<blocks, nt, g.total, s>>>(c, g, lmax, tau, vol, rkey, magic);
     return cudaGetLastError();
@@ -667,7 +737,7 @@ size_t cost_runs_smem_bytes(const CostCtx& c, int mode, int lmax) {
     const bool full = c.use_ad || c.use_grad;
     const bool prior = c.prior_ranges != 0;
     if (mode == 1) return run_geom(c, cross_tile(c, lmax, full), lmax, true, full, prior).total;
-    return run_geom(c, 256, 0, false, full, prior).total;
+    return run_geom(c, kMaxRun * run_warps(false), 0, false, full, prior).total;
 }
 
 bool cost_runs_supported(const CostCtx& c, int mode, int lmax) {
@@ -689,9 +759,9 @@ cudaError_t launch_cost_runs(const CostCtx& c, int mode, int lmax, int tau, uint
                     : launch_runs_t<true, true, false>(c, txc, lmax, tau, vol, rkey, magic, s);
     }
     if (mode == 0)
-        return full ? launch_runs_t<false, true, true>(c, 256, lmax, tau, vol, rkey, magic, s)
-                    : launch_runs_t<false, true, false>(c, 256, lmax, tau, vol, rkey, magic, s);
-    return launch_runs_t<false, false, false>(c, 256, lmax, tau, vol, rkey, magic, s);
+        return full ? launch_runs_t<false, true, true>(c, kMaxRun * run_warps(false), lmax, tau, vol, rkey, magic, s)
+                    : launch_runs_t<false, true, false>(c, kMaxRun * run_warps(false), lmax, tau, vol, rkey, magic, s);
+    return launch_runs_t<false, false, false>(c, kMaxRun * run_warps(false), lmax, tau, vol, rkey, magic, s);
 }
 
 }  // namespace apgcu
