@@ -34,6 +34,8 @@
 // warp on textured frames), then the population count (eight cycles a warp instruction).  Merging the keys in
 // shared memory, testing validity by two packed compares per word and walking the tiles by columns took the
 // kernel from 439 to 239 us (Fast 1920x1080 D256), 267 to 250 (Balanced 1280x720 D128), 264 to 235 (997x611).
+// Where the ranges are narrow (the coarse pass leaves about 10 of 128 disparities a pixel), 64 disparities a run
+// and quads by range: hierarchical 1280x720 D128 362 -> 268 us, HighQuality 1920x1080 D256 1466 -> 1437.
 //
 // Blocks are persistent: each builds its tables once and then walks (row, column tile) items.
 #include <algorithm>
@@ -188,17 +190,17 @@ __device__ __forceinline__ void store_counts(uint16_t* p, const uint32_t (&c)[N]
 // every lane of the warp (no per-voxel tests).
 // PRIOR: every left pixel has its own range [lo, hi) (staged in s_rng); a voxel outside it is
 // invalid, and the aggregation also keeps a prefix of valid counts (s_cnt, s_totc).
-template <bool V, bool CROSS, bool STORE, bool FULL, int WPL, bool PRIOR, bool U8>
+// W2: words per pixel of the volume.  The lanes' words start at kb (0 where the warp covers them all).
+template <bool V, bool CROSS, bool STORE, bool FULL, int WPL, int W2, bool PRIOR, bool U8>
 __device__ __forceinline__ void run_steps(const CostCtx& c, const RunGeom& g, int row, int xbase, int xs, int xe,
                                           const uint32_t* s_lc, const uint32_t* s_lg, const uint32_t* s_rc,
                                           const uint32_t* s_rg, const float* s_t2, const float* s_lgt,
                                           const uint32_t* s_q, const uint32_t* s_rng, uint32_t* s_pre,
                                           uint16_t* s_cnt, uint32_t* s_tot, uint16_t* s_totc, uint32_t* s_em,
-                                          uint32_t* s_key, int run, uint32_t* __restrict__ out_vol) {
+                                          uint32_t* s_key, int run, int kb, uint32_t* __restrict__ out_vol) {
     constexpr int P = 2 * WPL;
-    constexpr int W2 = 32 * WPL;
     const int lane = threadIdx.x & 31;
-    const int dbase = P * lane;  // first disparity index of this lane
+    const int dbase = P * lane + 2 * kb;  // first disparity index of this lane
     const unsigned long long scale2 = f2pack(c.scale, c.scale);
     const uint32_t cmax2 = (uint32_t)c.cost_max * 0x00010001u;
     // a step group's four right descriptors in one load where the lanes' windows allow it: at a stride of
@@ -219,8 +221,8 @@ __device__ __forceinline__ void run_steps(const CostCtx& c, const RunGeom& g, in
     }
 #pragma unroll
     for (int w = 0; w < WPL; ++w) pre[w] = cnt[w] = 0;
-    uint32_t* pp = s_pre + xs * W2 + WPL * lane;                             // prefix words of (xs)
-    uint16_t* cp = s_cnt + xs * W2 + WPL * lane;                             // count words of (xs)
+    uint32_t* pp = s_pre + xs * W2 + kb + WPL * lane;                             // prefix words of (xs)
+    uint16_t* cp = s_cnt + xs * W2 + kb + WPL * lane;                             // count words of (xs)
     uint32_t* vp = out_vol + ((size_t)row + (xbase + xs)) * W2 + WPL * lane;  // volume words of (xs)
     // byte volume: the lane's P disparities of (xs)
     uint8_t* vp8 = reinterpret_cast<uint8_t*>(out_vol) + ((size_t)row + (xbase + xs)) * (2 * W2) + P * lane;
@@ -353,16 +355,17 @@ __device__ __forceinline__ void run_steps(const CostCtx& c, const RunGeom& g, in
         // into the tile's keys (index 0: right pixel xbase - d0 - (Dp - 1)): the minima that left lane 31 at
         // step xs + e, and the partial ones still held (acc[j] is of right pixel xbase + xe - d0 - dbase - j)
         const int n = xe - xs;
+        uint32_t* ke = s_key + xs + 2 * (W2 - 32 * WPL - kb);
         for (int e = lane; e < n; e += 32)
-            if (s_em[e] < 0xFFFF0000u) atomicMin(s_key + xs + e, s_em[e]);
+            if (s_em[e] < 0xFFFF0000u) atomicMin(ke + e, s_em[e]);
         uint32_t* kp = s_key + xe - dbase + 2 * W2 - 1;
 #pragma unroll
         for (int j = 0; j < P; ++j)
             if (acc[j] < 0xFFFF0000u) atomicMin(kp - j, acc[j]);
     }
     __syncwarp();
-    if (CROSS) store_words<WPL>(s_tot + run * W2 + WPL * lane, pre);
-    if (CROSS && PRIOR) store_counts<WPL>(s_totc + run * W2 + WPL * lane, cnt);
+    if (CROSS) store_words<WPL>(s_tot + run * W2 + kb + WPL * lane, pre);
+    if (CROSS && PRIOR) store_counts<WPL>(s_totc + run * W2 + kb + WPL * lane, cnt);
 }
 
 // floor(s / n) of a window sum and its count, by the table's reciprocal m of n: 2^32 / n (div_by_magic),
@@ -502,21 +505,57 @@ __global__ void __launch_bounds__(CROSS ? 512 : 256, CROSS ? (WPL > 2 ? 1 : 2) :
                 s_arm[i] = (uint32_t)l | ((uint32_t)r << 8) | ((uint32_t)rlo << 16) | ((uint32_t)rhi << 24);
             }
         }
-        {
+        // Per-pixel ranges: a run whose pixels' ranges lie in 64 disparities (32 words from kb) is walked with
+        // two disparities a lane; its other words' prefixes, counts and totals are zero.
+        bool narrow = false;
+        if constexpr (CROSS && PRIOR && WPL > 1) {
+            unsigned ul = 0xFFFFu, uh = 0;
+            for (int i = xs + lane; i < xe; i += 32) {
+                const uint32_t rg = s_rng[i];
+                const int lo = max((int)(int16_t)(rg & 0xFFFFu) - c.d0, 0), hi = min((int)(int16_t)(rg >> 16) - c.d0, c.D);
+                if (lo < hi) {
+                    ul = min(ul, (unsigned)lo);
+                    uh = max(uh, (unsigned)hi);
+                }
+            }
+            ul = __reduce_min_sync(0xFFFFFFFFu, ul);
+            uh = __reduce_max_sync(0xFFFFFFFFu, uh);
+            const int kb = min((int)(ul >> 1) & ~3, W2 - 32);  // no valid voxel: uh = 0
+            narrow = (int)uh <= 2 * kb + 64;
+            if (narrow) {
+                run_steps<false, CROSS, STORE, FULL, 1, W2, PRIOR, U8>(c, g, row, xbase, xs, xe, s_lc, s_lg, s_rc, s_rg,
+                                                                   s_t2, s_lgt, s_q, s_rng, s_pre, s_cnt, s_tot,
+                                                                   s_totc, s_em, s_key, run, kb, out_vol);
+                constexpr int zq = (W2 - 32) / 4;
+                for (int i = lane; i < (xe - xs + 1) * zq; i += 32) {
+                    const int px = i / zq, q4 = 4 * (i - px * zq);
+                    const int k4 = q4 < kb ? q4 : q4 + 32;
+                    // the row past the last pixel: the run's totals
+                    uint32_t* zp = px < xe - xs ? s_pre + (xs + px) * W2 : s_tot + run * W2;
+                    uint16_t* zc = px < xe - xs ? s_cnt + (xs + px) * W2 : s_totc + run * W2;
+                    *reinterpret_cast<uint4*>(zp + k4) = make_uint4(0, 0, 0, 0);
+                    *reinterpret_cast<uint2*>(zc + k4) = make_uint2(0, 0);
+                }
+            }
+        }
+        if (!narrow) {
             const int xa = xbase + xs, xb = xbase + xe - 1;
             const int dlo = c.d0 + P * lane;
             const bool ok = xa >= 0 && xb < c.w && P * lane + P - 1 < c.D && xa - (dlo + P - 1) >= 0 &&
                             xb - dlo <= c.w - 1;
             if (__all_sync(0xFFFFFFFFu, ok))
-                run_steps<true, CROSS, STORE, FULL, WPL, PRIOR, U8>(c, g, row, xbase, xs, xe, s_lc, s_lg, s_rc, s_rg, s_t2,
-                                                                s_lgt, s_q, s_rng, s_pre, s_cnt, s_tot, s_totc, s_em,
-                                                                s_key, run, out_vol);
+                run_steps<true, CROSS, STORE, FULL, WPL, W2, PRIOR, U8>(c, g, row, xbase, xs, xe, s_lc, s_lg, s_rc, s_rg,
+                                                                    s_t2, s_lgt, s_q, s_rng, s_pre, s_cnt, s_tot,
+                                                                    s_totc, s_em, s_key, run, 0, out_vol);
             else
-                run_steps<false, CROSS, STORE, FULL, WPL, PRIOR, U8>(c, g, row, xbase, xs, xe, s_lc, s_lg, s_rc, s_rg,
-                                                                 s_t2, s_lgt, s_q, s_rng, s_pre, s_cnt, s_tot, s_totc,
-                                                                 s_em, s_key, run, out_vol);
+                run_steps<false, CROSS, STORE, FULL, WPL, W2, PRIOR, U8>(c, g, row, xbase, xs, xe, s_lc, s_lg, s_rc, s_rg,
+                                                                     s_t2, s_lgt, s_q, s_rng, s_pre, s_cnt, s_tot,
+                                                                     s_totc, s_em, s_key, run, 0, out_vol);
         }
-        __syncthreads();
+        // most runs of the tile narrow: the output pass goes by the pixels' ranges too
+        bool sparse = false;
+        if constexpr (CROSS && PRIOR && WPL > 1) sparse = 4 * __syncthreads_count(narrow) >= 3 * nt;
+        else __syncthreads();
         {
             // the tile's keys (from the last thread down: the first ones scan the run offsets)
             const int r0 = xbase - c.d0 - (c.Dp - 1);
@@ -551,8 +590,64 @@ __global__ void __launch_bounds__(CROSS ? 512 : 256, CROSS ? (WPL > 2 ? 1 : 2) :
             // four words of one pixel, so the pixel's arms, divisor and border tests serve eight
             // disparities and its loads are independent
             constexpr int quads = W2 / 4;
-            for (int item = tid; item < g.txc * quads; item += nt) {
-                const int xi = item / quads, k4 = 4 * (item - xi * quads);
+            // In a tile of narrow ranges only a pixel's quads that meet its range are worked out; the others are
+            // filled.  Each warp takes a share of the pixels and deals their quads to its lanes.
+            const int share = (g.txc + g.nrun - 1) / g.nrun;  // at most 32 (cross_tile)
+            int items = g.txc * quads, step = nt, first = tid, px = 0, q0 = 0, upto = 0;
+            if (sparse) {
+                for (int i = tid; i < g.txc * quads; i += nt) {
+                    const int xi = i / quads, k4 = 4 * (i - xi * quads);
+                    if (x0 + xi >= c.w) break;
+                    const uint32_t rg = s_rng[xi + g.ha];
+                    const int lo = (int)(int16_t)(rg & 0xFFFFu) - c.d0, hi = (int)(int16_t)(rg >> 16) - c.d0;
+                    if (lo < hi && 2 * k4 + 8 > lo && 2 * k4 < hi) continue;
+                    if constexpr (U8)
+                        *reinterpret_cast<uint2*>(reinterpret_cast<uint8_t*>(out_vol) + ((size_t)row + x0 + xi) * (2 * W2) + 2 * k4) =
+                            make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu);
+                    else
+                        *reinterpret_cast<uint4*>(out_vol + ((size_t)row + x0 + xi) * W2 + k4) =
+                            make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
+                }
+                // this lane's pixel of the share: its first quad, and the running total of quads
+                px = run * share + lane;
+                int nq = 0;
+                if (lane < share && px < g.txc && x0 + px < c.w) {
+                    const uint32_t rg = s_rng[px + g.ha];
+                    const int lo = max((int)(int16_t)(rg & 0xFFFFu) - c.d0, 0);
+                    const int hi = min((int)(int16_t)(rg >> 16) - c.d0, 8 * quads);
+                    if (lo < hi) {
+                        q0 = lo >> 3;
+                        nq = ((hi - 1) >> 3) - q0 + 1;
+                    }
+                }
+                upto = nq;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xFFFFFFFFu, upto, o);
+                    if (lane >= o) upto += v;
+                }
+                q0 -= upto - nq;  // so that item i of the pixel is quad q0 + i
+                items = __shfl_sync(0xFFFFFFFFu, upto, 31);
+                items = (items + 31) & ~31;  // whole warps: the owners' search shuffles
+                step = 32;
+                first = lane;
+            }
+            for (int item = first; item < items; item += step) {
+                int xi, k4;
+                if (sparse) {
+                    // the owner: the first lane whose running total exceeds the item
+                    int o = 0;
+#pragma unroll
+                    for (int b = 16; b; b >>= 1)
+                        if (__shfl_sync(0xFFFFFFFFu, upto, o + b - 1) <= item) o += b;
+                    const int oq = __shfl_sync(0xFFFFFFFFu, q0, o);
+                    if (item >= __shfl_sync(0xFFFFFFFFu, upto, 31)) continue;
+                    xi = run * share + o;
+                    k4 = 4 * (oq + item);
+                } else {
+                    xi = item / quads;
+                    k4 = 4 * (item - xi * quads);
+                }
                 const int x = x0 + xi;
                 if (x >= c.w) break;
                 const uint32_t arm = s_arm[xi];
@@ -650,6 +745,8 @@ int cross_tile(const CostCtx& c, int lmax, bool full) {
     const size_t budget = smem_per_block(c.Dp > 128 ? 1 : 2);
     for (int ntx = 1; ntx <= c.w; ++ntx) {
         const int txc = round_up((c.w + ntx - 1) / ntx, 4);
+        // (with per-pixel ranges a warp's share of the output pixels is one a lane at most)
+        if (prior && txc > 32 * run_warps(true)) continue;
         if (run_geom(c, txc, lmax, true, full, prior).total <= budget) return txc;
         if (txc <= 32) break;
     }
