@@ -13,8 +13,8 @@
 //   * every pair's phases after the SGM (confidence, LR, fill, median, frame counters) on its
 //     stream again.
 // The whole sequence is captured once into a CUDA graph per batch composition (the buckets and
-// their pair counts; per bucket and pair count with byte sweeps) and replayed; inputs are copied into the slots' fixed input buffers before
-// the replay and the outputs copied out after it.  The option "unified_sgm" 0 (or 16 lanes per
+// their pair counts; per bucket and pair count with byte sweeps) and replayed; inputs are copied into
+// the slots' fixed input buffers before the replay and the outputs copied out after it.  The option "unified_sgm" 0 (or 16 lanes per
 // chain from the tuner) runs each bucket on its own stream instead, with one SGM launch per phase
 // per bucket, captured per (bucket, pair count).
 //

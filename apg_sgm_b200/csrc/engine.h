@@ -236,7 +236,7 @@ private:
     int debug_ = 0;
     int sgm_lanes_ = 0;
     int sgm_split_ = 0;  // last sweep over two warps per chain: 0 auto, 1 never, 2 always
-    int cost8_ = 0;  // Fast volume at one byte per voxel: 0 = padded range 256, 1 = never, 2 = 128 and 256
+    int cost8_ = 0;  // byte sweeps: 0 = where exact, 1 = never, 2 = as 0, byte volume allocated at Dp 128 too
     bool fast_fused_ = false;
     int cost_tile_ = 0;
     int cost_kernel_ = 0;  // 0: pixel-run cost kernel where it applies, 1: column-tile kernel

@@ -196,35 +196,37 @@ class ClockSampler:
 
 
 def _volume_bytes(cfg, tuning) -> float:
-    """Bytes per voxel of the volume the sweeps read, as the engine lays it out: one at 256 padded
-    disparities for the census-only Fast volume and for the aggregated volume of one aggregation
-    pass (tuning cost8: 0 = at 256, 1 = never, 2 = also at 128; 32 lanes per chain), else two."""
+    """Bytes per voxel of the volume the sweeps read and of each path's values, as the engine runs them:
+    one where the byte sweeps apply (the census-only Fast volume, or the aggregated volume of one
+    aggregation pass; costs below 255, as every preset's are, P2 at most 255, 256 padded disparities at
+    most; tuning cost8 other than 1, 32 lanes per chain), else two."""
     t = dict(tuning)
     Dp = (cfg.max_disparity - cfg.min_disparity + 63) // 64 * 64
     fast_census = (not cfg.agg_enable and cfg.census_type == 1 and not cfg.use_ad and not cfg.use_grad
-                   and not cfg.prior_enable and not cfg.hier_enable and not t.get("fast_fused", 0)
-                   and t.get("cost_kernel", 0) != 1)
+                   and not t.get("fast_fused", 0) and t.get("cost_kernel", 0) != 1)
     one_pass = bool(cfg.agg_enable) and cfg.agg_iterations <= 1
     if t.get("cost8", 0) == 1 or t.get("sgm_lanes", 0) not in (0, 32) or not (fast_census or one_pass):
         return 2.0
-    return 1.0 if Dp == 256 or (Dp == 128 and t.get("cost8", 0) == 2) else 2.0
+    return 1.0 if Dp <= 256 else 2.0
 
 
 def _algorithmic_bytes(name: str, w: int, h: int, D: int, volume_source: bool, npath: int = 4,
                        vb: float = 2.0) -> float:
-    """Bytes a launch of `name` must move by design: the stage-boundary traffic of the kernel with
-    u16 path sums and vb bytes per voxel of the volume the sweeps read (see _volume_bytes); a
-    volume-fed sweep reads that volume once."""
+    """Bytes a launch of `name` must move by design: the stage-boundary traffic of the kernel with vb
+    bytes per voxel of the volume the sweeps read (see _volume_bytes).  16-bit sweeps (vb 2) read the
+    volume once a direction and keep path sums; byte sweeps read it once a direction, write one byte a
+    voxel and direction, and the last one reads all of them."""
     n = w * h
     vol = n * D * vb if volume_source else 0.0
     nfirst = npath - 1
-    nin = 3  # Path8: five first-phase buffers folded into one before the last sweep
+    byte = vb == 1.0
+    nin = nfirst if byte else 3  # 16-bit, Path8: five first-phase buffers folded into one before the last sweep
     return {
-        "sgm_first": nfirst * (n * D * 2.0 + vol),    # every first-phase sweep writes its own sums
-        "sgm_fold5": n * D * 12.0,                    # Path8: read 5 buffers, write 1
-        "sgm_last_wta": nin * n * D * 2.0 + vol + n * 12,  # read the partial sums, write the WTA maps
-        "cost+crossH": n * D * 2.0,                   # write the horizontally aggregated volume
-        "crossV": n * D * (2.0 + vb),                 # read T, write C
+        "sgm_first": nfirst * (n * D * vb + vol),     # every first-phase sweep writes its own values
+        "sgm_fold5": n * D * 12.0,                    # 16-bit Path8: read 5 buffers, write 1
+        "sgm_last_wta": nin * n * D * vb + vol + n * 12,  # read the others' values, write the WTA maps
+        "cost+crossH": n * D * vb,                    # write the horizontally aggregated volume
+        "crossV": n * D * 2.0 * vb,                   # read T, write C
         "cost": n * D * vb,                           # write the raw volume
     }.get(name, 0.0)
 
@@ -731,8 +733,8 @@ def run_b200(args, wl):
                  (statistics.mean(per_kernel[k]) / 1000.0) / 1e9 / peak, 4)
         for k in ("sgm_first", "sgm_fold5", "sgm_last_wta", "crossV") if k in per_kernel}
     if top in ("cost", "cost+crossH"):
-        roofline["note"] = ("issue-bound: integer and LUT work per voxel (ncu issue active ~73%, DRAM ~8%); "
-                            "the HBM fraction of its 2 B/voxel output is shown for reference")
+        roofline["note"] = ("issue-bound: integer and LUT work per voxel (ncu issue active ~68%, DRAM ~4%); "
+                            "the HBM fraction of its output is shown for reference")
     if "refine" in per_kernel:
         # the refiner: passes x a wavefront over the frame; a pixel's update needs its left and up
         # neighbours' values of the same pass, so a pass takes at least w + h - 1 dependent steps.

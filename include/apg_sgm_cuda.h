@@ -62,16 +62,18 @@ APGCU_API int apgcu_engine_set_debug(apgcu_engine_t e, int flags);
 
 /* Kernel tuning knobs (results never change, only speed):
  *   "sgm_lanes": lanes per SGM scanline chain, 8 / 16 / 32 (0 = default, 32);
- *   "sgm_split": the volume-fed last sweep with its recurrence and its sums / WTA on two warps per
- *                chain: 0 = for 64 padded disparities (default), 1 = never, 2 = always;
+ *   "sgm_split": the 16-bit volume-fed last sweep with its recurrence and its sums / WTA on two warps
+ *                per chain: 0 = for 64 padded disparities (default), 1 = never, 2 = always;
  *   "cost_tile": columns per block of the cost kernel, 64 / 128 / 256 (0 = default for the range);
  *   "fast_fused": 1 = census-only Fast mode recomputes its costs inside the SGM sweeps and stores no
  *                 cost volume (less memory, slower); 0 = store the volume once (default);
  *   "cost_kernel": 0 = pixel-run cost kernel where it applies (default), 1 = column-tile kernel;
  *   "cost8": the volume the SGM sweeps read (the census-only Fast volume, or the aggregated
- *            volume of one aggregation pass) at one byte per voxel (0xFF invalid; exact while
- *            every quantised cost is below 255): 0 = at 256 padded disparities (default),
- *            1 = never, 2 = at 128 and 256;
+ *            volume of one aggregation pass) and their path values (as distances above the costs) at
+ *            one byte per voxel, exact while every quantised cost is below 255, P2 at most 255 and
+ *            the padded range at most 256: 0 = wherever that holds (default), 1 = never (16-bit
+ *            sweeps), 2 = as 0, and the volume is allocated at one byte per voxel at 128 padded
+ *            disparities too (0 does so at 256 only);
  *   "refine_window": 0 = HighQuality refiner reads the right-image window from shared memory where
  *                 every band fits on the device at once (default), 1 = always through L1;
  *   "host_bands": frames whose outputs go to host memory (apgcu_engine_process, the session) run
