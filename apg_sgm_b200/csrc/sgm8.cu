@@ -903,17 +903,27 @@ cudaError_t by_dp(int Dp, F f) {
     }
 }
 
-// Blocks of `bytes` shared memory the device holds at once.
-int blocks_at_once(size_t bytes) {
+// The device's SMs, the shared memory of one and what each block reserves of it (bytes).
+struct SmShare {
+    int count;
+    size_t smem, reserved;
+};
+SmShare sm_share() {
     int dev = 0, nsm = 0, per_sm = 0, reserved = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess) {
         cudaGetLastError();
-        return 0;
+        return SmShare{148, 228 * 1024, 1024};
     }
-    return nsm * (int)(per_sm / (bytes + reserved));
+    return SmShare{nsm, (size_t)per_sm, (size_t)reserved};
+}
+
+// Blocks of `bytes` shared memory the device holds at once.
+int blocks_at_once(size_t bytes) {
+    const SmShare sm = sm_share();
+    return sm.count * (int)(sm.smem / (bytes + sm.reserved));
 }
 
 template <int DP, int NIN, bool PS, bool BAND>
@@ -930,7 +940,9 @@ cudaError_t launch_last_t(const Args8& a, const In8& in, int dx, int dy, int nsc
         kern<<<blocks, 64, smem, st>>>(a, in, dx, dy, nscan);
         return cudaGetLastError();
     }
-    constexpr int KG = DP == 256 ? (NIN == 3 ? 2 : 1) : (NIN == 3 ? 4 : 2), NG = 3;
+    // steps per group: four keep a group's loads long, two where four leave too few blocks on an SM (Fast
+    // 1920x1080, four / two, us: D128 260 / 295, D192 519 / 449; D256 two / one 438 / 512)
+    constexpr int KG = DP == 256 ? (NIN == 3 ? 2 : 1) : DP == 192 ? 2 : (NIN == 3 ? 4 : 2), NG = 3;
     auto kern = sgm8_last_kernel<DP, NIN, KG, NG, PS, BAND>;
     const size_t smem = last_bytes<DP, NIN, KG, NG>();
     const cudaError_t e = allow_dynamic_smem(kern, smem);
@@ -980,7 +992,19 @@ cudaError_t launch_sgm8_first(const SgmLaunch& l, int ndir, const int (*dirs)[2]
     }
     return by_dp(l.Dp, [&](auto dp) -> cudaError_t {
         constexpr int DP = decltype(dp)::value;
-        sgm8_first_kernel<DP><<<tab.warp_begin[ndir], 32, first_bytes<DP>(), st>>>(a, tab);
+        // Frames of many more chains than an SM's four schedulers can step at full rate: eight blocks at a time
+        // on each SM, the rest in their turn as chains end, so that fewer rows are open in DRAM and the last
+        // chains share an SM with fewer others.  Eight a SM against all that fit, us: 1920x1080 D128 285 / 313,
+        // D256 538 / 612, HighQuality D256 1237 / 1282, 2560x1440 D256 1003 / 1028; with fewer chains it loses
+        // (1280x720 D128 155 / 147, 1280x1024 D256 381 / 371), as with eight paths below 256 (1280x720 D128
+        // 367 / 362).
+        const int blocks = tab.warp_begin[ndir];
+        size_t smem = first_bytes<DP>();
+        const SmShare sm = sm_share();
+        if (blocks >= 12 * sm.count && (ndir <= 3 || DP == 256)) smem = std::max(smem, (sm.smem / 8 - sm.reserved) & ~size_t(15));
+        const cudaError_t e = allow_dynamic_smem(sgm8_first_kernel<DP>, smem);
+        if (e != cudaSuccess) return e;
+        sgm8_first_kernel<DP><<<blocks, 32, smem, st>>>(a, tab);
         return cudaGetLastError();
     });
 }

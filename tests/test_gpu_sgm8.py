@@ -36,6 +36,11 @@ CASES = [
     (1, 140, 70, 128, 0, {"P1": 60, "P2_base": 200}),
     (1, 140, 70, 192, 0, {"P1": 100, "P2_base": 255, "paths": 8}),
     (1, 120, 60, 64, 0, {"P1": 0, "P2_base": 1, "adaptive_penalties": 0}),
+    # more chains than the first sweep keeps on the device at once; last sweeps on one warp per pair
+    (0, 700, 1500, 130, 0, {}),
+    (0, 320, 800, 200, 0, {"paths": 8}),
+    (0, 1930, 60, 150, 0, {}),
+    (0, 1930, 45, 250, 0, {}),
 ]
 
 
