@@ -1106,7 +1106,13 @@ int Engine::host_band_count(bool device) const {
     // the chains' state between bands lives in the refiner's map, unused without the refiner
     const size_t carry = L.bytes ? sgm8_carry_words(L.w, L.Dp) : (size_t)L.w * 32 * (L.Dp / 64 + 1);
     if (carry > (size_t)L.w * L.h) return 0;
-    return req > 1 ? std::min(req, (int)kMaxBands) : (int)kBands;
+    if (req > 1) return std::min(req, (int)kMaxBands);
+    // a band for every 300,000 pixels, four at most: a band's launches cost about 9 us, and the copies it hides
+    // are 10 bytes a pixel.  Page-locked buffers, one sweep / best / six bands, us: 432x297 294 / 294 / 345,
+    // 640x480 D128 422 / 414 (two) / 442, 1280x720 D128 675 / 640 (three) / 658, 1920x1080 D256 1794 / 1620
+    // (four) / 1636
+    const int nb = (int)std::min<size_t>(4, ((size_t)L.w * L.h + 150000) / 300000);
+    return nb > 1 ? nb : 0;
 }
 
 int Engine::run_banded(int nb, float* hdisp, float* hconf, uint8_t* hreason, uint8_t* hrel, bool to_host) {

@@ -172,11 +172,10 @@ public:
     void set_refine_spin_limit(int n) { refine_.spin_limit = n; }
     void set_refine_window(int mode) { refine_.window = mode; }
     // the last sweep in this many row bands, each band's rows post-processed and copied to the
-    // outputs while the next band runs (0: kBands where the path allows it, 1: never)
+    // outputs while the next band runs (0: by the frame's pixels where the path allows it, 1: never)
     void set_host_bands(int n) { host_bands_ = n; }
     // device-output frames (process_device) in that many bands: 0 = never (default)
     void set_device_bands(int n) { device_bands_ = n; }
-    static constexpr int kBands = 6;
     static constexpr int kMaxBands = 16;
     // takes the calling thread's experimental scopes now (run_pre does so for every frame; the
     // batched form needs them before it builds SGM plans from sgm_launch)
