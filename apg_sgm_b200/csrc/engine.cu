@@ -791,7 +791,7 @@ int Engine::run_pre(const uint8_t* dl, int lstride, const uint8_t* dr, int rstri
     // after the refiner, the stage dumps); it runs in line: beside the sweeps' one-warp blocks, whose chains
     // are all resident at once, another stream's blocks decide how many chains each SM steps (Fast 1280x720
     // D128 0.520 ms per frame with it on a side stream, 0.490 in line)
-    right_written_ = refine_enabled() || debug_;
+    right_written_ = refine_enabled() || (debug_ & ~8);  // (the launch profile alone changes no work)
     if (right_written_)
         RUN(launch_right_wta_finalize(cc, ptr<uint32_t>(L.rkey), cfg_.subpixel, ptr<float>(L.disp_right), s), "right wta");
     cudaEventRecord(ev_[4], s);
