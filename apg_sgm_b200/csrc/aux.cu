@@ -34,19 +34,30 @@ __global__ void __launch_bounds__(TX * BY) aux_kernel(AuxImage im0, AuxImage im1
     __shared__ __align__(16) uint8_t g[SY][SX];  // rows of SX bytes, a multiple of 4
     const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
     const int tid = threadIdx.y * TX + threadIdx.x;
-    for (int i = tid; i < SX * SY; i += TX * BY) {
-        const int sy = i / SX, sx = i % SX;
-        const int yy = min(max(y0 + sy - HY, 0), h - 1);
-        const int xx = min(max(x0 + sx - HX, 0), w - 1);
-        const uint8_t* row = src + (size_t)yy * stride;
-        uint8_t v;
-        if (ch == 1) {
-            v = row[xx];
-        } else {
-            const int r = row[xx * ch], gg = row[xx * ch + 1], b = row[xx * ch + 2];
-            v = (uint8_t)((77 * r + 150 * gg + 29 * b) >> 8);
+    // interior tiles of aligned single-channel images by words (a tile's halo starts 4 columns left of a multiple
+    // of 32): a quarter of the loads and index divisions, 27.2 -> 25.4 us a 1280x720 pair, 1% of a Fast frame
+    if (ch == 1 && x0 >= HX && x0 + TX + HX <= w && ((reinterpret_cast<uintptr_t>(src) | (uintptr_t)stride) & 3) == 0) {
+        for (int i = tid; i < SX / 4 * SY; i += TX * BY) {
+            const int sy = i / (SX / 4), q = i - sy * (SX / 4);
+            const int yy = min(max(y0 + sy - HY, 0), h - 1);
+            reinterpret_cast<uint32_t*>(g[sy])[q] =
+                *reinterpret_cast<const uint32_t*>(src + (size_t)yy * stride + x0 - HX + 4 * q);
         }
-        g[sy][sx] = v;
+    } else {
+        for (int i = tid; i < SX * SY; i += TX * BY) {
+            const int sy = i / SX, sx = i % SX;
+            const int yy = min(max(y0 + sy - HY, 0), h - 1);
+            const int xx = min(max(x0 + sx - HX, 0), w - 1);
+            const uint8_t* row = src + (size_t)yy * stride;
+            uint8_t v;
+            if (ch == 1) {
+                v = row[xx];
+            } else {
+                const int r = row[xx * ch], gg = row[xx * ch + 1], b = row[xx * ch + 2];
+                v = (uint8_t)((77 * r + 150 * gg + 29 * b) >> 8);
+            }
+            g[sy][sx] = v;
+        }
     }
     __syncthreads();
     const int x = x0 + threadIdx.x;
