@@ -34,6 +34,7 @@
 #include "sgm8.cuh"
 
 #include <algorithm>
+#include <cstddef>
 #include <cstring>
 #include <vector>
 
@@ -56,7 +57,7 @@ struct Args8 {
     int w, h, d0, D, dmax;
     int def_ranges;  // every pixel has the default range
     int P1;
-    uint8_t p2[256];  // adaptive P2 by |gray difference|
+    alignas(16) uint8_t p2[256];  // adaptive P2 by |gray difference|
     const uint8_t* gray;
     const uint8_t* vol;
     WtaOut wta;
@@ -64,6 +65,7 @@ struct Args8 {
     int t_begin, t_end;
     uint32_t* carry;
 };
+static_assert(offsetof(Args8, p2) % 8 == 0, "gray_init copies the table eight bytes a lane");
 struct Dirs8 {
     int n;
     int dx[kMaxIn], dy[kMaxIn], nscan[kMaxIn];
