@@ -229,7 +229,7 @@ __device__ __forceinline__ Pair pair_start(const Args8& a, int dx, int dy, int s
     int y;
     scan_start8(a.w, a.h, dx, dy, s, nscan, q.xA, y, q.lenA);
     q.pA = y * a.w + q.xA;
-    // an odd last scanline runs as both halves of its warp (the same values, stored twice)
+    // an odd last scanline runs as both halves of its warp (the same values, stored twice; pB == pA)
     scan_start8(a.w, a.h, dx, dy, s + 1 < nscan ? s + 1 : s, nscan, q.xB, y, q.lenB);
     q.pB = y * a.w + q.xB;
     q.step = dy * a.w + dx;
@@ -538,12 +538,13 @@ __device__ __forceinline__ void put_sums(const Args8& a, const Pair& q, uint32_t
     }
 }
 
-// The WTA of the block of 16 steps at tb: lane l takes step tb + l % 16 of scanline A (l < 16) or B.
+// The WTA of the block of 16 steps at tb: lane l takes step tb + l % 16 of scanline A (l < 16) or B (none
+// where B repeats A, an odd last scanline: the sub-pixel telemetry counts a pixel once).
 template <int DP, int NIN>
 __device__ __forceinline__ void wta_block(const Args8& a, const Pair& q, uint32_t* s_wta, int tb, int lane) {
     const int t = tb + (lane & 15);
     const bool b = lane >= 16;
-    if (t < (b ? q.lenB : q.lenA))
+    if (t < (b ? q.lenB : q.lenA) && !(b && q.pB == q.pA))
         wta_row<DP / 2, sum_inf<NIN>(), sum_bias<NIN>()>(a.wta, a.d0, a.D, s_wta + lane * Geo<DP>::RS,
                                                          (b ? q.pB : q.pA) + t * q.step);
 }
