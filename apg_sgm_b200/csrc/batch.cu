@@ -137,6 +137,7 @@ private:
     int ensure_slots(Bucket& b, int m);
     int ensure_plan(Bucket& b, int m);
     bool byte_sweeps(const Bucket& b) const;
+    void apply_tune(const Bucket& b, Engine& e) const;
     int enqueue(Bucket& b, int m, bool batched_sgm);
     int run_bucket(Bucket& b, int m, bool batched_sgm);
     int autotune(Bucket& b, const apgcu_pair_t& sample, bool device_buffers);
@@ -200,8 +201,7 @@ int Batch::ensure_slots(Bucket& b, int m) {
         } catch (...) {
             return fail(kAllocationFailure, "engine creation failed");
         }
-        e->set_sgm_lanes(b.tune.sgm_lanes);
-        e->set_cost_tile(b.tune.cost_tile);
+        apply_tune(b, *e);
         b.slots.push_back(std::move(e));
         cudaEvent_t ev;
         if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) {
@@ -229,6 +229,14 @@ void drop_plans(Bucket& b) {
 bool Batch::byte_sweeps(const Bucket& b) const {
     return forced_lanes_ != 16 &&
            Engine::make_layout(b.cfg, b.key.w, b.key.h, b.key.ch, 0).bytes;
+}
+
+// The bucket's tuning on one of its slots.  A slot off the byte sweeps keeps two-byte volumes, which the
+// persistent launch reads, whatever number of lanes the tuner tries on it.
+void Batch::apply_tune(const Bucket& b, Engine& e) const {
+    e.set_sgm_lanes(b.tune.sgm_lanes);
+    e.set_cost_tile(b.tune.cost_tile);
+    e.set_cost8(byte_sweeps(b) ? 0 : 1);
 }
 
 int Batch::ensure_plan(Bucket& b, int m) {
@@ -477,6 +485,8 @@ int Batch::autotune(Bucket& b, const apgcu_pair_t& sample, bool device_buffers) 
     int rc = ensure_slots(b, 1);
     if (rc) return rc;
     Engine& e = *b.slots[0];
+    b.tune = cand[0];
+    apply_tune(b, e);  // the slot may have run under other options: its form is decided by the upload
     rc = e.upload(sample.left, sample.right, sample.width, sample.height, sample.stride, sample.channels,
                   device_buffers, b.stream);
     if (rc) return fail(rc, e.last_error());
@@ -487,8 +497,7 @@ int Batch::autotune(Bucket& b, const apgcu_pair_t& sample, bool device_buffers) 
     Tuning best = cand[0];
     for (const Tuning& t : cand) {
         b.tune = t;
-        e.set_sgm_lanes(t.sgm_lanes);
-        e.set_cost_tile(t.cost_tile);
+        apply_tune(b, e);
         drop_plans(b);
         rc = bytes ? kOk : ensure_plan(b, 1);
         if (rc) break;
@@ -519,10 +528,7 @@ int Batch::autotune(Bucket& b, const apgcu_pair_t& sample, bool device_buffers) 
     if (rc) return rc;
     b.tune = best;
     b.tuned = true;
-    for (auto& s : b.slots) {
-        s->set_sgm_lanes(best.sgm_lanes);
-        s->set_cost_tile(best.cost_tile);
-    }
+    for (auto& s : b.slots) apply_tune(b, *s);
     drop_plans(b);
     std::lock_guard<std::mutex> lk(g_tune_mu);
     tune_store_locked(key, best);
@@ -570,10 +576,7 @@ int Batch::process(int n, const apgcu_pair_t* pairs, bool device_buffers) {
         if (forced_lanes_) b.tune.sgm_lanes = forced_lanes_;
         if (forced_max_blocks_ >= 0) b.tune.max_blocks_per_sm = forced_max_blocks_;
         if (forced_tile_ >= 0) b.tune.cost_tile = forced_tile_;
-        for (auto& sl : b.slots) {
-            sl->set_sgm_lanes(b.tune.sgm_lanes);
-            sl->set_cost_tile(b.tune.cost_tile);
-        }
+        for (auto& sl : b.slots) apply_tune(b, *sl);
         drop_plans(b);
         drop_unified();  // graphs of compositions with this bucket hold its old tuning
     }
