@@ -14,6 +14,10 @@
 // Every wait is bounded: on timeout the band sets an error flag (read by the host) and stops.  This is
 // exactly the reference's read-after-write order.
 //
+// A band keeps the row above whole in shared memory (5 bytes a column), so frames whose bands do not all
+// fit on the device at once that way take a pass in several runs of columns, one launch after another: every
+// row of a run comes before the next run's first column, whose left neighbours are then read from the map.
+//
 // Measured (one B200, all three passes of HighQuality with their per-pixel kernels): 1920x1080 D256
 // 1.97 ms, 1280x720 D128 1.27 ms, where steps with divergent branches, per-step hand-overs by polling
 // and per-lane copies took 5.61 and 3.70 ms; a step costs about 300 cycles.
@@ -230,6 +234,9 @@ __device__ __forceinline__ float cand_cost(const CostCtx& c, const float* lut, c
     return 1e6f;
 }
 
+// A value as a neighbour candidate: rounded when it is non-negative, else none (-1).
+__device__ __forceinline__ int neighbour(float v) { return v >= 0.f ? (int)roundf(v) : -1; }
+
 // Wavefront order: the records and right-image pixels of a band's step lie together, lane
 // by lane ([band][step][lane]), so a chunk of steps is one contiguous bulk copy each.  The right pixels
 // start wave_lead(D) steps before the first step: the window of the first columns.
@@ -242,11 +249,17 @@ constexpr uint32_t kOutside = 0xFF000000u;
 constexpr uint32_t kGradWeights = 0x03010100u;  // index = |dgx| + |dgy| + 3 * byte 3
 constexpr int kGradIn = 511, kGradAll = 3 * 255 + kGradIn;
 
-// One pixel record per (band, step, lane), neutral where the lane has no pixel at that step, and the
-// right-image pixel that enters its window at that step (column u of a row brings image column
-// x(u) - eoff).
+// A run of a pass's columns: cols of them from column begin, in pass order.
+struct ColRun {
+    int begin, cols;
+};
+
+// One pixel record per (band, step, lane), neutral where the lane has no pixel of the run at that step, and
+// the right-image pixel that enters its window at that step (column u of a row brings image column
+// x(u) - eoff).  Columns u count from the run's first; the neutral record of column -1 hands the lane the
+// candidate that the run before left there.
 template <bool C64, bool WIN>
-__global__ void __launch_bounds__(256) refine_prep_kernel(CostCtx c, int fwd, const uint8_t* __restrict__ reliable,
+__global__ void __launch_bounds__(256) refine_prep_kernel(CostCtx c, int fwd, ColRun run, const uint8_t* __restrict__ reliable,
                                    const int* __restrict__ prefix, const int16_t* __restrict__ draw_value,
                                    const unsigned* __restrict__ rej, int nrej, const unsigned* __restrict__ P_ptr,
                                    const RPack<C64>* __restrict__ lp, const RPack<C64>* __restrict__ rp,
@@ -257,14 +270,14 @@ __global__ void __launch_bounds__(256) refine_prep_kernel(CostCtx c, int fwd, co
     __syncthreads();
     const int w = c.w, h = c.h, n = w * h;
     const unsigned P = *P_ptr;
-    const int lead = WIN ? wave_lead(c.D) : 0, nstep = wave_chunks(w) * kChunk, tt = lead + nstep;
+    const int lead = WIN ? wave_lead(c.D) : 0, nstep = wave_chunks(run.cols) * kChunk, tt = lead + nstep;
     const int nbands = (h + kBand - 1) / kBand;
     const int eoff = fwd ? c.d0 : c.d0 + c.D - 1;
     const int lane = threadIdx.x & 31, per = blockDim.x >> 5;
     for (int j = blockIdx.x * per + (threadIdx.x >> 5); j < nbands * tt; j += gridDim.x * per) {
         const int band = j / tt, t = j - band * tt - lead;
         const int v = band * kBand + lane, u = t - lane;
-        const int x = fwd ? u : w - 1 - u;
+        const int x = fwd ? run.begin + u : w - 1 - run.begin - u;
         const int y = fwd ? v : h - 1 - v;
         if constexpr (WIN) {
             const int pe = x - eoff;
@@ -278,7 +291,8 @@ __global__ void __launch_bounds__(256) refine_prep_kernel(CostCtx c, int fwd, co
         st.c_cur = __int_as_float(0xff800000);
         st.c_draw = 1e9f;
         st.d_cur = -1;
-        if (v < h && (unsigned)u < (unsigned)w) {
+        if (v < h && u == -1 && run.begin > 0) st.d_cur = neighbour(work[y * w + x]);
+        if (v < h && (unsigned)u < (unsigned)run.cols) {
             const int i = y * w + x;
             const float cur = work[i];
             const int lo = c.rmin[i], hi = c.rmax[i];
@@ -286,7 +300,7 @@ __global__ void __launch_bounds__(256) refine_prep_kernel(CostCtx c, int fwd, co
             st.lo = lo;
             st.hi1 = hi - 1;
             if (reliable[i] || hi <= lo) {
-                if (cur >= 0.f) st.d_cur = (int)roundf(cur);
+                st.d_cur = neighbour(cur);
             } else if (cur >= 0.f) {
                 st.d_cur = min(max((int)roundf(cur), lo), hi - 1);
                 st.c_cur = cand_cost<C64>(c, s_lut, st.left, rp, x, y, st.d_cur, lo, hi);
@@ -392,14 +406,15 @@ __device__ __forceinline__ void cluster_sync() {
 // The link warp of a band that receives from (recv) or publishes to (send) another cluster.  Every wait
 // is bounded: after spin_limit polls in which nothing moved it sets the error word and `abort`, and after
 // as many again it leaves.
-__device__ void band_link(BandLink* s_link, int* s_up, uint64_t* upbar, int band, int w, int h, int fwd,
-                          const float* work, int* progress, int* err, int spin_limit, bool recv, bool send) {
+__device__ void band_link(BandLink* s_link, int* s_up, uint64_t* upbar, int band, int width, int h, ColRun run,
+                          int fwd, const float* work, int* progress, int* err, int spin_limit, bool recv, bool send) {
     const int lane = threadIdx.x & 31;
     volatile BandLink* L = s_link;
     volatile int* vprog = progress;
-    const int xs = fwd ? 1 : -1, xb = fwd ? 0 : w - 1;
+    const int w = run.cols;
+    const int xs = fwd ? 1 : -1, xb = fwd ? run.begin : width - 1 - run.begin;
     const int y_above = recv ? (fwd ? band * kBand - 1 : h - band * kBand) : 0;
-    const float* above = work + (size_t)y_above * w;
+    const float* above = work + (size_t)y_above * width;
     int fetched = recv ? 0 : w;      // columns of the row above copied
     int blocks = 0;                  // barriers arrived on
     int published = send ? 0 : w;
@@ -427,8 +442,7 @@ __device__ void band_link(BandLink* s_link, int* s_up, uint64_t* upbar, int band
                 if (lane == 0) fence_acq_rel();
                 __syncwarp();
                 for (int col = fetched + lane; col < prog; col += 32) {
-                    const float a = __ldcg(above + (xb + xs * col));
-                    s_up[col + kUpShift] = a >= 0.f ? (int)roundf(a) : -1;
+                    s_up[col + kUpShift] = neighbour(__ldcg(above + (xb + xs * col)));
                 }
                 __syncwarp();
                 fetched = prog;
@@ -476,17 +490,17 @@ struct BandRing {
 // instead: every lane misses L1 at a different step and the compute warp waits for the slowest, so the
 // window's first kAhead steps are prefetched first and its entering edge kAhead steps ahead of the copies.
 template <bool C64, bool WIN>
-__device__ void band_loader(const CostCtx& c, int band, int fwd, BandRing<C64>* ring, RPack<C64>* s_win, int wmask,
+__device__ void band_loader(const CostCtx& c, int band, ColRun run, int fwd, BandRing<C64>* ring, RPack<C64>* s_win, int wmask,
                             const RStep<C64>* steps, const RPack<C64>* wr, const RPack<C64>* rp, int spin_limit) {
     const int w = c.w, lane = threadIdx.x & 31;
-    const int nchunks = wave_chunks(w), nstep = nchunks * kChunk;
+    const int nchunks = wave_chunks(run.cols), nstep = nchunks * kChunk;
     const int lead = WIN ? wave_lead(c.D) : 0;
     const RStep<C64>* gs = steps + (size_t)band * nstep * 32;
     const RPack<C64>* gr = wr + ((size_t)band * (lead + nstep) + lead) * 32;
     constexpr int kSlots = BandRing<C64>::kSlots;
     constexpr unsigned bs = kChunk * 32 * sizeof(RStep<C64>), bp = kChunk * 32 * sizeof(RPack<C64>);
     const int v = band * kBand + lane, y = fwd ? v : c.h - 1 - v;
-    const int xs = fwd ? 1 : -1, xb = fwd ? 0 : w - 1, eoff = fwd ? c.d0 : c.d0 + c.D - 1;
+    const int xs = fwd ? 1 : -1, xb = fwd ? run.begin : w - 1 - run.begin, eoff = fwd ? c.d0 : c.d0 + c.D - 1;
     const RPack<C64>* rrow = rp + (size_t)(v < c.h ? y : 0) * w;
     if (!WIN)
         for (int k = -c.D; k <= kAhead; k += 8) prefetch_l1(rrow + min(max(xb + xs * k - eoff, 0), w - 1));
@@ -547,7 +561,7 @@ __device__ __forceinline__ float step_cost(const float* lut, const RPack<C64>& l
 // records come by bulk copies that use no issue slot or load path of the SM, and a band hands its last
 // row to the next one through the cluster's shared memory.
 template <bool C64, bool WIN, bool FWD>
-__global__ void __launch_bounds__(96) refine_band_kernel(CostCtx c, int nbands, int csize,
+__global__ void __launch_bounds__(96) refine_band_kernel(CostCtx c, int nbands, int csize, ColRun run,
                                                          const RStep<C64>* __restrict__ steps,
                                                          const RPack<C64>* __restrict__ wr,
                                                          const RPack<C64>* __restrict__ rp, float* work,
@@ -558,7 +572,7 @@ __global__ void __launch_bounds__(96) refine_band_kernel(CostCtx c, int nbands, 
     __shared__ __align__(128) BandRing<C64> s_ring;
     __shared__ BandLink s_link;
     extern __shared__ __align__(128) unsigned char s_dyn[];
-    const int w = c.w;
+    const int w = run.cols;  // columns of the run: everything below but addresses counts in them
     const int ublk = up_blocks(w);
     RPack<C64>* s_win = reinterpret_cast<RPack<C64>*>(s_dyn);
     int* s_up = reinterpret_cast<int*>(s_dyn + (WIN ? (size_t)(wmask + 1) * 32 * sizeof(RPack<C64>) : 0));
@@ -591,15 +605,15 @@ __global__ void __launch_bounds__(96) refine_band_kernel(CostCtx c, int nbands, 
     const int lane = threadIdx.x & 31;
     if (live && warp == 1) {
         if (from_link || to_link)
-            band_link(&s_link, s_up, s_upbar, band, w, c.h, fwd, work, progress, err, spin_limit, from_link, to_link);
+            band_link(&s_link, s_up, s_upbar, band, c.w, c.h, run, fwd, work, progress, err, spin_limit, from_link, to_link);
     } else if (live && warp == 2) {
-        band_loader<C64, WIN>(c, band, fwd, &s_ring, s_win, wmask, steps, wr, rp, spin_limit);
+        band_loader<C64, WIN>(c, band, run, fwd, &s_ring, s_win, wmask, steps, wr, rp, spin_limit);
     } else if (live) {
         volatile BandLink* link = &s_link;
         const int v = band * kBand + lane;
         const int yrow = fwd ? v : c.h - 1 - v;
-        const int xs = fwd ? 1 : -1, xb = fwd ? 0 : w - 1;
-        const size_t rowoff = (size_t)(v < c.h ? yrow : 0) * w;
+        const int xs = fwd ? 1 : -1, xb = fwd ? run.begin : c.w - 1 - run.begin;
+        const size_t rowoff = (size_t)(v < c.h ? yrow : 0) * c.w;
         float* wrow = work + rowoff;
         const RPack<C64>* rrow = rp + rowoff;
         const unsigned peer_up = to_peer ? peer_smem(smem_u32(s_up), rank + 1) : 0u;
@@ -609,7 +623,9 @@ __global__ void __launch_bounds__(96) refine_band_kernel(CostCtx c, int nbands, 
         const int back_0 = fwd ? -c.d0 : c.d0 + c.D - 1;
         // Neighbour values travel as candidates: roundf(value) when value >= 0, else -1 (the
         // reference takes a neighbour only when it is non-negative, rounded), or any negative value.
-        int prev = -1;  // candidate of this lane's previous column (its left neighbour)
+        // candidate of this lane's previous column (its left neighbour); the neutral records before a lane's
+        // first column set it again
+        int prev = run.begin > 0 && v < c.h ? neighbour(wrow[xb - xs]) : -1;
         bool abort = false;
         const int nchunks = wave_chunks(w);
         int upc = band > 0 ? 0 : ublk;  // barriers of the row above known to be complete
@@ -656,7 +672,7 @@ __global__ void __launch_bounds__(96) refine_band_kernel(CostCtx c, int nbands, 
                     pu = *reinterpret_cast<const RPack<C64>*>(win + ((FWD ? base - du * B : base + du * B) & m));
                 } else {
                     const int xl = x0 + xs * i - dl, xu = x0 + xs * i - du;
-                    const bool in_l = (unsigned)xl < (unsigned)w, in_u = (unsigned)xu < (unsigned)w;
+                    const bool in_l = (unsigned)xl < (unsigned)c.w, in_u = (unsigned)xu < (unsigned)c.w;
                     pl = rrow[in_l ? xl : 0];
                     pu = rrow[in_u ? xu : 0];
                     pl.g = in_l ? pl.g : kOutside;
@@ -853,10 +869,16 @@ size_t refine_steps_bytes(int w, int h, int D, bool c64) {
 
 namespace {
 
+// How a pass runs: in clusters of `csize` bands, `cols` columns a launch, `smem` bytes and a window ring of
+// wmask + 1 steps a block (csize 0: not at all).
+struct PassPlan {
+    int csize, cols, wmask;
+    size_t smem;
+};
+
 template <bool C64, bool WIN>
 cudaError_t launch_pass_t(const CostCtx& c, const Layout& L, unsigned char* arena, const RefineTables& tab, int it,
-                          float* work, int spin_limit, int wmask, size_t smem, int csize, cudaStream_t s,
-                          unsigned* launches) {
+                          float* work, int spin_limit, const PassPlan& plan, cudaStream_t s, unsigned* launches) {
     const int fwd = (it % 2) == 0;
     const int n = L.w * L.h;
     const int nbands = refine_band_count(L.h);
@@ -867,35 +889,40 @@ cudaError_t launch_pass_t(const CostCtx& c, const Layout& L, unsigned char* aren
     int* progress = reinterpret_cast<int*>(arena + L.rf_state) + kRefineProgWord;
     const RPack<C64>* lpk = reinterpret_cast<const RPack<C64>*>(arena + L.rf_pack);
     const RPack<C64>* rpk = lpk + n;
-    const size_t ns = (size_t)nbands * wave_chunks(L.w) * kChunk * 32;
     RStep<C64>* steps = reinterpret_cast<RStep<C64>*>(arena + L.rf_steps);
-    RPack<C64>* wr = reinterpret_cast<RPack<C64>*>(steps + ns);
-    const size_t items = ns / 32 + (WIN ? (size_t)nbands * wave_lead(c.D) : 0);
-    const int blocks = (int)std::min<size_t>((items + 7) / 8, 148 * 8);
-    refine_prep_kernel<C64, WIN><<<blocks, 256, 0, s>>>(c, fwd, rel, prefix, tab.value[it], tab.rejected[it],
-                                                        tab.nrej[it], P + it, lpk, rpk, work, steps, wr);
-    ++*launches;
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    // every band at once (a band waits for the one above): a cooperative launch in clusters of csize
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((nbands + csize - 1) / csize * csize);
-    cfg.blockDim = dim3(3 * kBand);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = csize;
-    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 2;
-    e = cudaLaunchKernelEx(&cfg, fwd ? refine_band_kernel<C64, WIN, true> : refine_band_kernel<C64, WIN, false>, c, nbands,
-                           csize, (const RStep<C64>*)steps, (const RPack<C64>*)wr, rpk, work, progress, err, spin_limit,
-                           wmask);
-    if (e != cudaSuccess) return e;
-    ++*launches;
+    for (int begin = 0; begin < L.w; begin += plan.cols) {
+        const ColRun run{begin, std::min(plan.cols, L.w - begin)};
+        const size_t ns = (size_t)nbands * wave_chunks(run.cols) * kChunk * 32;
+        RPack<C64>* wr = reinterpret_cast<RPack<C64>*>(steps + ns);
+        const size_t items = ns / 32 + (WIN ? (size_t)nbands * wave_lead(c.D) : 0);
+        const int blocks = (int)std::min<size_t>((items + 7) / 8, 148 * 8);
+        refine_prep_kernel<C64, WIN><<<blocks, 256, 0, s>>>(c, fwd, run, rel, prefix, tab.value[it], tab.rejected[it],
+                                                            tab.nrej[it], P + it, lpk, rpk, work, steps, wr);
+        ++*launches;
+        cudaError_t e = cudaGetLastError();
+        // the bands' progress counts a run's columns; refine_advance clears it behind the last run
+        if (e == cudaSuccess && begin > 0) e = cudaMemsetAsync(progress, 0, (size_t)nbands * 4, s);
+        if (e != cudaSuccess) return e;
+        // every band at once (a band waits for the one above): a cooperative launch in clusters
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((nbands + plan.csize - 1) / plan.csize * plan.csize);
+        cfg.blockDim = dim3(3 * kBand);
+        cfg.dynamicSmemBytes = plan.smem;
+        cfg.stream = s;
+        cudaLaunchAttribute at[2];
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+        at[1].id = cudaLaunchAttributeClusterDimension;
+        at[1].val.clusterDim.x = plan.csize;
+        at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 2;
+        e = cudaLaunchKernelEx(&cfg, fwd ? refine_band_kernel<C64, WIN, true> : refine_band_kernel<C64, WIN, false>, c,
+                               nbands, plan.csize, run, (const RStep<C64>*)steps, (const RPack<C64>*)wr, rpk, work,
+                               progress, err, spin_limit, plan.wmask);
+        if (e != cudaSuccess) return e;
+        ++*launches;
+    }
     // start of the next pass, and cleared progress counters
     refine_advance_kernel<<<1, 64, 0, s>>>(P, it, prefix + n, tab.rejected[it], tab.nrej[it], progress, nbands);
     ++*launches;
@@ -939,24 +966,32 @@ cudaError_t launch_refine_pass(const CostCtx& c, const Layout& L, unsigned char*
     const bool fwd = (it % 2) == 0;
     // about a second of waiting at most per wait, unless the engine's tuning sets a smaller poll budget
     const int spin_limit = tune.spin_limit > 0 ? tune.spin_limit : 1 << 23;
-    const size_t up = (size_t)up_blocks(L.w) * (kChunk * 4 + 8);
     // the right-image window in shared memory (32-bit census): a power-of-two ring of steps holding the
-    // window (rounded up to whole chunks) plus the kRing steps copied ahead, when every band still fits
-    // on the device at once
-    if (!c.census64 && tune.window == 0) {
-        int rs = 1;
-        while (rs < wave_lead(c.D) + kRing + kChunk) rs <<= 1;
-        const size_t smem = (size_t)rs * 32 * sizeof(RPack<false>) + up;
-        if (rs <= 512) {
-            const int cs = cluster_size_of<false, true>(fwd, nbands, smem);
-            if (cs) return launch_pass_t<false, true>(c, L, arena, tab, it, work, spin_limit, rs - 1, smem, cs, s, launches);
+    // window (rounded up to whole chunks) plus the kRing steps copied ahead
+    int rs = 1;
+    while (rs < wave_lead(c.D) + kRing + kChunk) rs <<= 1;
+    const bool win = !c.census64 && tune.window == 0 && rs <= 512;
+    // whole rows where every band of the frame is resident at once with the row above in its block, with the
+    // window beside it if that fits too; else in the fewest runs of columns in which they are
+    for (int runs = 1;; runs *= 2) {
+        PassPlan plan{0, (L.w + runs - 1) / runs, 0, 0};
+        const size_t up = (size_t)up_blocks(plan.cols) * (kChunk * 4 + 8);
+        if (win) {
+            plan.smem = up + (size_t)rs * 32 * sizeof(RPack<false>);
+            plan.wmask = rs - 1;
+            plan.csize = cluster_size_of<false, true>(fwd, nbands, plan.smem);
+            if (plan.csize) return launch_pass_t<false, true>(c, L, arena, tab, it, work, spin_limit, plan, s, launches);
+            cudaGetLastError();
         }
+        plan.smem = up;
+        plan.wmask = 0;
+        plan.csize = c.census64 ? cluster_size_of<true, false>(fwd, nbands, up) : cluster_size_of<false, false>(fwd, nbands, up);
+        if (plan.csize)
+            return c.census64 ? launch_pass_t<true, false>(c, L, arena, tab, it, work, spin_limit, plan, s, launches)
+                              : launch_pass_t<false, false>(c, L, arena, tab, it, work, spin_limit, plan, s, launches);
         cudaGetLastError();
+        if (plan.cols <= 8 * kBand) return cudaErrorCooperativeLaunchTooLarge;
     }
-    const int cs = c.census64 ? cluster_size_of<true, false>(fwd, nbands, up) : cluster_size_of<false, false>(fwd, nbands, up);
-    if (!cs) return cudaErrorCooperativeLaunchTooLarge;
-    return c.census64 ? launch_pass_t<true, false>(c, L, arena, tab, it, work, spin_limit, 0, up, cs, s, launches)
-                      : launch_pass_t<false, false>(c, L, arena, tab, it, work, spin_limit, 0, up, cs, s, launches);
 }
 
 }  // namespace apgcu
