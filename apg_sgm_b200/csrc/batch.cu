@@ -610,7 +610,7 @@ int Batch::process(int n, const apgcu_pair_t* pairs, bool device_buffers) {
         SgmLaunch probe;
         uint32_t* s7[7];
         b.slots[0]->sgm_launch(&probe, s7);
-        const bool batched = use_batched_sgm_ && sgm_batch_supported(Dp) && probe.cvol != nullptr && !probe.cost8;
+        const bool batched = use_batched_sgm_ && sgm_batch_supported(Dp) && probe.cvol != nullptr && !probe.bytes;
         if (!batched || b.tune.sgm_lanes != 32) unified = false;
         batched_of.push_back(batched);
         comp.emplace_back(g.first, m);

@@ -206,16 +206,19 @@ Layout Engine::make_layout(const apg_pipeline_config_t& c, int w, int h, int ch,
     // voxels exactly, and the largest P2 is at most 255, so the path values' distances above the costs
     // fit a byte: the census-only Fast volume (written by the pixel-run cost kernel) and the aggregated
     // volume of one aggregation pass (window averages of quantised costs, written by the vertical
-    // aggregation).  kLayoutCost16 (tuning cost8 = 1, other lane counts) keeps the 16-bit sweeps.  The
-    // arena's volume and sum buffers keep the 16-bit sweeps' sizes, so either form runs in it, but for
-    // the volume at a padded range of 256 (at 128 on request, kLayoutCost8).
+    // aggregation).  kLayoutCost16 (tuning cost8 = 1, other lane counts) keeps the 16-bit sweeps over
+    // two-byte volumes.  The arena's volume and sum buffers keep the 16-bit sweeps' sizes, so either form
+    // runs in it, but for the volume at a padded range of 256 (at 128 on request, kLayoutCost8): the
+    // 16-bit sweeps read one byte per voxel there too (larger penalties, frames of 2^32 voxels and more;
+    // 1920x1080 D256 with P2 300, over one byte / two: Fast 2.15 / 2.40 ms a frame, Balanced 3.55 / 3.81).
     const bool fast8 = !L.cross && !L.fused_fast && c.census_type == APG_CENSUS_SYMMETRIC_9X7 && !c.use_ad &&
                        !c.use_grad && max_census_cost(c) < 255;
     const bool cross8 = L.cross && c.agg_iterations <= 1 && max_full_cost(c) < 255;
     // (the byte sweeps address a volume by 32-bit byte offsets)
     L.bytes = (fast8 || cross8) && sgm8_supported(L.Dp, pen_of(c)) && !(debug & kLayoutCost16) &&
               (unsigned long long)w * h * L.Dp < (1ull << 32);
-    L.cost8 = L.bytes && (L.Dp == 256 || (L.Dp == 128 && (debug & kLayoutCost8)));
+    L.cost8 = (fast8 || cross8) && (L.Dp == 256 || (L.Dp == 128 && (debug & kLayoutCost8))) &&
+              !(debug & kLayoutCost16);
     const size_t n = (size_t)w * h;
     const size_t csz = c.census_type == APG_CENSUS_9X7 ? 8 : 4;
     const size_t vol = n * (size_t)L.Dp * 2;
@@ -782,7 +785,7 @@ int Engine::run_pre(const uint8_t* dl, int lstride, const uint8_t* dr, int rstri
         if (!L.raw_cost) RUN(launch_cost(cc, 2, lmax, 0, nullptr, ptr<uint32_t>(L.rkey), magic, s), "right argmin");
     } else {
         CostCtx cv = cc;
-        cv.vol8 = L.bytes ? 1 : 0;
+        cv.vol8 = L.vol8() ? 1 : 0;
         RUN(launch_cost(cv, 0, lmax, 0, ptr<uint32_t>(L.volA), ptr<uint32_t>(L.rkey), magic, s), "cost");
         sgm_src = ptr<uint32_t>(L.volA);
     }
@@ -802,7 +805,7 @@ int Engine::run_pre(const uint8_t* dl, int lstride, const uint8_t* dr, int rstri
                                 ptr<uint8_t>(L.volA), ptr<uint8_t>(L.volB), !ranged(), s), "crossV");
         else
             RUN(launch_cross_v(w, h, d0, D, Dp, lmax, tau, ptr<uint8_t>(L.lgray), ptr<int16_t>(L.rmin), ptr<int16_t>(L.rmax),
-                           ptr<uint32_t>(L.volA), ptr<uint32_t>(L.volB), magic, !ranged(), L.bytes, s), "crossV");
+                           ptr<uint32_t>(L.volA), ptr<uint32_t>(L.volB), magic, !ranged(), L.vol8(), s), "crossV");
         const int iters = std::max(1, cfg_.agg_iterations);
         for (int it = 1; it < iters; ++it) {
             RUN(launch_cross_h(w, h, d0, D, Dp, lmax, tau, ptr<uint8_t>(L.lgray), ptr<int16_t>(L.rmin), ptr<int16_t>(L.rmax),
@@ -836,7 +839,8 @@ int Engine::sgm_launch(SgmLaunch* out, uint32_t** sbufs) const {
     pl.store_final = (debug_ & 2) != 0;
     pl.lanes = sgm_lanes_;
     pl.split = sgm_split_;
-    pl.cost8 = L.bytes ? 1 : 0;
+    pl.cost8 = (!L.fused_fast && L.vol8()) ? 1 : 0;
+    pl.bytes = L.bytes ? 1 : 0;
     pl.default_ranges = ranged() ? 0 : 1;
     if (L.bytes) {
         // two directions' byte buffers in each of the sum buffers but the first, which the stage
@@ -1458,7 +1462,7 @@ int Engine::dump(int what, void* dst, size_t bytes) {
             if (!L.cross) return fail(kInternalError, "no aggregated volume");
             off = L.volB;
             vol = true;
-            vol8 = L.bytes;
+            vol8 = L.vol8();
             break;
         case 12: if (!(debug_ & 2)) return fail(kInternalError, "path sum not kept"); off = L.sbuf[0]; vol = true; break;
         case 13: off = L.disp_wta; sz = n * 4; break;

@@ -40,7 +40,8 @@ struct Layout {
     bool raw_cost = false;    // debug: materialise the raw volume
     bool bytes = false;       // the byte sweeps (sgm8.cu): the volume they read holds one byte per voxel (0xFF
                               // invalid) and the first phase one byte per voxel and direction
-    bool cost8 = false;       // with `bytes`: the volume is allocated at one byte per voxel
+    bool cost8 = false;       // the volume is allocated at one byte per voxel (and holds that: 16-bit sweeps too)
+    bool vol8() const { return bytes || cost8; }  // the volume the sweeps read holds one byte per voxel
     size_t total = 0;
     // offsets
     size_t in_left, in_right;
@@ -235,7 +236,7 @@ private:
     int debug_ = 0;
     int sgm_lanes_ = 0;
     int sgm_split_ = 0;  // last sweep over two warps per chain: 0 auto, 1 never, 2 always
-    int cost8_ = 0;  // byte sweeps: 0 = where exact, 1 = never, 2 = as 0, byte volume allocated at Dp 128 too
+    int cost8_ = 0;  // byte volumes and sweeps: 0 = where exact, 1 = never, 2 = as 0, byte volume allocated at Dp 128 too
     bool fast_fused_ = false;
     int cost_tile_ = 0;
     int cost_kernel_ = 0;  // 0: pixel-run cost kernel where it applies, 1: column-tile kernel

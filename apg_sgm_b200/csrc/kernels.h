@@ -82,7 +82,8 @@ struct SgmLaunch {
     int lanes;        // lanes per scanline chain (8, 16, 32; 0 = default for Dp)
     int split = 0;    // volume-fed last sweep over two warps per chain: 0 = where it pays (Dp 64),
                       // 1 = never, 2 = always (32 lanes per chain only)
-    int cost8 = 0;    // cvol holds one byte per voxel, 0xFF invalid: the byte sweeps (launch_sgm8_*)
+    int cost8 = 0;    // cvol holds one byte per voxel, 0xFF invalid (16-bit sweeps: 32 lanes, Dp 128 or 256)
+    int bytes = 0;    // the byte sweeps (launch_sgm8_*) over such a volume
     int default_ranges = 0;    // byte sweeps: every pixel has the default range
     uint32_t* sum = nullptr;   // byte sweeps: the final sums as a 16-bit volume (stage dumps), or none
 };
@@ -98,7 +99,7 @@ cudaError_t launch_sgm_last(const SgmLaunch& l, int dx, int dy, int nin, const u
 bool sgm_last_band_supported(const SgmLaunch& l, int nin);
 cudaError_t launch_sgm_last_band(const SgmLaunch& l, int dx, int dy, int nin, const uint32_t* const* in, int t_begin,
                                  int t_end, uint32_t* carry, cudaStream_t s);
-// sgm8.cu: the same sweeps over the byte volume (l.cost8), two scanlines per warp, the first phase
+// sgm8.cu: the same sweeps over the byte volume (l.bytes), two scanlines per warp, the first phase
 // writing one byte per voxel and direction (Dp bytes per pixel): where every quantised cost is below
 // 255, the largest P2 at most 255 and Dp at most 256.  nin is 3 or 7 (every direction of the first
 // phase); bands as above with nin 3 and sgm8_carry_words(w, Dp) words in `carry`.

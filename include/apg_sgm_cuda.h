@@ -73,7 +73,9 @@ APGCU_API int apgcu_engine_set_debug(apgcu_engine_t e, int flags);
  *            one byte per voxel, exact while every quantised cost is below 255, P2 at most 255 and
  *            the padded range at most 256: 0 = wherever that holds (default), 1 = never (16-bit
  *            sweeps), 2 = as 0, and the volume is allocated at one byte per voxel at 128 padded
- *            disparities too (0 does so at 256 only);
+ *            disparities too (0 does so at 256 only).  Where only the costs fit (larger P2, frames of 2^32
+ *            voxels and more), the 16-bit sweeps read one byte per voxel at 256 padded disparities (2: and
+ *            at 128);
  *   "refine_window": 0 = HighQuality refiner reads the right-image window from shared memory where
  *                 every band fits on the device at once (default), 1 = always through L1;
  *   "host_bands": frames whose outputs go to host memory (apgcu_engine_process, the session) run
