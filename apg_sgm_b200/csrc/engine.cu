@@ -242,6 +242,7 @@ Layout Engine::make_layout(const apg_pipeline_config_t& c, int w, int h, int ch,
     L.volB = L.cross ? take(L.cost8 ? vol / 2 : vol) : 0;
     L.nsbuf = (c.paths == 8 ? 8 : 4) - 1;
     for (int i = 0; i < L.nsbuf; ++i) L.sbuf[i] = (i == 0 && (L.cross || L.fused_fast)) ? L.volA : take(vol);
+    const size_t sums_end = o;
     L.volRaw = L.raw_cost ? take(vol) : 0;
     L.tel = take(sizeof(apg_subpixel_telemetry_t) + sizeof(apg_inpaint_telemetry_t));
     L.lut = take(kLutSize * 4);
@@ -273,7 +274,10 @@ Layout Engine::make_layout(const apg_pipeline_config_t& c, int w, int h, int ch,
         L.rf_scan_tmp = take(L.rf_scan_tmp_bytes);
         L.rf_state = take((size_t)(kRefineProgWord + refine_band_count(h)) * 4);
         L.rf_pack = take(refine_pack_bytes((int)n, c.census_type == APG_CENSUS_9X7));
-        L.rf_steps = take(refine_steps_bytes(w, h, L.D, c.census_type == APG_CENSUS_9X7));
+        // a pass's records lie in the sum buffers behind the first (which a stage dump reads), free once the
+        // last sweep has run; frames of a few rows or columns, whose records are mostly padding, take their own
+        const size_t steps = refine_steps_bytes(w, h, L.D, c.census_type == APG_CENSUS_9X7);
+        L.rf_steps = steps <= sums_end - L.sbuf[1] ? L.sbuf[1] : take(steps);
     }
     L.total = o;
     return L;

@@ -16,3 +16,13 @@ def test_frames_of_four_gigavoxels_keep_the_byte_volume(apg):
     for mode, vols in ((0, 3.5), (1, 3.5), (2, 7.5)):
         vol = w * h * 256 * 2
         assert apg.workspace_bytes(apg.config_from_mode(mode, 256), w, h) < (vols + 0.3) * vol
+
+
+@pytest.mark.parametrize("w,h,dmax", [(64, 64, 16), (160, 120, 64), (1242, 375, 192), (1920, 1080, 256), (20, 2000, 16)])
+@pytest.mark.parametrize("over", [{}, {"census_type": 0}, {"paths": 4}])
+def test_refiner_workspace(apg, w, h, dmax, over):
+    """The refiner's own buffers: a 4-byte draw index, two packed images and one 32-byte record per pixel at
+    most, and scratch that does not grow with the frame's area (a kilobyte per 32 rows, 16 KB in all)."""
+    pack = 32 if over.get("census_type") == 0 else 16
+    ws = [apg.workspace_bytes(apg.config_from_mode(2, dmax, 0, refine_enable=r, **over), w, h) for r in (0, 1)]
+    assert 0 < ws[1] - ws[0] <= w * h * (4 + pack + 32) + h * 32 + 16384
