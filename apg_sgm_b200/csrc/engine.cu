@@ -1475,12 +1475,16 @@ int Engine::dump(int what, void* dst, size_t bytes) {
         case 16:
             off = L.disp_right;
             sz = n * 4;
-            // without the refiner the confidence stage works the right disparities out itself: write the map
-            // now (the same values where the frame wrote it)
-            if (const cudaError_t e = launch_right_wta_finalize(cost_ctx(), ptr<uint32_t>(L.rkey), cfg_.subpixel,
-                                                                ptr<float>(L.disp_right), stream_);
-                e != cudaSuccess)
-                return cuda_fail(e, "right disparity");
+            // where only the confidence stage reads the right disparities, it works them out itself and the frame
+            // left the keys alone: write the map now
+            if (!right_written_) {
+                cudaSetDevice(device_);
+                if (const cudaError_t e = launch_right_wta_finalize(cost_ctx(), ptr<uint32_t>(L.rkey), cfg_.subpixel,
+                                                                    ptr<float>(L.disp_right), stream_);
+                    e != cudaSuccess)
+                    return cuda_fail(e, "right disparity");
+                count_launches(1);
+            }
             break;
         case 17: off = L.confidence; sz = n * 4; break;
         case 18: off = L.reliable; sz = n; break;
