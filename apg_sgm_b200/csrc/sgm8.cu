@@ -18,19 +18,22 @@
 //   * per word: t = min(L'(d-1), L'(d+1)); x = min(t + P1, L'(d)); delta = min(x - m', P2);
 //     L = C + delta: three DPX / SIMD minima and one 32-bit add.  m' enters last, so the warp's two
 //     min-reductions run beside the neighbour shuffles and the first two minima.
-// Values: valid costs are at most 254 and valid path values at most 254 + 255.  An invalid cost is
-// widened to at least 0x0F00, above any candidate min' + P2, so an invalid neighbour never wins; all
-// halves stay below 0x2000, so plain 32-bit adds never carry between them and the signed minima are
-// exact.  A pixel whose predecessor has no valid entry (m' >= 0x0800) takes L = C: P2 reads as 0
-// there, which makes every delta 0; the first pixel of a scanline does the same with L' = 0.
+// Values (each biased by 0x0400): valid costs are at most 254 and valid path values at most 254 + 255 = 509.
+// An invalid cost is widened to 0x03FF, a padded one to at least 0x0300 = 768.  The room is tight: no valid
+// entry takes a candidate from an invalid neighbour while 768 > m' + P2 for every valid m', so 768 - 509 = 259
+// must exceed the largest P2, 255.  All halves of path values stay below 0x2000, so plain 32-bit adds never carry between
+// them and the signed minima are exact.  A pixel whose predecessor has no valid entry (m' >= 0x0300) takes
+// L = C: P2 reads as 0 there, which makes every delta 0; the first pixel of a scanline does the same with
+// L' = 0.
 //
 // Steps whose pixels have every disparity of the range valid (default ranges: x >= dmax - 1) skip the
 // invalid-byte test: only the padded disparities are invalid there, a constant mask per lane.
 //
-// Loads run PF steps ahead through a per-warp shared-memory ring of cp.async groups, 16 bytes per
-// lane: one copy instruction brings both scanlines' costs of a step (two at 128 padded disparities
-// with three partial sums).  Bound: HBM for full frames, else each step's dependent chain (reduction,
-// two minima, add; about 60 cycles).
+// Loads run one to three groups of steps ahead through a per-warp shared-memory ring, a cp.async group each,
+// 16 bytes per lane: at 256 padded disparities one copy instruction brings both scanlines' costs of a step, at
+// 64 those of four.  Bound: HBM for full frames (1920x1080 D256: the first phase at 91% of the copy rate, the
+// last sweep at 76%), else each step's dependent chain (reduction, two minima, add; 135 cycles at 640x480
+// D64).
 #include "sgm8.cuh"
 
 #include <algorithm>
@@ -47,11 +50,17 @@ constexpr int kMaxIn = 7;                   // first-phase directions of Path8
 // subtraction negates both halves (n = 0x10000 - acc, exact in each half modulo 2^16).
 constexpr uint32_t kBias = 0x0400u;
 constexpr uint32_t kBias2 = 0x04000400u;
-constexpr uint32_t kPad2 = 0x07000700u;     // bias and the invalid marker 0x0300 (with the byte 0xFF: 0x03FF)
+constexpr uint32_t kInvalid = 0x0300u;      // invalid path values are at least this, valid ones below
+constexpr uint32_t kPad2 = 0x07000700u;     // bias and the invalid marker (with the byte 0xFF: 0x03FF)
 constexpr uint32_t kEdge2 = 0x0FFF0FFFu;    // beyond the ends of the range: above every path value
 // A max-reduction of negated minima holds -(kBias + m') in its high half; below this m' is invalid.
-constexpr uint32_t kNoPred = (0x10000u - kBias - 0x0300u) << 16;
+constexpr uint32_t kNoPred = (0x10000u - kBias - kInvalid) << 16;
 constexpr uint32_t kFresh = (0x10000u - kBias) << 16;  // m' = 0
+constexpr uint32_t kMaxCost = 254, kMaxP2 = 255;       // what the callers keep to (sgm8_supported, the engine's layout)
+static_assert(kPad2 == (kBias + kInvalid) * 0x00010001u, "padded disparities are invalid");
+static_assert(kInvalid > kMaxCost + kMaxP2 + kMaxP2, "an invalid neighbour never wins over m' + P2");
+static_assert((kEdge2 & 0xFFFFu) > kBias + (kInvalid | 0xFFu) + kMaxP2 + kMaxP2, "nor does the edge");
+static_assert((kBias + (kInvalid | 0xFFu) + kMaxP2) * (kMaxIn + 1) < 0x8000u, "sums of all directions fit their halves");
 
 struct Args8 {
     int w, h, d0, D, dmax;
@@ -459,7 +468,7 @@ __device__ __forceinline__ void run_first8(const Args8& a, uint8_t* smem, int dx
 template <int NIN>
 __host__ __device__ constexpr uint32_t sum_bias() { return kBias * (NIN + 1); }
 template <int NIN>
-__host__ __device__ constexpr uint32_t sum_inf() { return (kBias + 0x0300u) * (NIN + 1); }
+__host__ __device__ constexpr uint32_t sum_inf() { return (kBias + kInvalid) * (NIN + 1); }
 
 // The deltas of NIN arrays at sl (layout [array][A, B][DP]); with PS in pairs, added as bytes.
 template <int DP, int NIN, bool PS>
@@ -976,7 +985,7 @@ cudaError_t launch_last_any(const SgmLaunch& l, const Args8& a, int dx, int dy, 
 
 }  // namespace
 
-bool sgm8_supported(int Dp, const SgmPen& pen) { return Dp <= 256 && Dp % 64 == 0 && max_p2(pen) <= 255; }
+bool sgm8_supported(int Dp, const SgmPen& pen) { return Dp <= 256 && Dp % 64 == 0 && max_p2(pen) <= (int)kMaxP2; }
 
 size_t sgm8_carry_words(int w, int Dp) { return (size_t)((w + 1) / 2) * 32 * ((Dp >= 192 ? 8 : Dp / 32)); }
 
