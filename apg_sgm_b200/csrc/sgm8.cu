@@ -21,10 +21,10 @@
 // Values (each biased by 0x0400): valid costs are at most 254 and valid path values at most 254 + 255 = 509.
 // An invalid cost is widened to 0x03FF, a padded one to at least 0x0300 = 768.  The room is tight: no valid
 // entry takes a candidate from an invalid neighbour while 768 > m' + P2 for every valid m', so 768 - 509 = 259
-// must exceed the largest P2, 255.  All halves of path values stay below 0x2000, so plain 32-bit adds never carry between
-// them and the signed minima are exact.  A pixel whose predecessor has no valid entry (m' >= 0x0300) takes
-// L = C: P2 reads as 0 there, which makes every delta 0; the first pixel of a scanline does the same with
-// L' = 0.
+// must exceed the largest P2, 255.  All halves of path values stay below 0x2000, so plain 32-bit adds never
+// carry between them and the signed minima are exact.  A pixel whose predecessor has no valid entry (m' >=
+// 0x0300) takes L = C: P2 reads as 0 there, which makes every delta 0; the first pixel of a scanline does the
+// same with L' = 0.
 //
 // Steps whose pixels have every disparity of the range valid (default ranges: x >= dmax - 1) skip the
 // invalid-byte test: only the padded disparities are invalid there, a constant mask per lane.
