@@ -1098,8 +1098,9 @@ def _result_arrays(h: int, w: int, out=None) -> dict:
 class Batch:
     """Batched form (apgcu_batch_*): many pairs of uneven sizes and disparity ranges per call.
 
-    Pairs of equal size and range form a bucket; a bucket's pairs run their per-pixel stages
-    concurrently and share one persistent SGM launch per phase, replayed from a cached CUDA graph.
+    Pairs of equal size and range form a bucket; a bucket's pairs run concurrently, replayed from a
+    cached CUDA graph (configurations with 16-bit sweeps, which no preset is, share one persistent SGM
+    launch per phase between their per-pixel stages).
     Each pair's outputs equal those of Engine.process for that pair alone."""
 
     def __init__(self, config: PipelineConfig, device: int = 0, **options):

@@ -116,7 +116,8 @@ APGCU_API int apgcu_engine_sync(apgcu_engine_t e);
 APGCU_API int apgcu_engine_dump(apgcu_engine_t e, int what, void* host_dst, size_t bytes);
 
 /* Per-stage device times of the last pair (ms): aux, prior, cost, cross, right_wta, sgm, wta,
- * confidence, refine, post, total -- the reference StageTiming fields in declaration order. */
+ * confidence, refine, post, total -- the reference StageTiming fields in declaration order.  Without the
+ * refiner the right-image disparities are worked out in the confidence stage and right_wta reads near 0. */
 APGCU_API int apgcu_engine_stage_times(apgcu_engine_t e, double* ms11);
 
 /* Per-launch device times of the last pair (needs APGCU_DEBUG_PROFILE): up to max entries of
@@ -256,11 +257,13 @@ APGCU_API unsigned long long apgcu_kernel_launch_count(void);
  *
  * No counterpart in the reference (which processes one pair per call): pairs are grouped into
  * buckets of equal size and disparity range; every pair runs its per-pixel stages on its own
- * stream, and the pairs of ALL buckets share one persistent SGM launch per phase (a work queue of
- * (pair, direction, scanline) units over pairs of any size and padded range); the whole call is a
- * cached CUDA graph per composition (buckets and pair counts); the cost kernel's tile width is
- * autotuned per bucket.  With the option "unified_sgm" 0 each bucket runs on its own stream with
- * its own SGM launches, and the tuner also chooses lanes per scanline and the persistent-grid cap.
+ * stream, and its byte sweeps there too (see "cost8"; every preset), in a cached CUDA graph per
+ * bucket and pair count.  Pairs with 16-bit sweeps, of ALL buckets, share one persistent SGM launch per
+ * phase (a work queue of (pair, direction, scanline) units over pairs of any size and padded range) in a
+ * cached graph per composition (buckets and pair counts).  The cost kernel's tile width is autotuned
+ * per bucket.  With the option "unified_sgm" 0 each bucket of 16-bit pairs runs on its own stream with
+ * its own SGM launches, and the tuner also chooses lanes per scanline and the persistent-grid cap; the
+ * option "sgm_lanes" 16 runs every bucket with 16-bit sweeps.
  * Every pair's outputs equal what apgcu_engine_process gives for it alone. */
 typedef struct apgcu_batch_s* apgcu_batch_t;
 typedef struct {
