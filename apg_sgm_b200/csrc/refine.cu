@@ -17,6 +17,8 @@
 // A band keeps the row above whole in shared memory (5 bytes a column), so frames whose bands do not all
 // fit on the device at once that way take a pass in several runs of columns, one launch after another: every
 // row of a run comes before the next run's first column, whose left neighbours are then read from the map.
+// Frames of more bands than the device holds whatever the columns (740, 23,680 rows) take a pass in groups of
+// bands, one launch after another: the band above a group's first has ended, its last row lies in the map.
 //
 // Measured (one B200, all three passes of HighQuality with their per-pixel kernels): 1920x1080 D256
 // 1.97 ms, 1280x720 D128 1.27 ms, where steps with divergent branches, per-step hand-overs by polling
@@ -561,7 +563,7 @@ __device__ __forceinline__ float step_cost(const float* lut, const RPack<C64>& l
 // records come by bulk copies that use no issue slot or load path of the SM, and a band hands its last
 // row to the next one through the cluster's shared memory.
 template <bool C64, bool WIN, bool FWD>
-__global__ void __launch_bounds__(96) refine_band_kernel(CostCtx c, int nbands, int csize, ColRun run,
+__global__ void __launch_bounds__(96) refine_band_kernel(CostCtx c, int band0, int nbands, int csize, ColRun run,
                                                          const RStep<C64>* __restrict__ steps,
                                                          const RPack<C64>* __restrict__ wr,
                                                          const RPack<C64>* __restrict__ rp, float* work,
@@ -577,8 +579,8 @@ __global__ void __launch_bounds__(96) refine_band_kernel(CostCtx c, int nbands, 
     RPack<C64>* s_win = reinterpret_cast<RPack<C64>*>(s_dyn);
     int* s_up = reinterpret_cast<int*>(s_dyn + (WIN ? (size_t)(wmask + 1) * 32 * sizeof(RPack<C64>) : 0));
     uint64_t* s_upbar = reinterpret_cast<uint64_t*>(s_up + ublk * kChunk);
-    const int band = blockIdx.x;
-    const int rank = band % csize;
+    const int band = band0 + (int)blockIdx.x;  // a group of bands starts with a cluster
+    const int rank = (int)blockIdx.x % csize;
     const bool live = band < nbands;
     // the row above comes from the cluster's previous band, from another cluster, or (band 0) nowhere
     const bool from_peer = live && rank > 0, from_link = live && band > 0 && rank == 0;
@@ -869,10 +871,10 @@ size_t refine_steps_bytes(int w, int h, int D, bool c64) {
 
 namespace {
 
-// How a pass runs: in clusters of `csize` bands, `cols` columns a launch, `smem` bytes and a window ring of
-// wmask + 1 steps a block (csize 0: not at all).
+// How a pass runs: in clusters of `csize` bands, `cols` columns and up to `group` bands (whole clusters) a
+// launch, `smem` bytes and a window ring of wmask + 1 steps a block (csize 0: not at all).
 struct PassPlan {
-    int csize, cols, wmask;
+    int csize, group, cols, wmask;
     size_t smem;
 };
 
@@ -903,25 +905,28 @@ cudaError_t launch_pass_t(const CostCtx& c, const Layout& L, unsigned char* aren
         // the bands' progress counts a run's columns; refine_advance clears it behind the last run
         if (e == cudaSuccess && begin > 0) e = cudaMemsetAsync(progress, 0, (size_t)nbands * 4, s);
         if (e != cudaSuccess) return e;
-        // every band at once (a band waits for the one above): a cooperative launch in clusters
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((nbands + plan.csize - 1) / plan.csize * plan.csize);
-        cfg.blockDim = dim3(3 * kBand);
-        cfg.dynamicSmemBytes = plan.smem;
-        cfg.stream = s;
-        cudaLaunchAttribute at[2];
-        at[0].id = cudaLaunchAttributeCooperative;
-        at[0].val.cooperative = 1;
-        at[1].id = cudaLaunchAttributeClusterDimension;
-        at[1].val.clusterDim.x = plan.csize;
-        at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 2;
-        e = cudaLaunchKernelEx(&cfg, fwd ? refine_band_kernel<C64, WIN, true> : refine_band_kernel<C64, WIN, false>, c,
-                               nbands, plan.csize, run, (const RStep<C64>*)steps, (const RPack<C64>*)wr, rpk, work,
-                               progress, err, spin_limit, plan.wmask);
-        if (e != cudaSuccess) return e;
-        ++*launches;
+        for (int b0 = 0; b0 < nbands; b0 += plan.group) {
+            // every band of the group at once (a band waits for the one above): a cooperative launch in clusters
+            const int nb = std::min(plan.group, nbands - b0);
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((nb + plan.csize - 1) / plan.csize * plan.csize);
+            cfg.blockDim = dim3(3 * kBand);
+            cfg.dynamicSmemBytes = plan.smem;
+            cfg.stream = s;
+            cudaLaunchAttribute at[2];
+            at[0].id = cudaLaunchAttributeCooperative;
+            at[0].val.cooperative = 1;
+            at[1].id = cudaLaunchAttributeClusterDimension;
+            at[1].val.clusterDim.x = plan.csize;
+            at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 2;
+            e = cudaLaunchKernelEx(&cfg, fwd ? refine_band_kernel<C64, WIN, true> : refine_band_kernel<C64, WIN, false>, c,
+                                   b0, nbands, plan.csize, run, (const RStep<C64>*)steps, (const RPack<C64>*)wr, rpk,
+                                   work, progress, err, spin_limit, plan.wmask);
+            if (e != cudaSuccess) return e;
+            ++*launches;
+        }
     }
     // start of the next pass, and cleared progress counters
     refine_advance_kernel<<<1, 64, 0, s>>>(P, it, prefix + n, tab.rejected[it], tab.nrej[it], progress, nbands);
@@ -929,33 +934,41 @@ cudaError_t launch_pass_t(const CostCtx& c, const Layout& L, unsigned char* aren
     return cudaGetLastError();
 }
 
-// The largest cluster (8, 4, 2, 1 bands) in which every band of the frame is resident at once with
-// `smem` bytes each, or 0.
+// Sets plan's cluster and group for blocks of plan.smem bytes: the largest cluster (8, 4, 2, 1 bands) in which
+// every band of the frame is resident at once; with `parts`, else the largest that fits at all and as many bands
+// as are.
 template <bool C64, bool WIN, bool FWD>
-int cluster_size(int nbands, size_t smem) {
+bool place_bands(int nbands, bool parts, PassPlan& plan) {
     auto kern = refine_band_kernel<C64, WIN, FWD>;
-    if (allow_dynamic_smem(kern, smem) != cudaSuccess) return 0;
-    for (int cs = 8; cs >= 1; cs >>= 1) {
-        if (cs > 1 && cs > nbands) continue;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((nbands + cs - 1) / cs * cs);
-        cfg.blockDim = dim3(3 * kBand);
-        cfg.dynamicSmemBytes = smem;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = cs;
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        int nc = 0;
-        if (cudaOccupancyMaxActiveClusters(&nc, kern, &cfg) == cudaSuccess && nc * cs >= (int)cfg.gridDim.x) return cs;
-        cudaGetLastError();
+    plan.csize = 0;
+    if (allow_dynamic_smem(kern, plan.smem) == cudaSuccess) {
+        for (int cs = 8; cs >= 1; cs >>= 1) {
+            if (cs > 1 && cs > nbands) continue;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((nbands + cs - 1) / cs * cs);
+            cfg.blockDim = dim3(3 * kBand);
+            cfg.dynamicSmemBytes = plan.smem;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = cs;
+            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            int nc = 0;
+            if (cudaOccupancyMaxActiveClusters(&nc, kern, &cfg) != cudaSuccess) nc = 0;
+            if (nc * cs >= (int)cfg.gridDim.x || (parts && nc > 0)) {
+                plan.csize = cs;
+                plan.group = nc * cs;
+                return true;
+            }
+        }
     }
-    return 0;
+    cudaGetLastError();
+    return false;
 }
 template <bool C64, bool WIN>
-int cluster_size_of(bool fwd, int nbands, size_t smem) {
-    return fwd ? cluster_size<C64, WIN, true>(nbands, smem) : cluster_size<C64, WIN, false>(nbands, smem);
+bool place_bands(bool fwd, int nbands, bool parts, PassPlan& plan) {
+    return fwd ? place_bands<C64, WIN, true>(nbands, parts, plan) : place_bands<C64, WIN, false>(nbands, parts, plan);
 }
 
 }  // namespace
@@ -971,25 +984,34 @@ cudaError_t launch_refine_pass(const CostCtx& c, const Layout& L, unsigned char*
     int rs = 1;
     while (rs < wave_lead(c.D) + kRing + kChunk) rs <<= 1;
     const bool win = !c.census64 && tune.window == 0 && rs <= 512;
+    PassPlan plan{};
+    const auto bare = [&](bool parts) {  // without the window
+        plan.wmask = 0;
+        plan.smem = (size_t)up_blocks(plan.cols) * (kChunk * 4 + 8);
+        return c.census64 ? place_bands<true, false>(fwd, nbands, parts, plan)
+                          : place_bands<false, false>(fwd, nbands, parts, plan);
+    };
+    const auto run_bare = [&] {
+        return c.census64 ? launch_pass_t<true, false>(c, L, arena, tab, it, work, spin_limit, plan, s, launches)
+                          : launch_pass_t<false, false>(c, L, arena, tab, it, work, spin_limit, plan, s, launches);
+    };
     // whole rows where every band of the frame is resident at once with the row above in its block, with the
     // window beside it if that fits too; else in the fewest runs of columns in which they are
     for (int runs = 1;; runs *= 2) {
-        PassPlan plan{0, (L.w + runs - 1) / runs, 0, 0};
-        const size_t up = (size_t)up_blocks(plan.cols) * (kChunk * 4 + 8);
+        plan.cols = (L.w + runs - 1) / runs;
         if (win) {
-            plan.smem = up + (size_t)rs * 32 * sizeof(RPack<false>);
             plan.wmask = rs - 1;
-            plan.csize = cluster_size_of<false, true>(fwd, nbands, plan.smem);
-            if (plan.csize) return launch_pass_t<false, true>(c, L, arena, tab, it, work, spin_limit, plan, s, launches);
-            cudaGetLastError();
+            plan.smem = (size_t)up_blocks(plan.cols) * (kChunk * 4 + 8) + (size_t)rs * 32 * sizeof(RPack<false>);
+            if (place_bands<false, true>(fwd, nbands, false, plan))
+                return launch_pass_t<false, true>(c, L, arena, tab, it, work, spin_limit, plan, s, launches);
         }
-        plan.smem = up;
-        plan.wmask = 0;
-        plan.csize = c.census64 ? cluster_size_of<true, false>(fwd, nbands, up) : cluster_size_of<false, false>(fwd, nbands, up);
-        if (plan.csize)
-            return c.census64 ? launch_pass_t<true, false>(c, L, arena, tab, it, work, spin_limit, plan, s, launches)
-                              : launch_pass_t<false, false>(c, L, arena, tab, it, work, spin_limit, plan, s, launches);
-        cudaGetLastError();
+        if (bare(false)) return run_bare();
+        if (plan.cols <= 8 * kBand) break;
+    }
+    // more bands than any run of columns leaves room for: groups of bands, in the fewest runs that a block holds
+    for (int runs = 1;; runs *= 2) {
+        plan.cols = (L.w + runs - 1) / runs;
+        if (bare(true)) return run_bare();
         if (plan.cols <= 8 * kBand) return cudaErrorCooperativeLaunchTooLarge;
     }
 }
