@@ -242,6 +242,15 @@ inline cudaError_t allow_dynamic_smem(F kern, size_t smem) {
     return (long long)smem > limit ? cudaErrorInvalidValue : cudaSuccess;
 }
 
+// Pageable host memory to device memory, there for every stream when it returns.  cudaMemcpy alone may return
+// with the bytes staged and their last copy still to run on the default stream, behind other streams' work that
+// shares its hardware queue; the streams here do not wait for the default one, so a kernel could read what lay
+// there before.
+inline cudaError_t copy_in(void* dst, const void* src, size_t bytes) {
+    const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+    return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+}
+
 #define APGCU_CHECK(expr)                                                    \
     do {                                                                     \
         cudaError_t _e = (expr);                                             \

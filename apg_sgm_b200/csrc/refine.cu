@@ -805,14 +805,14 @@ int RefineTables::build(int iterations, int base_radius, int n) {
     for (int it = 0; it < iterations; ++it) {
         const DrawTable& t = *tabs[it];
         value[it] = reinterpret_cast<int16_t*>(p);
-        if (cudaMemcpy(p, t.value.data(), len[it] * 2, cudaMemcpyHostToDevice) != cudaSuccess) return 1;
+        if (copy_in(p, t.value.data(), len[it] * 2) != cudaSuccess) return 1;
         p += (len[it] * 2 + 255) & ~size_t(255);
         rejected[it] = reinterpret_cast<unsigned*>(p);
         size_t nr = 0;
         for (unsigned r : t.rejected)
             if (r < len[it]) ++nr;
         nrej[it] = (int)nr;
-        if (nr && cudaMemcpy(p, t.rejected.data(), nr * 4, cudaMemcpyHostToDevice) != cudaSuccess) return 1;
+        if (nr && copy_in(p, t.rejected.data(), nr * 4) != cudaSuccess) return 1;
         p += kMaxRejected * 4;
     }
     n_built = n;

@@ -1719,7 +1719,7 @@ cudaError_t sgm_batch_plan_create(const SgmLaunch* pl, uint32_t* const* sbufs, i
         plan->dev = nullptr;
         return e;
     }
-    e = cudaMemcpy(plan->dev, host.data(), total, cudaMemcpyHostToDevice);
+    e = copy_in(plan->dev, host.data(), total);
     if (e != cudaSuccess) sgm_batch_plan_destroy(plan);
     // the sum buffers of every pair, for the Path8 fold
     plan->sums.assign(sbufs, sbufs + (size_t)npairs * nsbuf);
