@@ -781,16 +781,15 @@ int RefineTables::build(int iterations, int base_radius, int n) {
     release();
     std::vector<const DrawTable*> tabs(iterations);
     std::vector<size_t> len(iterations);
-    {
-        std::lock_guard<std::mutex> lk(g_rng_mu);
-        for (int it = 0; it < iterations; ++it) {
-            const int radius = std::max(1, base_radius >> it);
-            if (radius > 32767) return 1;
-            // pass `it` starts at most it * n outputs (plus rejections) into the stream
-            len[it] = (size_t)(it + 1) * n + 64;
-            tabs[it] = &draw_table_locked(radius, len[it]);
-            if (tabs[it]->rejected.size() > (size_t)kMaxRejected) return 1;
-        }
+    // until the tables are copied: another thread's longer frame moves a table as it grows it
+    std::lock_guard<std::mutex> lk(g_rng_mu);
+    for (int it = 0; it < iterations; ++it) {
+        const int radius = std::max(1, base_radius >> it);
+        if (radius > 32767) return 1;
+        // pass `it` starts at most it * n outputs (plus rejections) into the stream
+        len[it] = (size_t)(it + 1) * n + 64;
+        tabs[it] = &draw_table_locked(radius, len[it]);
+        if (tabs[it]->rejected.size() > (size_t)kMaxRejected) return 1;
     }
     iters = iterations;
     size_t total = 0;
